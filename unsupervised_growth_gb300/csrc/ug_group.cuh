@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? UG_RA_MIN_BLOCKS : 1)
     }
     for_items(members, items, *count, M, [&](const GroupMember<R>& m, int bx, int by) {
         if constexpr (sizeof(R) == 4)
-            interval_ra_x2_body<R, kTrack>(m.n, m.bt, q, s0, s1, m.rc, bx * kBlock + (int)threadIdx.x, by);
+            interval_ra_v_body<f2, R, kTrack>(m.n, m.bt, q, s0, s1, m.rc, bx * kBlock + (int)threadIdx.x, by);
         else interval_ra_body<R, kTrack>(m.n, m.bt, q, s0, s1, m.rc, bx, by);
     });
 }

@@ -86,7 +86,7 @@ __device__ __forceinline__ void trial_ra_part(const NetDev<R>& n, const BatchDev
 {
     if (threadIdx.x >= ra_w) return;
     if constexpr (sizeof(R) == 4) {
-        interval_ra_x2_body<R>(n, bt, q, s0, s1, rc, k * ra_w + (int)threadIdx.x, 0);   // pairs [ra_w k, ra_w (k + 1))
+        interval_ra_v_body<f2, R>(n, bt, q, s0, s1, rc, k * ra_w + (int)threadIdx.x, 0);   // pairs [ra_w k, ra_w (k + 1))
     } else {
         interval_ra_body<R>(n, bt, q, s0, s1, rc, k, 0, ra_w);
     }

@@ -17,7 +17,7 @@
 // order (exc before inh within a step).  The integrator then applies kicks at
 // their steps with no double-precision work in its loop.
 #pragma once
-#include "ug_ra_f32x2.cuh"
+#include "ug_ra_f32.cuh"
 
 namespace ug {
 

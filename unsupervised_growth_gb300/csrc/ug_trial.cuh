@@ -20,7 +20,7 @@
 #pragma once
 #include <stdint.h>
 #include "ug_neuron.cuh"
-#include "ug_ra_f32x2.cuh"
+#include "ug_ra_f32.cuh"
 #include "ug_i_f32.cuh"
 
 namespace ug {
@@ -441,125 +441,157 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 8 : 1) k_interval_ra(
     interval_ra_body<R, kTrack>(n, bt, q, s0, s1, rc, (int)blockIdx.x, (int)blockIdx.y);
 }
 
-// Single-precision HVC(RA) part of one interval, two neurons per thread
-// (neurons 2t and 2t+1) so that every floating-point instruction of the
-// integrator is a packed f32x2 operation.
-template <class R, bool kTrack = false>
-__device__ __forceinline__ void interval_ra_x2_body(const NetDev<R>& n, const BatchDev<R>& bt, int q, int s0, int s1,
-                                                    const RAStep<R>& rc, int t, int b)
+// The lanes' entries of a per-neuron parameter array.
+template <class V>
+__device__ __forceinline__ V load_param(const float* p, const uint32_t* ent)
 {
-    // t: the thread's neuron pair (neurons 2t, 2t + 1; none when 2t >= n_ra), b: its instance
-    static_assert(sizeof(R) == 4, "the packed RA kernel is single precision");
-    const int i0 = 2 * t, i1 = 2 * t + 1;
-    const bool v0 = i0 < n.n_ra, v1 = i1 < n.n_ra;
-    uint32_t soma0 = 0, dend0 = 0, soma1 = 0, dend1 = 0;
-    if (v0) {
-        const size_t x0 = (size_t)b * n.n_ra + i0;
-        const size_t x1 = v1 ? x0 + 1 : x0;
-        RA2 s;
-        f2 Ge, Gi;
-        s.Vs = make_float2(bt.ra[0][x0], bt.ra[0][x1]);
-        s.Vd = make_float2(bt.ra[1][x0], bt.ra[1][x1]);
-        s.n = make_float2(bt.ra[2][x0], bt.ra[2][x1]);
-        s.h = make_float2(bt.ra[3][x0], bt.ra[3][x1]);
-        s.l = make_float2(bt.ra[4][x0], bt.ra[4][x1]);
-        s.r = make_float2(bt.ra[5][x0], bt.ra[5][x1]);
-        s.c = make_float2(bt.ra[6][x0], bt.ra[6][x1]);
-        s.Ca = make_float2(bt.ra[7][x0], bt.ra[7][x1]);
-        Ge = make_float2(bt.ra[8][x0], bt.ra[8][x1]);
-        Gi = make_float2(bt.ra[9][x0], bt.ra[9][x1]);
-        int fl0 = bt.ra_flags[x0], fl1 = bt.ra_flags[x1];
-        if (q > 0) {
-            const size_t base = (size_t)((q - 1) % n.ring) * bt.B * n.n_ra;
-            const long long ai0 = bt.ring_ra_inh[base + x0], ae0 = bt.ring_ra_exc[base + x0];
-            const long long ai1 = v1 ? bt.ring_ra_inh[base + x1] : 0, ae1 = v1 ? bt.ring_ra_exc[base + x1] : 0;
-            if (ai0 | ae0) {
-                bt.ring_ra_inh[base + x0] = 0;
-                bt.ring_ra_exc[base + x0] = 0;
-                Gi.x = Gi.x + (float)((double)ai0 * kFixInv);
-                Ge.x = Ge.x + (float)(((double)ae0 * kFixInv) / RAConst::Ad);
-            }
-            if (ai1 | ae1) {
-                bt.ring_ra_inh[base + x1] = 0;
-                bt.ring_ra_exc[base + x1] = 0;
-                Gi.y = Gi.y + (float)((double)ai1 * kFixInv);
-                Ge.y = Ge.y + (float)(((double)ae1 * kFixInv) / RAConst::Ad);
-            }
+    float v[Lanes<V>::n];
+#pragma unroll
+    for (int k = 0; k < Lanes<V>::n; ++k) v[k] = p[ent[k]];
+    return Lanes<V>::make(v);
+}
+
+// The training kick, in the lanes whose kick step is st.
+__device__ __forceinline__ void add_kick(float& Ge, const int* kick, int st)
+{
+    if (st == kick[0]) Ge = Ge + 3.0f;
+}
+__device__ __forceinline__ void add_kick(f2& Ge, const int* kick, int st)
+{
+    if (st == kick[0]) Ge.x = Ge.x + 3.0f;
+    if (st == kick[1]) Ge.y = Ge.y + 3.0f;
+}
+
+// Single-precision HVC(RA) part of one interval over the lane type V of ug_ra_f32.cuh:
+// thread t steps neuron t (V float) or neurons 2t and 2t + 1 (V f2).
+template <class V, class R, bool kTrack = false>
+__device__ __forceinline__ void interval_ra_v_body(const NetDev<R>& n, const BatchDev<R>& bt, int q, int s0, int s1,
+                                                   const RAStep<R>& rc, int t, int b)
+{
+    // t: the thread's first neuron / Lanes<V>::n (none when that is >= n_ra), b: its instance
+    static_assert(sizeof(R) == 4, "the lane-typed RA kernel is single precision");
+    typedef Lanes<V> L;
+    constexpr int N = L::n;
+    const int i0 = N * t;
+    uint32_t soma[N] = {}, dend[N] = {};
+    if (i0 < n.n_ra) {
+        // the lanes' neurons; a lane past the last neuron repeats its thread's first one and
+        // stores nothing
+        bool valid[N];
+        size_t x[N];
+        uint32_t ent[N];
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            valid[k] = i0 + k < n.n_ra;
+            ent[k] = (uint32_t)(valid[k] ? i0 + k : i0);
+            x[k] = (size_t)b * n.n_ra + ent[k];
         }
-        const RAPair P = ra_pair(make_float2(n.Erest[i0], n.Erest[v1 ? i1 : i0]),
-                                 make_float2(n.GCa[i0], n.GCa[v1 ? i1 : i0]),
-                                 (float)(100000.0 / RAConst::As) * rc.mu_s, (float)(100000.0 / RAConst::Ad) * rc.mu_d);
-        const int k0 = bt.kick_step[x0], k1 = v1 ? bt.kick_step[x1] : 0x7fffffff;
-        const StreamId sid0 = make_stream(n.seed, kNoiseRAWhite, n.net_id, (uint32_t)i0, bt.trial[b]);
-        const uint32_t ent1 = (uint32_t)(v1 ? i1 : i0);
-        for (int st = s0; st <= s1; ++st) {
-            if (st == k0) Ge.x = Ge.x + 3.0f;   // raiseE(G_TRAINING_KICK)
-            if (st == k1) Ge.y = Ge.y + 3.0f;
-            if constexpr (kTrack) {
-                trace_ra_row(bt, n.num_steps, b, i0, st, s.Vs.x, s.Vd.x, Ge.x, Gi.x);
-                if (v1) trace_ra_row(bt, n.num_steps, b, i1, st, s.Vs.y, s.Vd.y, Ge.y, Gi.y);
+        auto load = [&](const R* p) {
+            float v[N];
+#pragma unroll
+            for (int k = 0; k < N; ++k) v[k] = p[x[k]];
+            return L::make(v);
+        };
+        RAVec<V> s;
+        s.Vs = load(bt.ra[0]); s.Vd = load(bt.ra[1]); s.n = load(bt.ra[2]); s.h = load(bt.ra[3]);
+        s.l = load(bt.ra[4]); s.r = load(bt.ra[5]); s.c = load(bt.ra[6]); s.Ca = load(bt.ra[7]);
+        float ge[N], gi[N];
+        int fs[N], fd[N], kick[N];
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            ge[k] = bt.ra[8][x[k]];
+            gi[k] = bt.ra[9][x[k]];
+            const int fl = bt.ra_flags[x[k]];
+            fs[k] = fl & 1;
+            fd[k] = (fl >> 1) & 1;
+            kick[k] = valid[k] ? bt.kick_step[x[k]] : 0x7fffffff;
+        }
+        if (q > 0) {
+            // sync q-1: raiseI(sum Gi), raiseExcWeight(sum w) = Gexc_d += w / Ad
+            const size_t base = (size_t)((q - 1) % n.ring) * bt.B * n.n_ra;
+            long long ai[N], ae[N];
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+                ai[k] = valid[k] ? bt.ring_ra_inh[base + x[k]] : 0;
+                ae[k] = valid[k] ? bt.ring_ra_exc[base + x[k]] : 0;
             }
-            bool fs, fd;
-            RAState<float> c0, c1;
-            c0.Vs = s.Vs.x; c0.Vd = s.Vd.x; c1.Vs = s.Vs.y; c1.Vd = s.Vd.y;
-            ra_state_check(c0, fl0, fs, fd);
-            soma0 |= (uint32_t)fs << (st - s0);
-            dend0 |= (uint32_t)fd << (st - s0);
-            ra_state_check(c1, fl1, fs, fd);
-            soma1 |= (uint32_t)fs << (st - s0);
-            dend1 |= (uint32_t)fd << (st - s0);
-            const Philox4 w0 = philox_sched((uint32_t)(st - 1), sid0.entity, sid0.trial, sid0.tag, rc.ks);
-            const Philox4 w1 = philox_sched((uint32_t)(st - 1), ent1, sid0.trial, sid0.tag, rc.ks);
-            ra_debrabant_x2(s, Ge, Gi, P, rc, make_float2(ra_point_f(w0.x), ra_point_f(w1.x)),
-                            make_float2(ra_point_f(w0.y), ra_point_f(w1.y)), make_float2(ra_point_f(w0.z), ra_point_f(w1.z)),
-                            make_float2(ra_point_f(w0.w), ra_point_f(w1.w)));
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+                if (ai[k] | ae[k]) {
+                    bt.ring_ra_inh[base + x[k]] = 0;
+                    bt.ring_ra_exc[base + x[k]] = 0;
+                    gi[k] = gi[k] + (float)((double)ai[k] * kFixInv);
+                    ge[k] = ge[k] + (float)(((double)ae[k] * kFixInv) / RAConst::Ad);
+                }
+        }
+        V Ge = L::make(ge), Gi = L::make(gi);
+        const RACell<V> P = ra_cell<V>(load_param<V>(n.Erest, ent), load_param<V>(n.GCa, ent),
+                                       (float)(100000.0 / RAConst::As) * rc.mu_s,
+                                       (float)(100000.0 / RAConst::Ad) * rc.mu_d);
+        const float ns = rc.sq * rc.sig_s * (float)(1.0 / (RAConst::As * RAConst::cm));
+        const float nd = rc.sq * rc.sig_d * (float)(1.0 / (RAConst::Ad * RAConst::cm));
+        RANoiseStream<V> rng;
+        rng.init(ent, bt.trial[b], make_stream(n.seed, kNoiseRAWhite, n.net_id, 0, 0).tag, rc.ks);
+        for (int st = s0; st <= s1; ++st) {
+            add_kick(Ge, kick, st);   // raiseE(G_TRAINING_KICK)
+            if constexpr (kTrack) {
+#pragma unroll
+                for (int k = 0; k < N; ++k)
+                    if (valid[k])
+                        trace_ra_row(bt, n.num_steps, b, i0 + k, st, L::get(s.Vs, k), L::get(s.Vd, k), L::get(Ge, k),
+                                     L::get(Gi, k));
+            }
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+                ra_check_f(L::get(s.Vs, k), L::get(s.Vd, k), fs[k], fd[k], soma[k], dend[k], st - s0);
+            ra_debrabant_v(s, Ge, Gi, P, rc, rng.draw((uint32_t)st, ns, nd, rc.ks));
             if constexpr (kTrack) {   // inhibition tracking; a group may mix tracked and untracked members
                 if (bt.ginh_slot && bt.ginh_rec) {
                     const int sl = bt.ginh_slot[st];
                     if (sl > 0) {
                         R* rec = bt.ginh_rec + (size_t)sl * bt.B * n.n_ra;
-                        rec[x0] = Gi.x;
-                        if (v1) rec[x1] = Gi.y;
+#pragma unroll
+                        for (int k = 0; k < N; ++k)
+                            if (valid[k]) rec[x[k]] = L::get(Gi, k);
                     }
                 }
             }
         }
-        bt.ra[0][x0] = s.Vs.x; bt.ra[1][x0] = s.Vd.x; bt.ra[2][x0] = s.n.x; bt.ra[3][x0] = s.h.x; bt.ra[4][x0] = s.l.x;
-        bt.ra[5][x0] = s.r.x; bt.ra[6][x0] = s.c.x; bt.ra[7][x0] = s.Ca.x; bt.ra[8][x0] = Ge.x; bt.ra[9][x0] = Gi.x;
-        bt.ra_flags[x0] = fl0;
-        if (v1) {
-            bt.ra[0][x1] = s.Vs.y; bt.ra[1][x1] = s.Vd.y; bt.ra[2][x1] = s.n.y; bt.ra[3][x1] = s.h.y; bt.ra[4][x1] = s.l.y;
-            bt.ra[5][x1] = s.r.y; bt.ra[6][x1] = s.c.y; bt.ra[7][x1] = s.Ca.y; bt.ra[8][x1] = Ge.y; bt.ra[9][x1] = Gi.y;
-            bt.ra_flags[x1] = fl1;
-        } else {
-            soma1 = dend1 = 0;
-        }
-        for (int k = 0; k < 2; ++k) {
-            const uint32_t so = k ? soma1 : soma0, de = k ? dend1 : dend0;
-            const size_t x = k ? x1 : x0;
-            const int i = k ? i1 : i0;
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            if (!valid[k]) {
+                soma[k] = dend[k] = 0;
+                continue;
+            }
+            const size_t xk = x[k];
+            bt.ra[0][xk] = L::get(s.Vs, k); bt.ra[1][xk] = L::get(s.Vd, k); bt.ra[2][xk] = L::get(s.n, k);
+            bt.ra[3][xk] = L::get(s.h, k); bt.ra[4][xk] = L::get(s.l, k); bt.ra[5][xk] = L::get(s.r, k);
+            bt.ra[6][xk] = L::get(s.c, k); bt.ra[7][xk] = L::get(s.Ca, k); bt.ra[8][xk] = L::get(Ge, k);
+            bt.ra[9][xk] = L::get(Gi, k);
+            bt.ra_flags[xk] = fs[k] | fd[k] << 1;
+            const uint32_t so = soma[k], de = dend[k];
+            const int i = i0 + k;
             if (so) {
-                bt.ra_nsoma[x] += __popc(so);
-                if (bt.ra_first_soma[x] < 0) bt.ra_first_soma[x] = s0 + __ffs(so) - 1;
+                bt.ra_nsoma[xk] += __popc(so);
+                if (bt.ra_first_soma[xk] < 0) bt.ra_first_soma[xk] = s0 + __ffs(so) - 1;
                 record_spikes(bt.spk_count, bt.spk_buf, bt.spk_cap, bt.error, b, i, kSpikeSoma, so, s0);
             }
             if (de) {
-                bt.ra_ndend[x] += __popc(de);
-                if (bt.ra_first_dend[x] < 0) bt.ra_first_dend[x] = s0 + __ffs(de) - 1;
+                bt.ra_ndend[xk] += __popc(de);
+                if (bt.ra_first_dend[xk] < 0) bt.ra_first_dend[xk] = s0 + __ffs(de) - 1;
                 record_spikes(bt.spk_count, bt.spk_buf, bt.spk_cap, bt.error, b, i, kSpikeDend, de, s0);
             }
-            if (bt.soma_bits && (k == 0 || v1)) bt.soma_bits[(size_t)(q & 1) * bt.B * n.n_ra + x] = (int)so;
-            if (bt.act_rows && (k == 0 || v1)) queue_row(bt, q, (int)x, so);
+            if (bt.soma_bits) bt.soma_bits[(size_t)(q & 1) * bt.B * n.n_ra + xk] = (int)so;
+            if (bt.act_rows) queue_row(bt, q, (int)xk, so);
         }
     }
-    for (int k = 0; k < 2; ++k) {
-        const uint32_t so = k ? soma1 : soma0;
-        const int i = k ? i1 : i0;
-        scatter_warp(so, i, s0, n.T, n.num_steps, n.syncidx, n.ring, n.ra2i_off, n.ra2i_tgt, n.ra2i_wq, n.ra2i_d,
-                     bt.ring_i_exc, (size_t)bt.B * n.n_i, (size_t)b * n.n_i);
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        scatter_warp(soma[k], i0 + k, s0, n.T, n.num_steps, n.syncidx, n.ring, n.ra2i_off, n.ra2i_tgt, n.ra2i_wq,
+                     n.ra2i_d, bt.ring_i_exc, (size_t)bt.B * n.n_i, (size_t)b * n.n_i);
         if (bt.scatter_rara)
-            scatter_warp(so, i, s0, n.T, n.num_steps, n.syncidx, n.ring, n.rara_off, n.rara_tgt, n.rara_wq, n.rara_d,
-                         bt.ring_ra_exc, (size_t)bt.B * n.n_ra, (size_t)b * n.n_ra);
+            scatter_warp(soma[k], i0 + k, s0, n.T, n.num_steps, n.syncidx, n.ring, n.rara_off, n.rara_tgt, n.rara_wq,
+                         n.rara_d, bt.ring_ra_exc, (size_t)bt.B * n.n_ra, (size_t)b * n.n_ra);
     }
 }
 
@@ -584,7 +616,7 @@ __global__ void __launch_bounds__(kBlock, UG_RA_MIN_BLOCKS) k_interval_ra_x2(Net
 {
     int t, b;   // one flat grid over (instance, neuron pair)
     flat_unit(blockIdx.x * (unsigned)kBlock + threadIdx.x, (unsigned)(n.n_ra + 1) / 2u, bt.B, t, b);
-    interval_ra_x2_body<R, kTrack>(n, bt, q, s0, s1, rc, t, b);
+    interval_ra_v_body<f2, R, kTrack>(n, bt, q, s0, s1, rc, t, b);
 }
 
 // Single build: draws every Poisson noise event of the trial for each
@@ -715,7 +747,7 @@ __global__ void __launch_bounds__(kBlock, UG_RA_MIN_BLOCKS) k_interval_x(NetDev<
     int u, b;
     if (blockIdx.x < nb_ra) {
         flat_unit(blockIdx.x * (unsigned)kBlock + threadIdx.x, (unsigned)(n.n_ra + 1) / 2u, bt.B, u, b);
-        interval_ra_x2_body<R>(n, bt, q, s0, s1, rc, u, b);
+        interval_ra_v_body<f2, R>(n, bt, q, s0, s1, rc, u, b);
     } else {
         flat_unit((blockIdx.x - nb_ra) * (unsigned)kBlock + threadIdx.x, (unsigned)n.n_i, bt.B, u, b);
         interval_i_x_body<R>(n, bt, q, s0, s1, ic, u, b);
