@@ -667,6 +667,31 @@ __global__ void __launch_bounds__(kBlock) k_noise_events(NetDev<R> n, BatchDev<R
     noise_events_body(n, bt, (int)blockIdx.x, (int)blockIdx.y);
 }
 
+// The noise events of one channel of an interneuron (k_noise_events): the next one and the
+// one after it, which is loaded when its predecessor becomes the next, so that taking an
+// event waits for no memory.  A trial's list ends with an event that never comes.
+struct IEvents {
+    const int2* ev;
+    int cap, idx;
+    int2 cur, after;
+    template <class R>
+    __device__ __forceinline__ IEvents(const BatchDev<R>& bt, size_t x, int ch)
+        : ev(bt.i_events + (x * 2 + ch) * bt.ev_cap), cap(bt.ev_cap), idx(bt.i_ev_idx[2 * x + ch])
+    {
+        cur = ev[idx];
+        after = ev[min(idx + 1, cap - 1)];
+    }
+    // The next event's kick; moves to its successor.
+    __device__ __forceinline__ float take()
+    {
+        const float kick = __int_as_float(cur.y);
+        cur = after;
+        ++idx;
+        after = ev[min(idx + 1, cap - 1)];
+        return kick;
+    }
+};
+
 // Single-precision HVC(I) part of one interval: noise kicks from the pre-drawn
 // events, DP8 in the layout of ug_i_f32.cuh.
 template <class R, bool kTrack = false>
@@ -690,28 +715,19 @@ __device__ __forceinline__ void interval_i_x_body(const NetDev<R>& n, const Batc
                 s.Ge = s.Ge + (float)((double)ae * kFixInv);   // raiseE(sum w)
             }
         }
-        int ie = bt.i_ev_idx[2 * x], ii = bt.i_ev_idx[2 * x + 1];
-        const int2* eve = bt.i_events + (x * 2) * bt.ev_cap;
-        const int2* evi = bt.i_events + (x * 2 + 1) * bt.ev_cap;
-        int2 ne = eve[ie], ni = evi[ii];
+        IEvents ee(bt, x, 0), ei(bt, x, 1);
         int flag = bt.i_flag[x];
         for (int st = s0; st <= s1; ++st) {
             if constexpr (kTrack) trace_i_row(bt, n.num_steps, b, i, st, s.V, s.Ge, s.Gi);
-            if (i_state_check(s.V, flag)) fired_bits |= 1u << (st - s0);
-            if (st == ne.x) {
-                s.Ge += __int_as_float(ne.y);
-                ne = eve[++ie];
-            }
-            if (st == ni.x) {
-                s.Gi += __int_as_float(ni.y);
-                ni = evi[++ii];
-            }
+            i_check_f(s.V, flag, fired_bits, st - s0);
+            if (st == ee.cur.x) s.Ge += ee.take();
+            if (st == ei.cur.x) s.Gi += ei.take();
             i_dp8_x(s, ic);
         }
         bt.iv[0][x] = s.V; bt.iv[1][x] = s.n; bt.iv[2][x] = s.m; bt.iv[3][x] = s.h; bt.iv[4][x] = s.w;
         bt.iv[5][x] = s.Ge; bt.iv[6][x] = s.Gi;
-        bt.i_ev_idx[2 * x] = ie;
-        bt.i_ev_idx[2 * x + 1] = ii;
+        bt.i_ev_idx[2 * x] = ee.idx;
+        bt.i_ev_idx[2 * x + 1] = ei.idx;
         bt.i_flag[x] = flag;
         if (fired_bits) {
             bt.i_nspk[x] += __popc(fired_bits);
