@@ -70,14 +70,28 @@ __global__ void __launch_bounds__(kBlock) kl_trial_init(const GroupMember<R>* me
               [](const GroupMember<R>& m, int bx, int by) { trial_init_body(m.n, m.bt, bx, by); });
 }
 
+// items: (member, chunk of kNoiseThreads / 32 interneurons, b)
 template <class R>
-__global__ void __launch_bounds__(kBlock) kl_noise_events(const GroupMember<R>* members, const int4* items,
-                                                          const int* count)
+__global__ void __launch_bounds__(kNoiseThreads) kl_noise_gaps(const GroupMember<R>* members, const int4* items,
+                                                               const int* count)
 {
     __shared__ GroupMember<R> M;
     if constexpr (sizeof(R) == 4)
-        for_items(members, items, *count, M,
-                  [](const GroupMember<R>& m, int bx, int by) { noise_events_body(m.n, m.bt, bx, by); });
+        for_items(members, items, *count, M, [](const GroupMember<R>& m, int bx, int by) {
+            noise_gaps_body(m.n, m.bt, bx * (kNoiseThreads / 32) + (int)threadIdx.x / 32, by);
+        });
+}
+
+// items: (member, chunk of kNoiseWalk interneurons, b)
+template <class R>
+__global__ void __launch_bounds__(kNoiseWalk) kl_noise_events(const GroupMember<R>* members, const int4* items,
+                                                              const int* count)
+{
+    __shared__ GroupMember<R> M;
+    if constexpr (sizeof(R) == 4)
+        for_items(members, items, *count, M, [](const GroupMember<R>& m, int bx, int by) {
+            noise_events_body(m.n, m.bt, bx * kNoiseWalk + (int)threadIdx.x, by, m.n.num_steps - 1, false);
+        });
 }
 
 // act_cnt: the group's row-queue counters (null without growth members); the

@@ -287,7 +287,7 @@ private:
     int64_t batch_launches(const ug::LaunchCtx& lc) const
     {
         const int64_t per = ug::fused_interval<R>(nd_, bd_, lc) ? 1 : (h.n_i > 0 ? 2 : 1);
-        return per * ((int64_t)sync_steps.size() + 1) + 1 + (sizeof(R) == 4 && h.n_i > 0 ? 1 : 0);
+        return per * ((int64_t)sync_steps.size() + 1) + 1 + (sizeof(R) == 4 && h.n_i > 0 ? 2 : 0);
     }
     ug_status upload_connectivity(cudaStream_t st);
     ug_status growth_init(cudaStream_t st);
@@ -653,7 +653,10 @@ ug_status NetImpl<R>::ensure_batch(int B)
     b.ra_first_soma = ra_first_soma_.as<int>(); b.ra_first_dend = ra_first_dend_.as<int>();
     for (int k = 0; k < 7; ++k) b.iv[k] = iv_[k].as<R>();
     b.i_noise = i_noise_.as<double>(); b.i_noise_step = i_noise_step_.as<int>();
-    b.i_events = i_events_.as<int2>(); b.i_ev_idx = i_ev_idx_.as<int>(); b.ev_cap = ev_cap; b.i_word = i_word_.as<uint32_t>(); b.i_flag = i_flag_.as<int>();
+    b.i_events = i_events_.as<int2>(); b.i_ev_idx = i_ev_idx_.as<int>(); b.ev_cap = ev_cap;
+    // the intervals of the noise pre-pass share the inhibitory channel's list memory
+    b.i_gaps = reinterpret_cast<double*>(b.i_events + ev_cap); b.gap_stride = 2 * ev_cap; b.i_ev_cnt = nullptr;
+    b.i_word = i_word_.as<uint32_t>(); b.i_flag = i_flag_.as<int>();
     b.i_nspk = i_nspk_.as<int>(); b.i_first = i_first_.as<int>();
     b.ring_ra_exc = ring_ra_exc_.as<long long>(); b.ring_ra_inh = ring_ra_inh_.as<long long>();
     b.ring_i_exc = ring_i_exc_.as<long long>();
@@ -1059,7 +1062,7 @@ ug_status NetImpl<R>::issue_growth_trial(const ug::LaunchCtx& lc, int64_t* launc
 {
     int64_t cnt = 0;
     UG_CUDA(ug::launch_trial_init<R>(nd_, bd_, lc));
-    cnt += 1 + (sizeof(R) == 4 ? 1 : 0);
+    cnt += 1 + (sizeof(R) == 4 ? 2 : 0);
     UG_CUDA(ug::launch_growth_reset<R>(gd_, lc));
     ++cnt;
     const int Q = (int)sync_steps.size();
@@ -1118,7 +1121,7 @@ ug_status NetImpl<R>::run_growth_trials(uint32_t first_trial, int n_trials, int 
     uint32_t trial = first_trial;
     int left = n_trials;
     // kernels per trial: head, the trial (issue_growth_trial), check_bad_values, tail
-    const int64_t per_trial = 2 + (sizeof(R) == 4 ? 1 : 0) + 1 +
+    const int64_t per_trial = 2 + (sizeof(R) == 4 ? 2 : 0) + 1 +
                               (one_launch(lc) ? 1 : 5 * (int64_t)sync_steps.size() + 2) + 1 + 2;
     while (left > 0) {
         const int words[ug::kLoopWords] = {left, (int)trial, ug::kLoopRunning, 0};
@@ -1780,9 +1783,12 @@ ug_status GroupExec<R>::run_round(std::vector<RoundItem<R>>& items, const ug::La
         for (int b = 0; b < B; ++b) {
             for (int x = 0; x < nb_ra + nb_i; ++x) hitems_[ug::kListInit].push_back(make_int4(m, x, b, 0));
             for (int x = 0; x < nb_int; ++x) hitems_[ug::kListRA].push_back(make_int4(m, x, b, 0));
-            for (int x = 0; x < nb_i; ++x) {
-                hitems_[ug::kListI].push_back(make_int4(m, x, b, 0));
-                if (sizeof(R) == 4) hitems_[ug::kListNoise].push_back(make_int4(m, x, b, 0));
+            for (int x = 0; x < nb_i; ++x) hitems_[ug::kListI].push_back(make_int4(m, x, b, 0));
+            if (sizeof(R) == 4) {
+                const int per = ug::kNoiseThreads / 32;
+                for (int x = 0; x < (ni + per - 1) / per; ++x) hitems_[ug::kListGaps].push_back(make_int4(m, x, b, 0));
+                for (int x = 0; x < (ni + ug::kNoiseWalk - 1) / ug::kNoiseWalk; ++x)
+                    hitems_[ug::kListNoise].push_back(make_int4(m, x, b, 0));
             }
         }
         const int nchk = (int)(((size_t)B * nra + 255) / 256);
@@ -1824,7 +1830,7 @@ ug_status GroupExec<R>::run_round(std::vector<RoundItem<R>>& items, const ug::La
     // launch: one captured graph per kind (with or without growth members, with or
     // without inhibition tracking), reused across compositions
     const int64_t Q = (int64_t)sync_steps.size();
-    const int64_t n_launch = 2 + (sizeof(R) == 4 ? 1 : 0) + 2 * (Q + 1) + (growth ? 4 * Q + 2 : 0);
+    const int64_t n_launch = 2 + (sizeof(R) == 4 ? 2 : 0) + 2 * (Q + 1) + (growth ? 4 * Q + 2 : 0);
     if (!graphs || lc.timer) {
         UG_CUDA(ug::launch_group_trial<R>(dev_, sync_steps, num_steps, growth, lc, nullptr));
     } else {
@@ -2856,6 +2862,8 @@ extern "C" ug_status ug_run_test_trial_noalloc(ug_ctx* ctx, int32_t net_id, uint
     b.i_events = c.take<int2>(2 * (size_t)ni * ev_cap);
     b.i_ev_idx = c.take<int>(2 * (size_t)ni);
     b.ev_cap = ev_cap;
+    b.i_gaps = reinterpret_cast<double*>(b.i_events + ev_cap);   // as the batched path
+    b.gap_stride = 2 * ev_cap;
     b.i_word = c.take<uint32_t>(ni);
     b.i_flag = c.take<int>(ni);
     b.i_nspk = c.take<int>(ni);
@@ -2903,7 +2911,7 @@ extern "C" ug_status ug_run_test_trial_noalloc(ug_ctx* ctx, int32_t net_id, uint
         UG_CUDA(ug::launch_interval<float>(nd, b, q, s0, ss[q], rc, ic, lc));
     }
     UG_CUDA(ug::launch_interval<float>(nd, b, Q, nd.num_steps, nd.num_steps - 1, rc, ic, lc));
-    ctx->launches += 2 * ((int64_t)Q + 1) + 3;
+    ctx->launches += 2 * ((int64_t)Q + 1) + 4;
     const size_t ra_bytes = (size_t)nra * sizeof(int), i_bytes = (size_t)ni * sizeof(int);
     UG_CUDA(cudaMemcpyAsync(soma_count, b.ra_nsoma, ra_bytes, cudaMemcpyDeviceToDevice, lc.main));
     UG_CUDA(cudaMemcpyAsync(soma_first, b.ra_first_soma, ra_bytes, cudaMemcpyDeviceToDevice, lc.main));

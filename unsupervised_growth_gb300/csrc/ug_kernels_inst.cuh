@@ -23,7 +23,10 @@ inline void launch_noise_events(const NetDev<float>& n, const BatchDev<float>& b
 {
     if (n.n_i == 0) return;
     if (lc.timer) lc.timer->begin("k_noise_events", lc.main);
-    k_noise_events<float><<<dim3((n.n_i + kBlock - 1) / kBlock, b.B), kBlock, 0, lc.main>>>(n, b);
+    constexpr int kPer = kNoiseThreads / 32;
+    k_noise_gaps<float><<<dim3((n.n_i + kPer - 1) / kPer, b.B), kNoiseThreads, 0, lc.main>>>(n, b);
+    k_noise_events<float><<<dim3((n.n_i + kNoiseWalk - 1) / kNoiseWalk, b.B), kNoiseWalk, 0, lc.main>>>(
+        n, b, n.num_steps - 1, false);
     if (lc.timer) lc.timer->end(lc.main);
 }
 
@@ -301,7 +304,8 @@ cudaError_t group_grids(GroupDev& d, int ra_blocks_per_sm, int i_blocks_per_sm)
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
     d.grid[kListInit] = occupancy(kl_trial_init<R>, kBlock, 0);
-    d.grid[kListNoise] = occupancy(kl_noise_events<R>, kBlock, 0);
+    d.grid[kListGaps] = occupancy(kl_noise_gaps<R>, kNoiseThreads, 0);
+    d.grid[kListNoise] = occupancy(kl_noise_events<R>, kNoiseWalk, 0);
     d.grid[kListRA] = occupancy(kl_interval_ra<R>, kBlock, 0);
     d.grid[kListI] = occupancy(kl_interval_i<R>, kBlock, 0);
     if (ra_blocks_per_sm > 0) d.grid[kListRA] = std::min(d.grid[kListRA], ra_blocks_per_sm * sms);
@@ -337,8 +341,9 @@ cudaError_t launch_group_trial(const GroupDev& d, const std::vector<int>& sync_s
     UG_TIMED(lc, "k_trial_init", (kl_trial_init<R><<<d.grid[kListInit], kBlock, 0, lc.main>>>(mem, d.items[kListInit], c + kListInit)));
     ++cnt;
     if constexpr (sizeof(R) == 4) {
-        UG_TIMED(lc, "k_noise_events", (kl_noise_events<R><<<d.grid[kListNoise], kBlock, 0, lc.main>>>(mem, d.items[kListNoise], c + kListNoise)));
-        ++cnt;
+        UG_TIMED(lc, "k_noise_events", (kl_noise_gaps<R><<<d.grid[kListGaps], kNoiseThreads, 0, lc.main>>>(mem, d.items[kListGaps], c + kListGaps)));
+        UG_TIMED(lc, "k_noise_events", (kl_noise_events<R><<<d.grid[kListNoise], kNoiseWalk, 0, lc.main>>>(mem, d.items[kListNoise], c + kListNoise)));
+        cnt += 2;
     }
     if (growth) {
         UG_TIMED(lc, "k_growth_reset", (kl_growth_reset<R><<<d.grid[kListReset], 256, 0, lc.main>>>(mem, d.items[kListReset], c + kListReset)));

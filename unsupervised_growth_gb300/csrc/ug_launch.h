@@ -162,7 +162,7 @@ cudaError_t launch_growth_tail(const TailDev<R>& t, cudaStream_t st);
 
 // Group launches (ug_group.cuh): the work lists and row queue of a group, in
 // device memory, and the fixed grid of each list kernel.
-enum GroupList { kListInit = 0, kListNoise, kListRA, kListI, kListReset, kListNewpost, kListLtp, kListCheck, kNumLists };
+enum GroupList { kListInit = 0, kListGaps, kListNoise, kListRA, kListI, kListReset, kListNewpost, kListLtp, kListCheck, kNumLists };
 struct GroupDev {
     const void* members = nullptr;            // GroupMember<R>[members]
     const int4* items[kNumLists] = {};

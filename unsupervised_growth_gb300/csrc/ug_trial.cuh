@@ -74,6 +74,9 @@ struct BatchDev {
     int2* i_events;            // [B][n_i][2][ev_cap] (step, float kick) noise events (single build)
     int* i_ev_idx;             // [B][n_i][2] next unapplied event
     int ev_cap;
+    double* i_gaps;            // [B][n_i][ev_cap] noise intervals drawn ahead, gap_stride doubles per neuron:
+    int gap_stride;            // the interval of stream word w at w / 2 (k_noise_gaps); may share i_events
+    int* i_ev_cnt;             // [B][n_i][2] events listed so far, for a list drawn in segments; or null
     uint32_t* i_word;          // [B][n_i] words consumed from the neuron's stream
     int* i_flag; int* i_nspk; int* i_first;
     long long* ring_ra_exc;    // [ring][B][n_ra]
@@ -149,9 +152,16 @@ __device__ __forceinline__ int deliver_step(const double* T, int num_steps, int 
     const double td = T[s] + d;
     int k = (int)(d * 50.0) - 2;
     if (k < 0) k = 0;
-    int s2 = s + k;
-    while (s2 < num_steps && T[s2] < td) ++s2;
-    return s2;
+    // four steps of the rising grid per pass, their loads together: the answer is nearly always among the first
+    for (int s2 = s + k; s2 < num_steps; s2 += 4) {
+        bool before[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) before[j] = T[min(s2 + j, num_steps - 1)] < td;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (s2 + j >= num_steps || !before[j]) return s2 + j < num_steps ? s2 + j : num_steps;
+    }
+    return num_steps;
 }
 
 __device__ __forceinline__ void record_spikes(int* spk_count, int2* spk_buf, int cap, int* error, int b, int neuron,
@@ -243,8 +253,15 @@ __device__ __forceinline__ int first_step_after(const double* T, int num_steps, 
     int s = (int)(x * 50.0);
     if (s < s_from) s = s_from;
     if (s < 1) s = 1;
-    while (s < num_steps && !(T[s - 1] > x)) ++s;
-    return s;
+    for (; s < num_steps; s += 4) {   // loads as in deliver_step
+        bool past[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) past[j] = T[min(s + j, num_steps) - 1] > x;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (s + j >= num_steps || past[j]) return s + j < num_steps ? s + j : num_steps;
+    }
+    return num_steps;
 }
 
 // Poisson noise event of one interneuron channel (HHI_buffer::noise_check,
@@ -619,67 +636,172 @@ __global__ void __launch_bounds__(kBlock, UG_RA_MIN_BLOCKS) k_interval_ra_x2(Net
     interval_ra_v_body<f2, R, kTrack>(n, bt, q, s0, s1, rc, t, b);
 }
 
-// Single build: draws every Poisson noise event of the trial for each
-// interneuron of each instance (HHI_buffer::noise_check, HHI_buffer.cpp:278-294,
-// called as exc then inh every step, HHI_buffer.cpp:248-258).  Runs once per
-// batch after k_trial_init; the double-precision work of the noise lives here.
+// Single build: draws every Poisson noise event of the trial for each interneuron of each
+// instance (HHI_buffer::noise_check, HHI_buffer.cpp:278-294, called as exc then inh every
+// step, HHI_buffer.cpp:248-258) before the trial is integrated; the double-precision work
+// of the noise lives here.  Two passes after k_trial_init:
+//  * k_noise_gaps: the logarithm of every stream word that is an interval, a warp per
+//    neuron.  A neuron's words alternate kick, interval (a retry takes an interval and a
+//    kick more, which keeps the parity), so the intervals are the words of one parity.
+//    Bound by the FP64 pipe (a logarithm is some forty operations on it).
+//  * k_noise_events: a thread per neuron walks its intervals in order, which decides which
+//    channel takes which words, and lists the events.
+// In one pass, with the logarithm inside the walk, a trial's draw took 1.2 ms (a chain of
+// about 250 logarithms, 10 000 cycles an event), and 27.4 ms for 1024 trials of 550; in two
+// 0.32 and 14.8 ms.
+constexpr int kNoiseThreads = 128;   // k_noise_gaps: four neurons (warps) per block
+constexpr int kNoiseWalk = 32;       // k_noise_events: threads per block
+constexpr long long kTimestepBits = 0x3f947ae147ae147b;   // 0.02
+constexpr int kEvSegmentEnd = 0x7ffffffe, kEvTrialEnd = 0x7fffffff;   // steps that never come
+
 template <class R>
-__device__ __forceinline__ void noise_events_body(const NetDev<R>& n, const BatchDev<R>& bt, int bx, int b)
+__device__ __forceinline__ void noise_gaps_body(const NetDev<R>& n, const BatchDev<R>& bt, int i, int b)
 {
     static_assert(sizeof(R) == 4, "the noise pre-pass serves the single-precision build");
-    const int i = bx * kBlock + threadIdx.x;
+    if (i >= n.n_i) return;   // one neuron per warp
+    const size_t x = (size_t)b * n.n_i + i;
+    const StreamId sid = make_stream(n.seed, kNoiseIPoisson, n.net_id, (uint32_t)i, bt.trial[b]);
+    const uint32_t odd = (bt.i_word[x] + 1u) & 1u;   // parity of the interval words
+    double* gaps = bt.i_gaps + x * bt.gap_stride;
+    // the interval of word w; one below the time step is drawn again (0.5 % of them) from
+    // word w + 1: then minus that interval, unless it is too short as well
+    auto interval = [&](uint32_t u, uint32_t w) {
+        const double r = i_noise_interval_fast(u);
+        if (r >= 0.02) return r;
+        const double again = i_noise_interval_fast(stream_word(sid, w + 1));
+        return again >= 0.02 ? -again : fabs(r);
+    };
+    for (int j = threadIdx.x & 31; 2 * j < bt.ev_cap; j += 32) {
+        const Philox4 w = stream_block(sid, (uint32_t)j);
+        gaps[2 * j] = interval(odd ? w.y : w.x, 4u * j + odd);
+        if (2 * j + 1 < bt.ev_cap) gaps[2 * j + 1] = interval(odd ? w.w : w.z, 4u * j + 2u + odd);
+    }
+}
+
+template <class R>
+__global__ void __launch_bounds__(kNoiseThreads) k_noise_gaps(NetDev<R> n, BatchDev<R> bt)
+{
+    noise_gaps_body(n, bt, (int)(blockIdx.x * (kNoiseThreads / 32) + threadIdx.x / 32), (int)blockIdx.y);
+}
+
+// first_step_after for the walk below: x > 0.02, s_from >= 1.  A double-precision operation
+// costs a lone warp 64 cycles, so the comparisons are of bit patterns (positive doubles order
+// as integers) and the first guess, rounded down, is taken from x's upper bits.
+__device__ __forceinline__ int noise_step_after(const double* T, int num_steps, double x, int s_from)
+{
+    const long long xb = __double_as_longlong(x);
+    const float xf = __int_as_float((int)((xb - (896ll << 52)) >> 29));   // x truncated to single precision
+    if (!(xf < 1.0e5f)) return first_step_after(T, num_steps, x, s_from);   // the guess could overshoot
+    int s = max((int)(xf * 50.0f) - 1, s_from);
+    for (; s < num_steps; s += 4) {
+        bool past[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) past[j] = __double_as_longlong(T[min(s + j, num_steps) - 1]) > xb;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (s + j >= num_steps || past[j]) return s + j < num_steps ? s + j : num_steps;
+    }
+    return num_steps;
+}
+
+// Lists the events of steps up to `end`; `resume`: after the ones an earlier call listed, for
+// which the lists' counts are kept in i_ev_cnt.  The interval of a word lies in the list
+// memory of the inhibitory channel when i_gaps shares it: word w >= 3 at w / 2, so event k
+// reads slot k + 1 or a later one, and writes at slot k or an earlier one.
+template <class R>
+__device__ __forceinline__ void noise_events_body(const NetDev<R>& n, const BatchDev<R>& bt, int i, int b, int end,
+                                                  bool resume)
+{
+    static_assert(sizeof(R) == 4, "the noise pre-pass serves the single-precision build");
     if (i >= n.n_i) return;
     const size_t x = (size_t)b * n.n_i + i;
     const StreamId sid = make_stream(n.seed, kNoiseIPoisson, n.net_id, (uint32_t)i, bt.trial[b]);
     uint32_t word = bt.i_word[x];
     double nt[2] = {bt.i_noise[2 * x], bt.i_noise[2 * x + 1]};
     int ns[2] = {bt.i_noise_step[2 * x], bt.i_noise_step[2 * x + 1]};
-    int cnt[2] = {0, 0};
+    // a resumed list goes on behind the mark its last segment ended with
+    int cnt[2] = {resume ? bt.i_ev_cnt[2 * x] + 1 : 0, resume ? bt.i_ev_cnt[2 * x + 1] + 1 : 0};
     int2* out[2] = {bt.i_events + (x * 2) * bt.ev_cap, bt.i_events + (x * 2 + 1) * bt.ev_cap};
+    const double* gaps = bt.i_gaps + x * bt.gap_stride;
     const float gscale = (float)(IConst::G_noise / 4294967295.0);
+    auto gap = [&](uint32_t w) {
+        return (int)(w >> 1) < bt.ev_cap ? gaps[w >> 1] : i_noise_interval_fast(stream_word(sid, w));
+    };
+    double next = gap(word + 1);   // read one event ahead
     while (true) {
-        const int st = ns[0] < ns[1] ? ns[0] : ns[1];
-        if (st >= n.num_steps) break;
-#pragma unroll
-        for (int ch = 0; ch < 2; ++ch) {
-            if (ns[ch] != st) continue;
-            float dG = gscale * (float)stream_word(sid, word++);
-            double rnd = i_noise_interval_fast(stream_word(sid, word++));
-            while (rnd < 0.02) {
-                rnd = i_noise_interval_fast(stream_word(sid, word++));
-                dG += gscale * (float)stream_word(sid, word++);
+        // the channel whose noise time is passed first, exc before inh within a step
+        const bool inh = ns[1] < ns[0];
+        const int st = inh ? ns[1] : ns[0];
+        if (st > end || st >= n.num_steps) break;
+        float dG = gscale * (float)stream_word(sid, word);
+        word += 2;
+        double rnd = next;
+        if (__double_as_longlong(rnd) < kTimestepBits) {   // drawn again, or (negative) already resolved
+            if (rnd < 0.0) {
+                rnd = -rnd;
+                dG = __fmaf_rn(gscale, (float)stream_word(sid, word + 1), dG);
+                word += 2;
+            } else {
+                while (rnd < 0.02) {   // a retry's interval is a word of the kicks' parity
+                    rnd = i_noise_interval_fast(stream_word(sid, word));
+                    dG = __fmaf_rn(gscale, (float)stream_word(sid, word + 1), dG);
+                    word += 2;
+                }
             }
-            nt[ch] = nt[ch] + rnd;
-            if (cnt[ch] < bt.ev_cap - 1) out[ch][cnt[ch]++] = make_int2(st, __float_as_int(dG));
-            else atomicOr(bt.error, kErrEventCapacity);
-            ns[ch] = first_step_after(n.T, n.num_steps, nt[ch], st + 1);
+        }
+        next = gap(word + 1);
+        const double t = (inh ? nt[1] : nt[0]) + rnd;
+        const int s = noise_step_after(n.T, n.num_steps, t, st + 1);
+        int& c = inh ? cnt[1] : cnt[0];
+        if (c < bt.ev_cap - 1) (inh ? out[1] : out[0])[c++] = make_int2(st, __float_as_int(dG));
+        else atomicOr(bt.error, kErrEventCapacity);
+        if (inh) {
+            nt[1] = t;
+            ns[1] = s;
+        } else {
+            nt[0] = t;
+            ns[0] = s;
         }
     }
-    out[0][cnt[0]] = make_int2(0x7fffffff, 0);
-    out[1][cnt[1]] = make_int2(0x7fffffff, 0);
-    bt.i_ev_idx[2 * x] = 0;
-    bt.i_ev_idx[2 * x + 1] = 0;
+    const int mark = end >= n.num_steps - 1 ? kEvTrialEnd : kEvSegmentEnd;
+    out[0][cnt[0]] = make_int2(mark, 0);
+    out[1][cnt[1]] = make_int2(mark, 0);
+    if (!resume) {
+        bt.i_ev_idx[2 * x] = 0;
+        bt.i_ev_idx[2 * x + 1] = 0;
+    }
+    if (mark == kEvSegmentEnd) {
+        bt.i_word[x] = word;
+        for (int ch = 0; ch < 2; ++ch) {
+            bt.i_noise[2 * x + ch] = nt[ch];
+            bt.i_noise_step[2 * x + ch] = ns[ch];
+            bt.i_ev_cnt[2 * x + ch] = cnt[ch];
+        }
+    }
 }
 
 template <class R>
-__global__ void __launch_bounds__(kBlock) k_noise_events(NetDev<R> n, BatchDev<R> bt)
+__global__ void __launch_bounds__(kNoiseWalk) k_noise_events(NetDev<R> n, BatchDev<R> bt, int end, bool resume)
 {
-    noise_events_body(n, bt, (int)blockIdx.x, (int)blockIdx.y);
+    noise_events_body(n, bt, (int)(blockIdx.x * kNoiseWalk + threadIdx.x), (int)blockIdx.y, end, resume);
 }
 
 // The noise events of one channel of an interneuron (k_noise_events): the next one and the
 // one after it, which is loaded when its predecessor becomes the next, so that taking an
-// event waits for no memory.  A trial's list ends with an event that never comes.
+// event waits for no memory.  A list, and each of its segments, ends with a mark whose step
+// never comes; nothing behind the mark is read until the next segment's first interval.
 struct IEvents {
     const int2* ev;
-    int cap, idx;
+    int idx;
     int2 cur, after;
     template <class R>
     __device__ __forceinline__ IEvents(const BatchDev<R>& bt, size_t x, int ch)
-        : ev(bt.i_events + (x * 2 + ch) * bt.ev_cap), cap(bt.ev_cap), idx(bt.i_ev_idx[2 * x + ch])
+        : ev(bt.i_events + (x * 2 + ch) * bt.ev_cap), idx(bt.i_ev_idx[2 * x + ch])
     {
         cur = ev[idx];
-        after = ev[min(idx + 1, cap - 1)];
+        if (cur.x == kEvSegmentEnd) cur = ev[++idx];
+        after = cur;
+        if (cur.x < kEvSegmentEnd) after = ev[idx + 1];
     }
     // The next event's kick; moves to its successor.
     __device__ __forceinline__ float take()
@@ -687,7 +809,7 @@ struct IEvents {
         const float kick = __int_as_float(cur.y);
         cur = after;
         ++idx;
-        after = ev[min(idx + 1, cap - 1)];
+        if (cur.x < kEvSegmentEnd) after = ev[idx + 1];
         return kick;
     }
 };
