@@ -170,14 +170,16 @@ ug_status ug_set_growth_launch(ug_ctx* ctx, int32_t one_launch);
  * Results are the same bits for every shape; a shape whose blocks cannot all be resident
  * runs the per-interval launches.  UG_EINVAL for other widths. */
 ug_status ug_set_growth_trial_shape(ug_ctx* ctx, int32_t ra_threads, int32_t i_threads);
-/* Launch shape of test batches in the single-precision build, no counterpart in the
- * reference (whose ranks step every neuron in one loop, NetworkGrowthSimulator.cpp:12820-12835).
- * fuse 1 (the default): batches of 16 trials or more run the HVC(RA) and HVC(I) integration of
- * each sync interval in one kernel launch, the interneuron blocks after the RA blocks, so
- * they fill the SMs the RA part's last wave leaves idle; 0: two launches per interval
- * (per-kernel timing then reports k_interval_ra and k_interval_i apart; fused, the one
- * kernel is k_interval_x).  Recording and inhibition tracking always use two launches.
- * Results are the same bits either way. */
+/* Launch shape of test batches in the single-precision build, no counterpart in the reference
+ * (whose ranks step every neuron in one loop, NetworkGrowthSimulator.cpp:12820-12835).
+ * fuse 1 (the default): batches whose neurons can all be resident at once run the whole trial
+ * in one cooperative launch, in which a wait not satisfied within about a second ends the
+ * batch with UG_ETIMEOUT; larger ones (of 16 trials or more) run the HVC(RA) and HVC(I)
+ * integration of each sync interval in one kernel launch, the interneuron blocks after the RA
+ * blocks, so they fill the SMs the RA part's last wave leaves idle; 0: two launches per
+ * interval (per-kernel timing, which never uses the one cooperative launch, then reports
+ * k_interval_ra and k_interval_i apart; fused, the one kernel is k_interval_x).  Recording
+ * always uses two launches per interval.  Results are the same bits either way. */
 ug_status ug_set_interval_fusion(ug_ctx* ctx, int32_t fuse);
 /* Serving loop -- no counterpart in the reference.  A scheduler thread of the context
  * runs group rounds (see ug_run_group) over the requests on the GPU and, between

@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(kNoiseThreads) kl_noise_gaps(const GroupMember
     __shared__ GroupMember<R> M;
     if constexpr (sizeof(R) == 4)
         for_items(members, items, *count, M, [](const GroupMember<R>& m, int bx, int by) {
-            noise_gaps_body(m.n, m.bt, bx * (kNoiseThreads / 32) + (int)threadIdx.x / 32, by);
+            noise_gaps_body(m.n, m.bt, bx * (kNoiseThreads / 32) + (int)threadIdx.x / 32, by, 0, m.bt.ev_cap);
         });
 }
 
@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(kNoiseWalk) kl_noise_events(const GroupMember<
     __shared__ GroupMember<R> M;
     if constexpr (sizeof(R) == 4)
         for_items(members, items, *count, M, [](const GroupMember<R>& m, int bx, int by) {
-            noise_events_body(m.n, m.bt, bx * kNoiseWalk + (int)threadIdx.x, by, m.n.num_steps - 1, false);
+            noise_events_body(m.n, m.bt, bx * kNoiseWalk + (int)threadIdx.x, by, m.n.num_steps - 1, m.bt.ev_cap, false);
         });
 }
 

@@ -282,13 +282,42 @@ private:
     ug_status ensure_batch(int B);
     ug_status check_error(cudaStream_t st);
     ug_status issue_batch(const ug::LaunchCtx& lc, int64_t* launches);
-    // kernels of one test batch: initialisation (and the noise events), then one launch
-    // per sync interval and integrator, or one per interval when they are fused
+    // kernels of one test batch: initialisation and the two noise passes, then the trial in
+    // one launch (test_plan_) or one launch per sync interval and integrator, or one per
+    // interval when they are fused
     int64_t batch_launches(const ug::LaunchCtx& lc) const
     {
+        const int64_t noise = sizeof(R) == 4 && h.n_i > 0 ? 2 : 0;
+        if (test_plan_.lanes > 0) return segmented() ? 1 + 2 * noise + 2 : 1 + noise + 1;
         const int64_t per = ug::fused_interval<R>(nd_, bd_, lc) ? 1 : (h.n_i > 0 ? 2 : 1);
-        return per * ((int64_t)sync_steps.size() + 1) + 1 + (sizeof(R) == 4 && h.n_i > 0 ? 2 : 0);
+        return per * ((int64_t)sync_steps.size() + 1) + 1 + noise;
     }
+    // The one-launch form of the current batch.  Small batches integrate a first part of the
+    // trial while the noise of the rest is drawn beside it (they leave SMs idle); larger ones
+    // gain nothing from that.
+    ug::TestPlan test_plan_;
+    static constexpr int kSegmentBatch = 15;
+    bool segmented() const { return bd_.B <= kSegmentBatch && sync_steps.size() >= 64; }
+    // Where the noise pre-pass keeps its intervals: in the inhibitory channel's list memory,
+    // or, for lists drawn in segments, in an array of their own.
+    void share_gaps()
+    {
+        bd_.i_gaps = reinterpret_cast<double*>(bd_.i_events + bd_.ev_cap);
+        bd_.gap_stride = 2 * bd_.ev_cap;
+    }
+    void own_gaps()
+    {
+        bd_.i_gaps = i_gaps_.as<double>();
+        bd_.gap_stride = bd_.ev_cap;
+    }
+    ug_status plan_batch(const ug::LaunchCtx& lc)
+    {
+        test_plan_ = ug::TestPlan();
+        if (sizeof(R) == 4 && lc.fuse && !lc.timer && !bd_.trace_ra && !bd_.trace_i && !sync_steps.empty())
+            UG_CUDA(ug::test_trial_plan<R>(h.n_ra, h.n_i, bd_.B, &test_plan_));
+        return UG_OK;
+    }
+    ug_status issue_test_trial(const ug::LaunchCtx& lc);
     ug_status upload_connectivity(cudaStream_t st);
     ug_status growth_init(cudaStream_t st);
     ug_status issue_growth_trial(const ug::LaunchCtx& lc, int64_t* launches);
@@ -308,11 +337,11 @@ private:
     int spike_cap_per_neuron_ = 16;
     int B_ = 0;            // instances in the last batch
     int B_cap_ = 0;        // allocated instances
-    DevMem dT_, dSyncidx_, dRaDecay_, dIDecay_, dErest_, dGCa_, dSpread_, dTraining_;
+    DevMem dT_, dSyncidx_, dSyncEnd_, dRaDecay_, dIDecay_, dErest_, dGCa_, dSpread_, dTraining_;
     CsrDev ra2i_, i2ra_, rara_;
     DevMem ra_[10], ra_flags_, kick_step_, ra_nsoma_, ra_ndend_, ra_first_soma_, ra_first_dend_;
-    DevMem iv_[7], i_noise_, i_noise_step_, i_events_, i_ev_idx_, i_word_, i_flag_, i_nspk_, i_first_;
-    DevMem ring_ra_exc_, ring_ra_inh_, ring_i_exc_, spk_buf_, spk_count_, error_, trial_, mean_inj_;
+    DevMem iv_[7], i_noise_, i_noise_step_, i_events_, i_ev_idx_, i_ev_cnt_, i_gaps_, i_word_, i_flag_, i_nspk_, i_first_;
+    DevMem ring_ra_exc_, ring_ra_inh_, ring_i_exc_, spk_buf_, spk_count_, error_, trial_, mean_inj_, test_ctl_;
     cudaGraphExec_t graph_exec_ = nullptr;
     int graph_B_ = -1;
     int graph_fuse_ = -1;          // the fusion setting the test-batch graph was captured with
@@ -331,7 +360,7 @@ private:
     ug::TailDev<R> td_{};
     bool book_dirty_ = false;      // the device bookkeeping changed since the host copy was read
     // the one-launch growth trial (ug_growth_trial.cuh)
-    DevMem gTrialCtl_, gActRows_, gSyncEnd_;   // barrier and queue words, row queue, sync steps
+    DevMem gTrialCtl_, gActRows_;  // barrier and queue words, row queue
     bool trial_fits_ = false;      // every sync interval fits the trial's segment buffers
     int trial_key_ = -1;           // the launch mode and role widths trial_blocks_ was sized for
     int trial_blocks_ = 0;         // its grid (0: the network's blocks cannot all be resident)
@@ -541,6 +570,7 @@ ug_status NetImpl<R>::init_device(cudaStream_t st)
     const int NRA = H.n_ra, NI = H.n_i;
     UG_TRY(dT_.upload(T, st));
     UG_TRY(dSyncidx_.upload(syncidx_, st));
+    UG_TRY(dSyncEnd_.upload(sync_steps, st));
     if (sizeof(R) == 8) {   // per-step decay tables: the double build only
         UG_TRY(dRaDecay_.upload(ra_decay_, st));
         UG_TRY(dIDecay_.upload(i_decay_, st));
@@ -633,9 +663,13 @@ ug_status NetImpl<R>::ensure_batch(int B)
     UG_TRY(i_noise_.alloc(2 * ni * sizeof(double)));
     UG_TRY(i_noise_step_.alloc(2 * ni * sizeof(int)));
     // noise events per interneuron channel and trial: 250 Hz on average (HHI_buffer.cpp:37)
-    const int ev_cap = sizeof(R) == 4 ? (int)(h.num_steps * 0.02 * 0.25 * 2.0) + 64 : 1;
+    // (and the mark between the two segments of a small batch's lists)
+    const int ev_cap = sizeof(R) == 4 ? (int)(h.num_steps * 0.02 * 0.25 * 2.0) + 65 : 1;
     UG_TRY(i_events_.alloc(2 * ni * (size_t)ev_cap * sizeof(int2)));
     UG_TRY(i_ev_idx_.alloc(2 * ni * sizeof(int)));
+    UG_TRY(i_ev_cnt_.alloc(2 * ni * sizeof(int)));
+    UG_TRY(i_gaps_.alloc((size_t)std::min(B, kSegmentBatch) * h.n_i * ev_cap * sizeof(double)));   // segmented lists
+    UG_TRY(test_ctl_.alloc((size_t)B * ug::kCtlWords * sizeof(unsigned)));
     for (DevMem* m : {&i_word_, &i_flag_, &i_nspk_, &i_first_}) UG_TRY(m->alloc(ni * sizeof(int)));
     UG_TRY(ring_ra_exc_.alloc((size_t)ring * nra * sizeof(long long)));
     UG_TRY(ring_ra_inh_.alloc((size_t)ring * nra * sizeof(long long)));
@@ -654,8 +688,8 @@ ug_status NetImpl<R>::ensure_batch(int B)
     for (int k = 0; k < 7; ++k) b.iv[k] = iv_[k].as<R>();
     b.i_noise = i_noise_.as<double>(); b.i_noise_step = i_noise_step_.as<int>();
     b.i_events = i_events_.as<int2>(); b.i_ev_idx = i_ev_idx_.as<int>(); b.ev_cap = ev_cap;
-    // the intervals of the noise pre-pass share the inhibitory channel's list memory
-    b.i_gaps = reinterpret_cast<double*>(b.i_events + ev_cap); b.gap_stride = 2 * ev_cap; b.i_ev_cnt = nullptr;
+    share_gaps();
+    b.i_ev_cnt = i_ev_cnt_.as<int>();
     b.i_word = i_word_.as<uint32_t>(); b.i_flag = i_flag_.as<int>();
     b.i_nspk = i_nspk_.as<int>(); b.i_first = i_first_.as<int>();
     b.ring_ra_exc = ring_ra_exc_.as<long long>(); b.ring_ra_inh = ring_ra_inh_.as<long long>();
@@ -667,9 +701,43 @@ ug_status NetImpl<R>::ensure_batch(int B)
     return UG_OK;
 }
 
+// The batch in one cooperative launch, or in two with the noise of the second beside the first.
+template <class R>
+ug_status NetImpl<R>::issue_test_trial(const ug::LaunchCtx& lc)
+{
+    const int Q = (int)sync_steps.size();
+    const int* ends = dSyncEnd_.as<int>();
+    unsigned* ctl = test_ctl_.as<unsigned>();
+    UG_CUDA(ug::launch_state_init<R>(nd_, bd_, lc.main));
+    UG_CUDA(cudaMemsetAsync(ctl, 0, (size_t)bd_.B * ug::kCtlWords * sizeof(unsigned), lc.main));
+    if (!segmented()) {
+        UG_CUDA(ug::launch_noise_segment<R>(nd_, bd_, h.num_steps - 1, 0, bd_.ev_cap, lc.main));
+        UG_CUDA(ug::launch_test_trial<R>(nd_, bd_, rc_, ic_, test_plan_, ends, Q, 0, Q + 1, ctl, lc.main));
+        return UG_OK;
+    }
+    own_gaps();
+    const int qa = Q / 16;                                             // a sixteenth of the trial first,
+    const int ka = std::min((bd_.ev_cap / 4 + 63) / 64 * 64, bd_.ev_cap / 2 * 2);   // a quarter of the intervals
+    UG_CUDA(ug::launch_noise_segment<R>(nd_, bd_, sync_steps[qa - 1], 0, ka, lc.main));
+    UG_CUDA(cudaEventRecord(lc.fork, lc.main));
+    UG_CUDA(cudaStreamWaitEvent(lc.side, lc.fork, 0));
+    UG_CUDA(ug::launch_noise_segment<R>(nd_, bd_, h.num_steps - 1, ka, bd_.ev_cap, lc.side));
+    UG_CUDA(cudaEventRecord(lc.join, lc.side));
+    UG_CUDA(ug::launch_test_trial<R>(nd_, bd_, rc_, ic_, test_plan_, ends, Q, 0, qa, ctl, lc.main));
+    UG_CUDA(cudaStreamWaitEvent(lc.main, lc.join, 0));
+    UG_CUDA(ug::launch_test_trial<R>(nd_, bd_, rc_, ic_, test_plan_, ends, Q, qa, Q + 1, ctl, lc.main));
+    share_gaps();
+    return UG_OK;
+}
+
 template <class R>
 ug_status NetImpl<R>::issue_batch(const ug::LaunchCtx& lc, int64_t* launches)
 {
+    if (test_plan_.lanes > 0) {
+        UG_TRY(issue_test_trial(lc));
+        if (launches) *launches += batch_launches(lc);
+        return UG_OK;
+    }
     UG_CUDA(ug::launch_trial_init<R>(nd_, bd_, lc));
     const int Q = (int)sync_steps.size();
     for (int q = 0; q < Q; ++q) {
@@ -689,7 +757,12 @@ ug_status NetImpl<R>::run_test_trials(uint32_t first_trial, int n_trials, const 
 {
     cudaStream_t st = lc.main;
     UG_TRY(prepare_test(first_trial, n_trials, st));
-    if (!graphs || lc.timer) return issue_batch(lc, launches);
+    if (!graph_exec_ || graph_B_ != n_trials || graph_fuse_ != lc.fuse || !graphs || lc.timer) UG_TRY(plan_batch(lc));
+    if (!graphs || lc.timer) {
+        const ug_status s = issue_batch(lc, launches);
+        graph_B_ = -1;   // the plan in force is this call's, not a captured graph's
+        return s;
+    }
     if (!graph_exec_ || graph_B_ != n_trials || graph_fuse_ != lc.fuse) {
         if (graph_exec_) {
             cudaGraphExecDestroy(graph_exec_);
@@ -728,9 +801,9 @@ size_t NetImpl<R>::device_bytes() const
     for (int k = 0; k < 10; ++k) t += ra_[k].bytes();
     for (int k = 0; k < 7; ++k) t += iv_[k].bytes();
     for (const DevMem* m : {&ra_flags_, &kick_step_, &ra_nsoma_, &ra_ndend_, &ra_first_soma_, &ra_first_dend_,
-                            &i_noise_, &i_noise_step_, &i_events_, &i_ev_idx_, &i_word_, &i_flag_, &i_nspk_, &i_first_,
+                            &i_noise_, &i_noise_step_, &i_events_, &i_ev_idx_, &i_ev_cnt_, &i_gaps_, &i_word_, &i_flag_, &i_nspk_, &i_first_,
                             &ring_ra_exc_, &ring_ra_inh_, &ring_i_exc_, &spk_buf_, &spk_count_, &error_, &trial_,
-                            &mean_inj_})
+                            &mean_inj_, &test_ctl_, &dSyncEnd_})
         t += m->bytes();
     for (const DevMem* m : {&gW_, &gD_, &gPerm_, &gActive_, &gSuper_, &gActList_, &gActCnt_, &gSupList_, &gSupCnt_,
                             &gRemod_, &gPreStep_, &gPreCnt_, &gPostStep_, &gPostCnt_, &gPostLast_, &gSpikeLast_, &gStStep_, &gStCur_, &gStLen_,
@@ -752,9 +825,9 @@ size_t NetImpl<R>::footprint(int kind, int B) const
     t += 4 * (nra + 1) + 20 * e_ri + 4 * (ni + 1) + 20 * e_ir + 4 * (nra + 1) + 20 * act;
     if (kind == 1) B = 1;
     const size_t bra = (size_t)B * nra, bi = (size_t)B * ni;
-    const size_t ev_cap = r == 4 ? (size_t)(h.num_steps * 0.02 * 0.25 * 2.0) + 64 : 1;
+    const size_t ev_cap = r == 4 ? (size_t)(h.num_steps * 0.02 * 0.25 * 2.0) + 65 : 1;
     const size_t cap = (size_t)spike_cap_per_neuron_ * (2 * nra + ni);
-    t += bra * (10 * r + 24) + bi * (7 * r + 16 + 8 + 16 * ev_cap + 8 + 16);
+    t += bra * (10 * r + 24) + bi * (7 * r + 16 + 8 + 16 * ev_cap + 16 + 16) + 8 * ev_cap * ni * std::min(B, kSegmentBatch) + (size_t)B * 4 * ug::kCtlWords + 4 * sync_steps.size();
     t += (size_t)ring * 8 * (2 * bra + bi) + (size_t)B * (cap * 8 + 16);
     if (kind == 1) {
         const size_t nn = nra * nra;
@@ -968,10 +1041,9 @@ ug_status NetImpl<R>::growth_init(cudaStream_t st)
     UG_TRY(gRepCnt_.alloc(sizeof(int)));
     UG_TRY(gLoop_.alloc(ug::kLoopWords * sizeof(int)));
     if (!hloop_) UG_CUDA(cudaMallocHost(&hloop_, ug::kLoopWords * sizeof(int)));
-    // the one-launch trial: barrier and queue words, the row queue, the sync steps
+    // the one-launch trial: barrier and queue words, the row queue
     UG_TRY(gTrialCtl_.alloc(8 * sizeof(unsigned)));
     UG_TRY(gActRows_.alloc(4 * (size_t)n * sizeof(int2)));
-    UG_TRY(gSyncEnd_.upload(sync_steps, st));
     trial_blocks_ = 0;
     trial_key_ = -1;
     bool fits = !sync_steps.empty();
@@ -1078,7 +1150,7 @@ ug_status NetImpl<R>::issue_growth_trial(const ug::LaunchCtx& lc, int64_t* launc
         b.live_streams = gd_.st_num;
         b.heavy = 0;
         ug::TrialLoop L;
-        L.sync_end = gSyncEnd_.as<int>();
+        L.sync_end = dSyncEnd_.as<int>();
         L.Q = Q;
         int nb_sync = 0;
         ug::trial_widths<R>(lc.trial_ra_w, lc.trial_i_w, &L.ra_w, &L.i_w);   // checked by trial_grid

@@ -20,4 +20,11 @@ template cudaError_t launch_growth_tail<float>(const TailDev<float>&, cudaStream
 template cudaError_t group_grids<float>(GroupDev&, int, int);
 template cudaError_t launch_group_trial<float>(const GroupDev&, const std::vector<int>&, int, bool, const LaunchCtx&,
                                                 int64_t*);
+template cudaError_t launch_state_init<float>(const NetDev<float>&, const BatchDev<float>&, cudaStream_t);
+template cudaError_t launch_noise_segment<float>(const NetDev<float>&, const BatchDev<float>&, int, int, int, cudaStream_t);
+template cudaError_t test_trial_plan<float>(int, int, int, TestPlan*);
+template cudaError_t launch_test_trial<float>(const NetDev<float>&, const BatchDev<float>&, const RAStep<float>&,
+                                            const IStep<float>&, const TestPlan&, const int*, int, int, int, unsigned*,
+                                            cudaStream_t);
+
 }  // namespace ug

@@ -20,4 +20,11 @@ template cudaError_t launch_growth_tail<double>(const TailDev<double>&, cudaStre
 template cudaError_t group_grids<double>(GroupDev&, int, int);
 template cudaError_t launch_group_trial<double>(const GroupDev&, const std::vector<int>&, int, bool, const LaunchCtx&,
                                                 int64_t*);
+template cudaError_t launch_state_init<double>(const NetDev<double>&, const BatchDev<double>&, cudaStream_t);
+template cudaError_t launch_noise_segment<double>(const NetDev<double>&, const BatchDev<double>&, int, int, int, cudaStream_t);
+template cudaError_t test_trial_plan<double>(int, int, int, TestPlan*);
+template cudaError_t launch_test_trial<double>(const NetDev<double>&, const BatchDev<double>&, const RAStep<double>&,
+                                            const IStep<double>&, const TestPlan&, const int*, int, int, int, unsigned*,
+                                            cudaStream_t);
+
 }  // namespace ug

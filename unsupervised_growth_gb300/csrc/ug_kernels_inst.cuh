@@ -24,9 +24,9 @@ inline void launch_noise_events(const NetDev<float>& n, const BatchDev<float>& b
     if (n.n_i == 0) return;
     if (lc.timer) lc.timer->begin("k_noise_events", lc.main);
     constexpr int kPer = kNoiseThreads / 32;
-    k_noise_gaps<float><<<dim3((n.n_i + kPer - 1) / kPer, b.B), kNoiseThreads, 0, lc.main>>>(n, b);
+    k_noise_gaps<float><<<dim3((n.n_i + kPer - 1) / kPer, b.B), kNoiseThreads, 0, lc.main>>>(n, b, 0, b.ev_cap);
     k_noise_events<float><<<dim3((n.n_i + kNoiseWalk - 1) / kNoiseWalk, b.B), kNoiseWalk, 0, lc.main>>>(
-        n, b, n.num_steps - 1, false);
+        n, b, n.num_steps - 1, b.ev_cap, false);
     if (lc.timer) lc.timer->end(lc.main);
 }
 
@@ -67,6 +67,101 @@ cudaError_t launch_trial_init(const NetDev<R>& n, const BatchDev<R>& b, const La
     UG_TIMED(lc, "k_trial_init", (k_trial_init<R><<<grid, kBlock, 0, lc.main>>>(n, b)));
     launch_noise_events(n, b, lc);
     return cudaGetLastError();
+}
+
+template <class R>
+cudaError_t launch_state_init(const NetDev<R>& n, const BatchDev<R>& b, cudaStream_t st)
+{
+    const dim3 grid((n.n_ra + kBlock - 1) / kBlock + (n.n_i + kBlock - 1) / kBlock, b.B);
+    k_trial_init<R><<<grid, kBlock, 0, st>>>(n, b);
+    return cudaGetLastError();
+}
+
+template <class R>
+cudaError_t launch_noise_segment(const NetDev<R>& n, const BatchDev<R>& b, int end, int k0, int k1, cudaStream_t st)
+{
+    if constexpr (sizeof(R) == 4) {
+        if (n.n_i == 0) return cudaSuccess;
+        constexpr int kPer = kNoiseThreads / 32;
+        k_noise_gaps<float><<<dim3((n.n_i + kPer - 1) / kPer, b.B), kNoiseThreads, 0, st>>>(n, b, k0, k1);
+        k_noise_events<float><<<dim3((n.n_i + kNoiseWalk - 1) / kNoiseWalk, b.B), kNoiseWalk, 0, st>>>(n, b, end, k1,
+                                                                                                     k0 > 0);
+        return cudaGetLastError();
+    }
+    return cudaErrorNotSupported;
+}
+
+// Form of a batch of test trials: one launch when all its warps can be resident at once and
+// they make no more rounds of the GPU's schedulers (a warp each) than the per-interval
+// launches, which pack the neurons of all trials without a partly empty last warp per trial.
+// Measured, ms a batch, one launch against per-interval launches: 2000/550, 12 trials (600
+// warps) 33.2 / 36.2, 24 (1200) 46.5 / 52.4, 48 (2400) 75.9 / 82.4; 777/194, 24 (480 warps,
+// one round each) 27.7 / 32.7, 48 (960, two each) 41.0 / 46.7, but 32 (640 warps, two rounds
+// against one) 42.8 / 32.9.  One HVC(RA) neuron per thread while each warp has a scheduler to
+// itself (the step chain bounds it: 765 cycles a step against 1310 with two; 8 trials of
+// 777/194 24.5 ms against 27.7 for 24 with two), two from there on.
+constexpr int kTestMaxRounds = 4;   // 4 blocks of 4 warps per SM are resident
+template <class R>
+cudaError_t test_trial_plan(int n_ra, int n_i, int B, TestPlan* plan)
+{
+    *plan = TestPlan();
+    if constexpr (sizeof(R) == 4) {
+        int dev = 0, sms = 0, coop = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+        if (e != cudaSuccess || !coop) return e;
+        for (int lanes = 1; lanes <= 2; ++lanes) {
+            TestPlan p;
+            p.ra_units = (n_ra + 32 * lanes - 1) / (32 * lanes);
+            p.i_units = (n_i + 31) / 32;
+            const long long ra = (long long)B * p.ra_units, in = (long long)B * p.i_units;
+            const long long pad = (ra + kUnitWarps - 1) / kUnitWarps * kUnitWarps;
+            const long long blocks = (pad + in + kUnitWarps - 1) / kUnitWarps;
+            const long long flat = ((long long)B * ((n_ra + 1) / 2) + kBlock - 1) / kBlock +
+                                   ((long long)B * n_i + kBlock - 1) / kBlock;
+            const long long rounds = (blocks + sms - 1) / sms;   // a block has a warp per scheduler
+            if (rounds > (lanes == 1 ? 1 : std::min<long long>(kTestMaxRounds, (flat + sms - 1) / sms))) continue;
+            int per_sm = 0;
+            e = lanes == 1
+                    ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_test_trial<float>, 32 * kUnitWarps, 0)
+                    : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_test_trial<f2>, 32 * kUnitWarps, 0);
+            if (e != cudaSuccess) return e;
+            if (blocks > (long long)per_sm * sms) continue;
+            p.lanes = lanes;
+            p.blocks = (int)blocks;
+            p.ra_pad = (int)pad;
+            *plan = p;
+            return cudaSuccess;
+        }
+    }
+    return cudaSuccess;
+}
+
+template <class R>
+cudaError_t launch_test_trial(const NetDev<R>& n, const BatchDev<R>& b, const RAStep<R>& rc, const IStep<R>& ic,
+                              const TestPlan& plan, const int* sync_end, int Q, int q0, int q1, unsigned* ctl,
+                              cudaStream_t st)
+{
+    if constexpr (sizeof(R) == 4) {
+        TestLoop L;
+        L.sync_end = sync_end;
+        L.Q = Q; L.q0 = q0; L.q1 = q1;
+        L.ra_units = plan.ra_units; L.i_units = plan.i_units; L.ra_pad = plan.ra_pad;
+        L.ctl = ctl;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)plan.blocks);
+        cfg.blockDim = dim3(32 * kUnitWarps);
+        cfg.stream = st;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeCooperative;   // every block resident at once, or the launch fails
+        at[0].val.cooperative = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        return plan.lanes == 1 ? cudaLaunchKernelEx(&cfg, k_test_trial<float>, n, b, rc, ic, L)
+                               : cudaLaunchKernelEx(&cfg, k_test_trial<f2>, n, b, rc, ic, L);
+    }
+    return cudaErrorNotSupported;
 }
 
 // HVC(RA) interval kernel: the double build steps one neuron per thread, the

@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "ug_group.cuh"
+#include "ug_test_trial.cuh"
 #include "ug_growth_trial.cuh"
 #include "ug_tail.cuh"
 
@@ -119,6 +120,25 @@ inline bool fused_interval(const NetDev<R>& n, const BatchDev<R>& b, const Launc
 {
     return sizeof(R) == 4 && lc.fuse && n.n_i > 0 && b.B >= 16 && !b.trace_ra && !b.trace_i && !b.ginh_slot;
 }
+
+// The one-launch form of a small batch of test trials (k_test_trial, single build).
+struct TestPlan {
+    int lanes = 0;           // HVC(RA) neurons per thread; 0: per-interval launches
+    int blocks = 0;
+    int ra_units = 0, i_units = 0, ra_pad = 0;   // TestLoop
+};
+template <class R>
+cudaError_t test_trial_plan(int n_ra, int n_i, int B, TestPlan* plan);
+template <class R>
+cudaError_t launch_test_trial(const NetDev<R>& n, const BatchDev<R>& b, const RAStep<R>& rc, const IStep<R>& ic,
+                              const TestPlan& plan, const int* sync_end, int Q, int q0, int q1, unsigned* ctl,
+                              cudaStream_t st);
+// The noise pre-pass in segments, after k_trial_init: intervals k0 .. k1 - 1 of each neuron
+// (k0 even) and the events up to step `end`, after an earlier call's when k0 > 0.
+template <class R>
+cudaError_t launch_noise_segment(const NetDev<R>& n, const BatchDev<R>& b, int end, int k0, int k1, cudaStream_t st);
+template <class R>
+cudaError_t launch_state_init(const NetDev<R>& n, const BatchDev<R>& b, cudaStream_t st);
 
 template <class R>
 cudaError_t launch_interval(const NetDev<R>& n, const BatchDev<R>& b, int q, int s0, int s1, const RAStep<R>& rc,

@@ -102,8 +102,9 @@ __device__ __forceinline__ RACell<V> ra_cell(V EL, V GdCa, float mus, float mud)
     return P;
 }
 
+// G: Gexc_d + Ginh_d, Gi: Ginh_d, at the stage's time.
 template <class V>
-__device__ __forceinline__ RAVec<V> ra_rhs(const RAVec<V>& y, V Ge, V Gi, const RACell<V>& P)
+__device__ __forceinline__ RAVec<V> ra_rhs(const RAVec<V>& y, V G, V Gi, const RACell<V>& P)
 {
     typedef RAConst K;
 #define C(x) Lanes<V>::all(x)
@@ -159,7 +160,7 @@ __device__ __forceinline__ RAVec<V> ra_rhs(const RAVec<V>& y, V Ge, V Gi, const 
     V u = v_fma(vd, C(-(float)K::GdL), P.cd);
     u = v_fma(gr2, eca, u);
     u = v_fma(v_mul(v_sub(vd, C((float)K::EdK)), y.c), v_mul(v_mul(y.Ca, iDca), C(-(float)K::GdCaK)), u);
-    u = v_fma(v_add(Ge, Gi), v_sub(C(0.0f), vd), v_fma(Gi, C((float)K::Egaba), u));
+    u = v_fma(G, v_sub(C(0.0f), vd), v_fma(Gi, C((float)K::Egaba), u));
     k.Vd = v_fma(dv, C(-(float)(100000.0 / (K::Rc * K::Ad))), u);
     // kn = (nInf - n)/tauN = (1 - n (1 + En)) bn / Dn ; kh likewise
     k.n = v_mul(v_mul(v_fma(y.n, an, C(1.0f)), bn), iDn);
@@ -183,12 +184,15 @@ __device__ __forceinline__ void ra_debrabant_v(RAVec<V>& s, V& Ge, V& Gi, const 
                                                const RANoise<V>& z)
 {
     const V dt = C(p.dt);
-    const V Ge1 = v_mul(Ge, C(p.e1)), Gi1 = v_mul(Gi, C(p.e1)), Ge2 = v_mul(Ge, C(p.e2)), Gi2 = v_mul(Gi, C(p.e2));
+    const V Ge1 = v_mul(Ge, C(p.e1)), Gi1 = v_mul(Gi, C(p.e1)), Gi2 = v_mul(Gi, C(p.e2));
+    // Gexc + Ginh at the stages' times (the half step's has one rounding, as the compiler
+    // contracts the packed form; written out, so that the scalar form has it too)
+    const V G0 = v_add(Ge, Gi), G1 = v_add(Ge1, Gi1), G2 = v_fma(Ge, C(p.e2), Gi2);
 
     RAVec<V> y = s;
     y.Vs = v_fma(z.a1s, C(-0.01844540496323970f), v_fma(z.a2s, C(-0.1866426386543421f), s.Vs));
     y.Vd = v_fma(z.a1d, C(-0.01844540496323970f), v_fma(z.a2d, C(-0.1866426386543421f), s.Vd));
-    const RAVec<V> a1 = ra_rhs(y, Ge, Gi, P);
+    const RAVec<V> a1 = ra_rhs(y, G0, Gi, P);
 
     RAVec<V> h4, up;   // running sums of stage 4's increment and of the update
 #define M(f) h4.f = v_mul(a1.f, C(-0.4526683126055039f)); up.f = v_mul(a1.f, C(1.0f / 6.0f)); y.f = v_fma(dt, a1.f, s.f);
@@ -196,7 +200,7 @@ __device__ __forceinline__ void ra_debrabant_v(RAVec<V>& s, V& Ge, V& Gi, const 
 #undef M
     y.Vs = v_fma(z.a1s, C(0.8017012756521233f), v_fma(z.a2s, C(-0.8575745885712401f), y.Vs));
     y.Vd = v_fma(z.a1d, C(0.8017012756521233f), v_fma(z.a2d, C(-0.8575745885712401f), y.Vd));
-    const RAVec<V> a2 = ra_rhs(y, Ge1, Gi1, P);
+    const RAVec<V> a2 = ra_rhs(y, G1, Gi1, P);
 
     const V d8 = C(p.dt * 0.125f);
 #define M(f) h4.f = v_fma(a2.f, C(-0.4842227708685013f), h4.f); up.f = v_fma(a2.f, C(-0.005430430675258792f), up.f); \
@@ -205,7 +209,7 @@ __device__ __forceinline__ void ra_debrabant_v(RAVec<V>& s, V& Ge, V& Gi, const 
 #undef M
     y.Vs = v_fma(z.a1s, C(0.5092227024816198f), v_fma(z.a2s, C(-0.4723392695015512f), y.Vs));
     y.Vd = v_fma(z.a1d, C(0.5092227024816198f), v_fma(z.a2d, C(-0.4723392695015512f), y.Vd));
-    const RAVec<V> a3 = ra_rhs(y, Ge2, Gi2, P);
+    const RAVec<V> a3 = ra_rhs(y, G2, Gi2, P);
 
 #define M(f) h4.f = v_fma(a3.f, C(1.9368910834740051f), h4.f); up.f = v_fma(a3.f, C(2.0f / 3.0f), up.f); \
              y.f = v_fma(dt, h4.f, s.f);
@@ -213,7 +217,7 @@ __device__ __forceinline__ void ra_debrabant_v(RAVec<V>& s, V& Ge, V& Gi, const 
 #undef M
     y.Vs = v_fma(z.a1s, C(0.9758794209767762f), v_fma(z.a2s, C(0.3060354860326548f), y.Vs));
     y.Vd = v_fma(z.a1d, C(0.9758794209767762f), v_fma(z.a2d, C(0.3060354860326548f), y.Vd));
-    const RAVec<V> a4 = ra_rhs(y, Ge1, Gi1, P);
+    const RAVec<V> a4 = ra_rhs(y, G1, Gi1, P);
 
 #define M(f) s.f = v_fma(dt, v_fma(a4.f, C(0.1720970973419255f), up.f), s.f);
     UG_RA_FOR(M)

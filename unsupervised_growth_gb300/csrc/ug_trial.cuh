@@ -479,89 +479,116 @@ __device__ __forceinline__ void add_kick(f2& Ge, const int* kick, int st)
     if (st == kick[1]) Ge.y = Ge.y + 3.0f;
 }
 
-// Single-precision HVC(RA) part of one interval over the lane type V of ug_ra_f32.cuh:
-// thread t steps neuron t (V float) or neurons 2t and 2t + 1 (V f2).
-template <class V, class R, bool kTrack = false>
-__device__ __forceinline__ void interval_ra_v_body(const NetDev<R>& n, const BatchDev<R>& bt, int q, int s0, int s1,
-                                                   const RAStep<R>& rc, int t, int b)
-{
-    // t: the thread's first neuron / Lanes<V>::n (none when that is >= n_ra), b: its instance
-    static_assert(sizeof(R) == 4, "the lane-typed RA kernel is single precision");
+// A thread's HVC(RA) neurons in registers: neuron t (V float) or neurons 2t and 2t + 1 (V f2)
+// of instance b.  kAhead: the noise of the next step is drawn during this one, which leaves it
+// off the step's dependency chain (a lone warp 830 -> 765 cycles a step); a kernel that
+// integrates one interval only would draw a thirteenth step's for nothing.
+template <class V, bool kAhead>
+struct RAUnit {
     typedef Lanes<V> L;
-    constexpr int N = L::n;
-    const int i0 = N * t;
-    uint32_t soma[N] = {}, dend[N] = {};
-    if (i0 < n.n_ra) {
-        // the lanes' neurons; a lane past the last neuron repeats its thread's first one and
-        // stores nothing
-        bool valid[N];
-        size_t x[N];
-        uint32_t ent[N];
+    static constexpr int N = L::n;
+    RAVec<V> s;
+    V Ge, Gi;
+    RACell<V> P;
+    RANoiseStream<V> rng;
+    RANoise<V> z;
+    float ns, nd;
+    int fs[N], fd[N], kick[N];
+    uint32_t ent[N];   // the lanes' neurons; a lane past the last one repeats the thread's first
+    bool valid[N];     // and stores nothing
+    int b;
+
+    template <class R>
+    __device__ __forceinline__ size_t at(const NetDev<R>& n, int k) const { return (size_t)b * n.n_ra + ent[k]; }
+
+    template <class R>
+    __device__ __forceinline__ void load(const NetDev<R>& n, const BatchDev<R>& bt, const RAStep<R>& rc, int t, int b_,
+                                         int s0)
+    {
+        static_assert(sizeof(R) == 4, "the lane-typed RA integrator is single precision");
+        b = b_;
 #pragma unroll
         for (int k = 0; k < N; ++k) {
-            valid[k] = i0 + k < n.n_ra;
-            ent[k] = (uint32_t)(valid[k] ? i0 + k : i0);
-            x[k] = (size_t)b * n.n_ra + ent[k];
+            valid[k] = N * t + k < n.n_ra;
+            ent[k] = (uint32_t)(valid[k] ? N * t + k : N * t);
         }
-        auto load = [&](const R* p) {
+        auto get = [&](const R* p) {
             float v[N];
 #pragma unroll
-            for (int k = 0; k < N; ++k) v[k] = p[x[k]];
+            for (int k = 0; k < N; ++k) v[k] = p[at(n, k)];
             return L::make(v);
         };
-        RAVec<V> s;
-        s.Vs = load(bt.ra[0]); s.Vd = load(bt.ra[1]); s.n = load(bt.ra[2]); s.h = load(bt.ra[3]);
-        s.l = load(bt.ra[4]); s.r = load(bt.ra[5]); s.c = load(bt.ra[6]); s.Ca = load(bt.ra[7]);
-        float ge[N], gi[N];
-        int fs[N], fd[N], kick[N];
+        s.Vs = get(bt.ra[0]); s.Vd = get(bt.ra[1]); s.n = get(bt.ra[2]); s.h = get(bt.ra[3]);
+        s.l = get(bt.ra[4]); s.r = get(bt.ra[5]); s.c = get(bt.ra[6]); s.Ca = get(bt.ra[7]);
+        Ge = get(bt.ra[8]); Gi = get(bt.ra[9]);
 #pragma unroll
         for (int k = 0; k < N; ++k) {
-            ge[k] = bt.ra[8][x[k]];
-            gi[k] = bt.ra[9][x[k]];
-            const int fl = bt.ra_flags[x[k]];
+            const int fl = bt.ra_flags[at(n, k)];
             fs[k] = fl & 1;
             fd[k] = (fl >> 1) & 1;
-            kick[k] = valid[k] ? bt.kick_step[x[k]] : 0x7fffffff;
+            kick[k] = valid[k] ? bt.kick_step[at(n, k)] : 0x7fffffff;
         }
-        if (q > 0) {
-            // sync q-1: raiseI(sum Gi), raiseExcWeight(sum w) = Gexc_d += w / Ad
-            const size_t base = (size_t)((q - 1) % n.ring) * bt.B * n.n_ra;
-            long long ai[N], ae[N];
-#pragma unroll
-            for (int k = 0; k < N; ++k) {
-                ai[k] = valid[k] ? bt.ring_ra_inh[base + x[k]] : 0;
-                ae[k] = valid[k] ? bt.ring_ra_exc[base + x[k]] : 0;
-            }
-#pragma unroll
-            for (int k = 0; k < N; ++k)
-                if (ai[k] | ae[k]) {
-                    bt.ring_ra_inh[base + x[k]] = 0;
-                    bt.ring_ra_exc[base + x[k]] = 0;
-                    gi[k] = gi[k] + (float)((double)ai[k] * kFixInv);
-                    ge[k] = ge[k] + (float)(((double)ae[k] * kFixInv) / RAConst::Ad);
-                }
-        }
-        V Ge = L::make(ge), Gi = L::make(gi);
-        const RACell<V> P = ra_cell<V>(load_param<V>(n.Erest, ent), load_param<V>(n.GCa, ent),
-                                       (float)(100000.0 / RAConst::As) * rc.mu_s,
-                                       (float)(100000.0 / RAConst::Ad) * rc.mu_d);
-        const float ns = rc.sq * rc.sig_s * (float)(1.0 / (RAConst::As * RAConst::cm));
-        const float nd = rc.sq * rc.sig_d * (float)(1.0 / (RAConst::Ad * RAConst::cm));
-        RANoiseStream<V> rng;
+        P = ra_cell<V>(load_param<V>(n.Erest, ent), load_param<V>(n.GCa, ent),
+                       (float)(100000.0 / RAConst::As) * rc.mu_s, (float)(100000.0 / RAConst::Ad) * rc.mu_d);
+        ns = rc.sq * rc.sig_s * (float)(1.0 / (RAConst::As * RAConst::cm));
+        nd = rc.sq * rc.sig_d * (float)(1.0 / (RAConst::Ad * RAConst::cm));
         rng.init(ent, bt.trial[b], make_stream(n.seed, kNoiseRAWhite, n.net_id, 0, 0).tag, rc.ks);
+        if constexpr (kAhead) z = rng.draw((uint32_t)s0, ns, nd, rc.ks);
+    }
+
+    // Sync q: raiseI(sum Gi), raiseExcWeight(sum w) = Gexc_d += w / Ad.  The sums are read past
+    // the L1 cache: in the one-launch trials other SMs add to them while the kernel runs.
+    template <class R>
+    __device__ __forceinline__ void sync_kicks(const NetDev<R>& n, const BatchDev<R>& bt, int q)
+    {
+        const size_t base = (size_t)(q % n.ring) * bt.B * n.n_ra;
+        long long ai[N], ae[N];
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            ai[k] = valid[k] ? __ldcg(&bt.ring_ra_inh[base + at(n, k)]) : 0;
+            ae[k] = valid[k] ? __ldcg(&bt.ring_ra_exc[base + at(n, k)]) : 0;
+        }
+        float ge[N], gi[N];
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            ge[k] = L::get(Ge, k);
+            gi[k] = L::get(Gi, k);
+            if (ai[k] | ae[k]) {
+                bt.ring_ra_inh[base + at(n, k)] = 0;
+                bt.ring_ra_exc[base + at(n, k)] = 0;
+                gi[k] = gi[k] + (float)((double)ai[k] * kFixInv);
+                ge[k] = ge[k] + (float)(((double)ae[k] * kFixInv) / RAConst::Ad);
+            }
+        }
+        Ge = L::make(ge);
+        Gi = L::make(gi);
+    }
+
+    // Steps s0..s1; bit st - s0 of soma / dend is set where a neuron spiked at step st.
+    // kTrack: traces of instance 0 and inhibition tracking.
+    template <bool kTrack, class R>
+    __device__ __forceinline__ void steps(const NetDev<R>& n, const BatchDev<R>& bt, const RAStep<R>& rc, int s0, int s1,
+                                          uint32_t (&soma)[N], uint32_t (&dend)[N])
+    {
         for (int st = s0; st <= s1; ++st) {
             add_kick(Ge, kick, st);   // raiseE(G_TRAINING_KICK)
             if constexpr (kTrack) {
 #pragma unroll
                 for (int k = 0; k < N; ++k)
                     if (valid[k])
-                        trace_ra_row(bt, n.num_steps, b, i0 + k, st, L::get(s.Vs, k), L::get(s.Vd, k), L::get(Ge, k),
-                                     L::get(Gi, k));
+                        trace_ra_row(bt, n.num_steps, b, (int)ent[k], st, L::get(s.Vs, k), L::get(s.Vd, k),
+                                     L::get(Ge, k), L::get(Gi, k));
             }
 #pragma unroll
             for (int k = 0; k < N; ++k)
                 ra_check_f(L::get(s.Vs, k), L::get(s.Vd, k), fs[k], fd[k], soma[k], dend[k], st - s0);
-            ra_debrabant_v(s, Ge, Gi, P, rc, rng.draw((uint32_t)st, ns, nd, rc.ks));
+            if constexpr (kAhead) {
+                const RANoise<V> now = z;
+                z = rng.draw((uint32_t)st + 1u, ns, nd, rc.ks);
+                ra_debrabant_v(s, Ge, Gi, P, rc, now);
+            } else {
+                ra_debrabant_v(s, Ge, Gi, P, rc, rng.draw((uint32_t)st, ns, nd, rc.ks));
+            }
             if constexpr (kTrack) {   // inhibition tracking; a group may mix tracked and untracked members
                 if (bt.ginh_slot && bt.ginh_rec) {
                     const int sl = bt.ginh_slot[st];
@@ -569,47 +596,87 @@ __device__ __forceinline__ void interval_ra_v_body(const NetDev<R>& n, const Bat
                         R* rec = bt.ginh_rec + (size_t)sl * bt.B * n.n_ra;
 #pragma unroll
                         for (int k = 0; k < N; ++k)
-                            if (valid[k]) rec[x[k]] = L::get(Gi, k);
+                            if (valid[k]) rec[at(n, k)] = L::get(Gi, k);
                     }
                 }
             }
         }
 #pragma unroll
+        for (int k = 0; k < N; ++k)
+            if (!valid[k]) soma[k] = dend[k] = 0;
+    }
+
+    template <class R>
+    __device__ __forceinline__ void store(const NetDev<R>& n, const BatchDev<R>& bt) const
+    {
+#pragma unroll
         for (int k = 0; k < N; ++k) {
-            if (!valid[k]) {
-                soma[k] = dend[k] = 0;
-                continue;
-            }
-            const size_t xk = x[k];
-            bt.ra[0][xk] = L::get(s.Vs, k); bt.ra[1][xk] = L::get(s.Vd, k); bt.ra[2][xk] = L::get(s.n, k);
-            bt.ra[3][xk] = L::get(s.h, k); bt.ra[4][xk] = L::get(s.l, k); bt.ra[5][xk] = L::get(s.r, k);
-            bt.ra[6][xk] = L::get(s.c, k); bt.ra[7][xk] = L::get(s.Ca, k); bt.ra[8][xk] = L::get(Ge, k);
-            bt.ra[9][xk] = L::get(Gi, k);
-            bt.ra_flags[xk] = fs[k] | fd[k] << 1;
-            const uint32_t so = soma[k], de = dend[k];
-            const int i = i0 + k;
-            if (so) {
-                bt.ra_nsoma[xk] += __popc(so);
-                if (bt.ra_first_soma[xk] < 0) bt.ra_first_soma[xk] = s0 + __ffs(so) - 1;
-                record_spikes(bt.spk_count, bt.spk_buf, bt.spk_cap, bt.error, b, i, kSpikeSoma, so, s0);
-            }
-            if (de) {
-                bt.ra_ndend[xk] += __popc(de);
-                if (bt.ra_first_dend[xk] < 0) bt.ra_first_dend[xk] = s0 + __ffs(de) - 1;
-                record_spikes(bt.spk_count, bt.spk_buf, bt.spk_cap, bt.error, b, i, kSpikeDend, de, s0);
-            }
-            if (bt.soma_bits) bt.soma_bits[(size_t)(q & 1) * bt.B * n.n_ra + xk] = (int)so;
-            if (bt.act_rows) queue_row(bt, q, (int)xk, so);
+            if (!valid[k]) continue;
+            const size_t x = at(n, k);
+            bt.ra[0][x] = L::get(s.Vs, k); bt.ra[1][x] = L::get(s.Vd, k); bt.ra[2][x] = L::get(s.n, k);
+            bt.ra[3][x] = L::get(s.h, k); bt.ra[4][x] = L::get(s.l, k); bt.ra[5][x] = L::get(s.r, k);
+            bt.ra[6][x] = L::get(s.c, k); bt.ra[7][x] = L::get(s.Ca, k); bt.ra[8][x] = L::get(Ge, k);
+            bt.ra[9][x] = L::get(Gi, k);
+            bt.ra_flags[x] = fs[k] | fd[k] << 1;
+        }
+    }
+};
+
+// Counts, first steps and records of the interval's spikes of HVC(RA) neuron i (at x) of instance b.
+template <class R>
+__device__ __forceinline__ void ra_spike_stats(const BatchDev<R>& bt, size_t x, int i, int b, int s0, uint32_t soma,
+                                               uint32_t dend)
+{
+    if (soma) {
+        bt.ra_nsoma[x] += __popc(soma);
+        if (bt.ra_first_soma[x] < 0) bt.ra_first_soma[x] = s0 + __ffs(soma) - 1;
+        record_spikes(bt.spk_count, bt.spk_buf, bt.spk_cap, bt.error, b, i, kSpikeSoma, soma, s0);
+    }
+    if (dend) {
+        bt.ra_ndend[x] += __popc(dend);
+        if (bt.ra_first_dend[x] < 0) bt.ra_first_dend[x] = s0 + __ffs(dend) - 1;
+        record_spikes(bt.spk_count, bt.spk_buf, bt.spk_cap, bt.error, b, i, kSpikeDend, dend, s0);
+    }
+}
+
+// The RA->I kicks (and, in test trials, the RA->RA kicks over the static active lists) of the
+// interval's somatic spikes of neuron i of instance b; every lane of the warp takes part.
+template <class R>
+__device__ __forceinline__ void ra_scatter(const NetDev<R>& n, const BatchDev<R>& bt, uint32_t soma, int i, int b, int s0)
+{
+    scatter_warp(soma, i, s0, n.T, n.num_steps, n.syncidx, n.ring, n.ra2i_off, n.ra2i_tgt, n.ra2i_wq, n.ra2i_d,
+                 bt.ring_i_exc, (size_t)bt.B * n.n_i, (size_t)b * n.n_i);
+    if (bt.scatter_rara)
+        scatter_warp(soma, i, s0, n.T, n.num_steps, n.syncidx, n.ring, n.rara_off, n.rara_tgt, n.rara_wq, n.rara_d,
+                     bt.ring_ra_exc, (size_t)bt.B * n.n_ra, (size_t)b * n.n_ra);
+}
+
+// Single-precision HVC(RA) part of one interval: thread t of instance b takes the neurons of
+// RAUnit<V> (none when its first one is >= n_ra).
+template <class V, class R, bool kTrack = false>
+__device__ __forceinline__ void interval_ra_v_body(const NetDev<R>& n, const BatchDev<R>& bt, int q, int s0, int s1,
+                                                   const RAStep<R>& rc, int t, int b)
+{
+    constexpr int N = Lanes<V>::n;
+    const int i0 = N * t;
+    uint32_t soma[N] = {}, dend[N] = {};
+    if (i0 < n.n_ra) {
+        RAUnit<V, false> u;
+        u.load(n, bt, rc, t, b, s0);
+        if (q > 0) u.sync_kicks(n, bt, q - 1);
+        u.template steps<kTrack>(n, bt, rc, s0, s1, soma, dend);
+        u.store(n, bt);
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            if (!u.valid[k]) continue;
+            const size_t x = u.at(n, k);
+            ra_spike_stats(bt, x, i0 + k, b, s0, soma[k], dend[k]);
+            if (bt.soma_bits) bt.soma_bits[(size_t)(q & 1) * bt.B * n.n_ra + x] = (int)soma[k];
+            if (bt.act_rows) queue_row(bt, q, (int)x, soma[k]);
         }
     }
 #pragma unroll
-    for (int k = 0; k < N; ++k) {
-        scatter_warp(soma[k], i0 + k, s0, n.T, n.num_steps, n.syncidx, n.ring, n.ra2i_off, n.ra2i_tgt, n.ra2i_wq,
-                     n.ra2i_d, bt.ring_i_exc, (size_t)bt.B * n.n_i, (size_t)b * n.n_i);
-        if (bt.scatter_rara)
-            scatter_warp(soma[k], i0 + k, s0, n.T, n.num_steps, n.syncidx, n.ring, n.rara_off, n.rara_tgt, n.rara_wq,
-                         n.rara_d, bt.ring_ra_exc, (size_t)bt.B * n.n_ra, (size_t)b * n.n_ra);
-    }
+    for (int k = 0; k < N; ++k) ra_scatter(n, bt, soma[k], i0 + k, b, s0);
 }
 
 // Flat grids of the single build's integrators: thread g of a grid over (instance,
@@ -654,8 +721,9 @@ constexpr int kNoiseWalk = 32;       // k_noise_events: threads per block
 constexpr long long kTimestepBits = 0x3f947ae147ae147b;   // 0.02
 constexpr int kEvSegmentEnd = 0x7ffffffe, kEvTrialEnd = 0x7fffffff;   // steps that never come
 
+// Intervals k0 .. k1 - 1 of neuron i (k0 even).
 template <class R>
-__device__ __forceinline__ void noise_gaps_body(const NetDev<R>& n, const BatchDev<R>& bt, int i, int b)
+__device__ __forceinline__ void noise_gaps_body(const NetDev<R>& n, const BatchDev<R>& bt, int i, int b, int k0, int k1)
 {
     static_assert(sizeof(R) == 4, "the noise pre-pass serves the single-precision build");
     if (i >= n.n_i) return;   // one neuron per warp
@@ -671,17 +739,17 @@ __device__ __forceinline__ void noise_gaps_body(const NetDev<R>& n, const BatchD
         const double again = i_noise_interval_fast(stream_word(sid, w + 1));
         return again >= 0.02 ? -again : fabs(r);
     };
-    for (int j = threadIdx.x & 31; 2 * j < bt.ev_cap; j += 32) {
+    for (int j = k0 / 2 + (int)(threadIdx.x & 31); 2 * j < k1; j += 32) {
         const Philox4 w = stream_block(sid, (uint32_t)j);
         gaps[2 * j] = interval(odd ? w.y : w.x, 4u * j + odd);
-        if (2 * j + 1 < bt.ev_cap) gaps[2 * j + 1] = interval(odd ? w.w : w.z, 4u * j + 2u + odd);
+        if (2 * j + 1 < k1) gaps[2 * j + 1] = interval(odd ? w.w : w.z, 4u * j + 2u + odd);
     }
 }
 
 template <class R>
-__global__ void __launch_bounds__(kNoiseThreads) k_noise_gaps(NetDev<R> n, BatchDev<R> bt)
+__global__ void __launch_bounds__(kNoiseThreads) k_noise_gaps(NetDev<R> n, BatchDev<R> bt, int k0, int k1)
 {
-    noise_gaps_body(n, bt, (int)(blockIdx.x * (kNoiseThreads / 32) + threadIdx.x / 32), (int)blockIdx.y);
+    noise_gaps_body(n, bt, (int)(blockIdx.x * (kNoiseThreads / 32) + threadIdx.x / 32), (int)blockIdx.y, k0, k1);
 }
 
 // first_step_after for the walk below: x > 0.02, s_from >= 1.  A double-precision operation
@@ -704,13 +772,14 @@ __device__ __forceinline__ int noise_step_after(const double* T, int num_steps, 
     return num_steps;
 }
 
-// Lists the events of steps up to `end`; `resume`: after the ones an earlier call listed, for
-// which the lists' counts are kept in i_ev_cnt.  The interval of a word lies in the list
-// memory of the inhibitory channel when i_gaps shares it: word w >= 3 at w / 2, so event k
-// reads slot k + 1 or a later one, and writes at slot k or an earlier one.
+// Lists the events of steps up to `end`, with the first `drawn` intervals drawn ahead;
+// `resume`: after the ones an earlier call listed, for which the lists' counts are kept in
+// i_ev_cnt.  A list drawn in one call may share its inhibitory channel's memory with the
+// intervals: word w >= 3 lies at w / 2, so event k reads slot k + 1 or a later one, and
+// writes at slot k or an earlier one.
 template <class R>
 __device__ __forceinline__ void noise_events_body(const NetDev<R>& n, const BatchDev<R>& bt, int i, int b, int end,
-                                                  bool resume)
+                                                  int drawn, bool resume)
 {
     static_assert(sizeof(R) == 4, "the noise pre-pass serves the single-precision build");
     if (i >= n.n_i) return;
@@ -725,7 +794,7 @@ __device__ __forceinline__ void noise_events_body(const NetDev<R>& n, const Batc
     const double* gaps = bt.i_gaps + x * bt.gap_stride;
     const float gscale = (float)(IConst::G_noise / 4294967295.0);
     auto gap = [&](uint32_t w) {
-        return (int)(w >> 1) < bt.ev_cap ? gaps[w >> 1] : i_noise_interval_fast(stream_word(sid, w));
+        return (int)(w >> 1) < drawn ? gaps[w >> 1] : i_noise_interval_fast(stream_word(sid, w));
     };
     double next = gap(word + 1);   // read one event ahead
     while (true) {
@@ -781,25 +850,27 @@ __device__ __forceinline__ void noise_events_body(const NetDev<R>& n, const Batc
 }
 
 template <class R>
-__global__ void __launch_bounds__(kNoiseWalk) k_noise_events(NetDev<R> n, BatchDev<R> bt, int end, bool resume)
+__global__ void __launch_bounds__(kNoiseWalk) k_noise_events(NetDev<R> n, BatchDev<R> bt, int end, int drawn,
+                                                             bool resume)
 {
-    noise_events_body(n, bt, (int)(blockIdx.x * kNoiseWalk + threadIdx.x), (int)blockIdx.y, end, resume);
+    noise_events_body(n, bt, (int)(blockIdx.x * kNoiseWalk + threadIdx.x), (int)blockIdx.y, end, drawn, resume);
 }
 
 // The noise events of one channel of an interneuron (k_noise_events): the next one and the
 // one after it, which is loaded when its predecessor becomes the next, so that taking an
 // event waits for no memory.  A list, and each of its segments, ends with a mark whose step
-// never comes; nothing behind the mark is read until the next segment's first interval.
+// never comes; nothing behind the mark is read before the integration of the next segment
+// begins (`resumed`), which finds the index at the mark and steps over it.
 struct IEvents {
     const int2* ev;
     int idx;
     int2 cur, after;
     template <class R>
-    __device__ __forceinline__ IEvents(const BatchDev<R>& bt, size_t x, int ch)
+    __device__ __forceinline__ IEvents(const BatchDev<R>& bt, size_t x, int ch, bool resumed)
         : ev(bt.i_events + (x * 2 + ch) * bt.ev_cap), idx(bt.i_ev_idx[2 * x + ch])
     {
+        if (resumed) ++idx;
         cur = ev[idx];
-        if (cur.x == kEvSegmentEnd) cur = ev[++idx];
         after = cur;
         if (cur.x < kEvSegmentEnd) after = ev[idx + 1];
     }
@@ -814,51 +885,88 @@ struct IEvents {
     }
 };
 
-// Single-precision HVC(I) part of one interval: noise kicks from the pre-drawn
-// events, DP8 in the layout of ug_i_f32.cuh.
-template <class R, bool kTrack = false>
-__device__ __forceinline__ void interval_i_x_body(const NetDev<R>& n, const BatchDev<R>& bt, int q, int s0, int s1,
-                                                  const IStep<R>& ic, int i, int b)
-{
-    // i: the thread's interneuron (none when i >= n_i), b: its instance
-    static_assert(sizeof(R) == 4, "single-precision interneuron kernel");
-    const bool valid = i < n.n_i;
-    uint32_t fired_bits = 0;
-    if (valid) {
-        const size_t x = (size_t)b * n.n_i + i;
-        IStateR<float> s;
+// A thread's interneuron in registers: neuron i of instance b.
+struct IUnit {
+    IStateR<float> s;
+    IEvents ee, ei;
+    int flag;
+    size_t x;
+
+    template <class R>
+    __device__ __forceinline__ IUnit(const NetDev<R>& n, const BatchDev<R>& bt, int i, int b, bool resumed)
+        : ee(bt, (size_t)b * n.n_i + i, 0, resumed), ei(bt, (size_t)b * n.n_i + i, 1, resumed), x((size_t)b * n.n_i + i)
+    {
+        static_assert(sizeof(R) == 4, "single-precision interneuron integrator");
         s.V = bt.iv[0][x]; s.n = bt.iv[1][x]; s.m = bt.iv[2][x]; s.h = bt.iv[3][x]; s.w = bt.iv[4][x];
         s.Ge = bt.iv[5][x]; s.Gi = bt.iv[6][x];
-        if (q > 0) {
-            const size_t slot = (size_t)((q - 1) % n.ring) * bt.B * n.n_i + x;
-            const long long ae = bt.ring_i_exc[slot];
-            if (ae) {
-                bt.ring_i_exc[slot] = 0;
-                s.Ge = s.Ge + (float)((double)ae * kFixInv);   // raiseE(sum w)
-            }
+        flag = bt.i_flag[x];
+    }
+    // Sync q: raiseE(sum w); read past the L1 cache as RAUnit::sync_kicks.
+    template <class R>
+    __device__ __forceinline__ void sync_kicks(const NetDev<R>& n, const BatchDev<R>& bt, int q)
+    {
+        const size_t slot = (size_t)(q % n.ring) * bt.B * n.n_i + x;
+        const long long ae = __ldcg(&bt.ring_i_exc[slot]);
+        if (ae) {
+            bt.ring_i_exc[slot] = 0;
+            s.Ge = s.Ge + (float)((double)ae * kFixInv);
         }
-        IEvents ee(bt, x, 0), ei(bt, x, 1);
-        int flag = bt.i_flag[x];
+    }
+    // Steps s0..s1, the noise kicks from the pre-drawn events; bit st - s0 of fired is set
+    // where the neuron spiked at step st.
+    template <bool kTrack, class R>
+    __device__ __forceinline__ void steps(const NetDev<R>& n, const BatchDev<R>& bt, const IStep<R>& ic, int s0, int s1,
+                                          int i, int b, uint32_t& fired)
+    {
         for (int st = s0; st <= s1; ++st) {
             if constexpr (kTrack) trace_i_row(bt, n.num_steps, b, i, st, s.V, s.Ge, s.Gi);
-            i_check_f(s.V, flag, fired_bits, st - s0);
+            i_check_f(s.V, flag, fired, st - s0);
             if (st == ee.cur.x) s.Ge += ee.take();
             if (st == ei.cur.x) s.Gi += ei.take();
             i_dp8_x(s, ic);
         }
+    }
+    template <class R>
+    __device__ __forceinline__ void store(const BatchDev<R>& bt) const
+    {
         bt.iv[0][x] = s.V; bt.iv[1][x] = s.n; bt.iv[2][x] = s.m; bt.iv[3][x] = s.h; bt.iv[4][x] = s.w;
         bt.iv[5][x] = s.Ge; bt.iv[6][x] = s.Gi;
         bt.i_ev_idx[2 * x] = ee.idx;
         bt.i_ev_idx[2 * x + 1] = ei.idx;
         bt.i_flag[x] = flag;
-        if (fired_bits) {
-            bt.i_nspk[x] += __popc(fired_bits);
-            if (bt.i_first[x] < 0) bt.i_first[x] = s0 + __ffs(fired_bits) - 1;
-            record_spikes(bt.spk_count, bt.spk_buf, bt.spk_cap, bt.error, b, i, kSpikeInter, fired_bits, s0);
-        }
     }
-    scatter_warp(fired_bits, i, s0, n.T, n.num_steps, n.syncidx, n.ring, n.i2ra_off, n.i2ra_tgt, n.i2ra_wq,
-                 n.i2ra_d, bt.ring_ra_inh, (size_t)bt.B * n.n_ra, (size_t)b * n.n_ra);
+    template <class R>
+    __device__ __forceinline__ void spike_stats(const BatchDev<R>& bt, int i, int b, int s0, uint32_t fired) const
+    {
+        if (!fired) return;
+        bt.i_nspk[x] += __popc(fired);
+        if (bt.i_first[x] < 0) bt.i_first[x] = s0 + __ffs(fired) - 1;
+        record_spikes(bt.spk_count, bt.spk_buf, bt.spk_cap, bt.error, b, i, kSpikeInter, fired, s0);
+    }
+};
+
+// The I->RA kicks of the interval's spikes of interneuron i of instance b; every lane takes part.
+template <class R>
+__device__ __forceinline__ void i_scatter(const NetDev<R>& n, const BatchDev<R>& bt, uint32_t fired, int i, int b, int s0)
+{
+    scatter_warp(fired, i, s0, n.T, n.num_steps, n.syncidx, n.ring, n.i2ra_off, n.i2ra_tgt, n.i2ra_wq, n.i2ra_d,
+                 bt.ring_ra_inh, (size_t)bt.B * n.n_ra, (size_t)b * n.n_ra);
+}
+
+// Single-precision HVC(I) part of one interval: interneuron i (none when i >= n_i) of instance b.
+template <class R, bool kTrack = false>
+__device__ __forceinline__ void interval_i_x_body(const NetDev<R>& n, const BatchDev<R>& bt, int q, int s0, int s1,
+                                                  const IStep<R>& ic, int i, int b)
+{
+    uint32_t fired = 0;
+    if (i < n.n_i) {
+        IUnit u(n, bt, i, b, false);
+        if (q > 0) u.sync_kicks(n, bt, q - 1);
+        u.template steps<kTrack>(n, bt, ic, s0, s1, i, b, fired);
+        u.store(bt);
+        u.spike_stats(bt, i, b, s0, fired);
+    }
+    i_scatter(n, bt, fired, i, b, s0);
 }
 
 template <class R, bool kTrack = false>

@@ -483,8 +483,8 @@ class Engine:
         _check(self.L.ug_set_growth_launch(self.ctx, 1 if one_launch else 0))
 
     def set_interval_fusion(self, fuse: bool = True):
-        """Test batches of 16 trials or more: both integrators of an interval in one launch
-        (default) or two; the results are the same bits."""
+        """Test batches in one cooperative launch, or with both integrators of an interval in one
+        launch (default), or in two launches per interval; the results are the same bits."""
         _check(self.L.ug_set_interval_fusion(self.ctx, 1 if fuse else 0))
 
     def set_growth_trial_shape(self, ra_threads: int = 0, i_threads: int = 0):
