@@ -106,7 +106,8 @@ __device__ __forceinline__ void trial_i_part(const NetDev<R>& n, const BatchDev<
 
 template <class R>
 __global__ void __launch_bounds__(kTrialThreads, 1)
-    k_growth_trial(GrowthDev g, NetDev<R> n, BatchDev<R> bt, RAStep<R> rc, IStep<R> ic, TrialLoop L)
+    k_growth_trial(GrowthDev g, NetDev<R> n, BatchDev<R> bt, RAStep<R> rc,
+                   const __grid_constant__ IStep<R> ic, TrialLoop L)
 {
     extern __shared__ __align__(16) unsigned char trial_smem[];
     __shared__ double sh_T[kSegSteps];

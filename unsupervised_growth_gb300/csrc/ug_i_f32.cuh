@@ -164,14 +164,20 @@ __device__ __forceinline__ void i_check_f(float V, int& flag, uint32_t& fired, i
     flag = flag ? 1 - below : above;
 }
 
+// The step with the series, out of line: it runs a few times in a thousand spikes, and inlined
+// it cost a lone warp's step 90 cycles of 1540.  (p stays where it is, in the kernel's
+// parameters or in shared memory: the parameter is a __grid_constant__.)
+static __device__ __noinline__ IStateR<float> i_dp8_series(IStateR<float> s, const IStep<float>& p)
+{
+    i_dp8_form<true>(s, p);
+    return s;
+}
+
 // One DP8 step, with the series of the vtrap rates where a stage needs it.
 __device__ __forceinline__ void i_dp8_x(IStateR<float>& s, const IStep<float>& p)
 {
     IStateR<float> y = s;
-    if (i_dp8_form<false>(y, p) < kINear) {
-        y = s;
-        i_dp8_form<true>(y, p);
-    }
+    if (i_dp8_form<false>(y, p) < kINear) y = i_dp8_series(s, p);
     s = y;
 }
 

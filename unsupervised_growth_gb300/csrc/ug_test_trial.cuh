@@ -79,8 +79,9 @@ __device__ __forceinline__ bool unit_wait(const unsigned* count, unsigned want0,
 
 // V: the lane type of the HVC(RA) warps (ug_ra_f32.cuh).
 template <class V>
-__global__ void __launch_bounds__(32 * kUnitWarps, 4)
-    k_test_trial(NetDev<float> n, BatchDev<float> bt, RAStep<float> rc, IStep<float> ic, TestLoop L)
+__global__ void __launch_bounds__(32 * kUnitWarps, Lanes<V>::n == 1 ? 1 : 4)
+    k_test_trial(NetDev<float> n, BatchDev<float> bt, RAStep<float> rc, const __grid_constant__ IStep<float> ic,
+                 TestLoop L)
 {
     const int unit = (int)blockIdx.x * kUnitWarps + (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31);
     if (unit < L.ra_pad) {

@@ -971,7 +971,7 @@ __device__ __forceinline__ void interval_i_x_body(const NetDev<R>& n, const Batc
 
 template <class R, bool kTrack = false>
 __global__ void __launch_bounds__(kBlock, UG_I_MIN_BLOCKS) k_interval_i_x(NetDev<R> n, BatchDev<R> bt, int q, int s0, int s1,
-                                                                         IStep<R> ic)
+                                                                         const __grid_constant__ IStep<R> ic)
 {
     int i, b;   // one flat grid over (instance, interneuron)
     flat_unit(blockIdx.x * (unsigned)kBlock + threadIdx.x, (unsigned)n.n_i, bt.B, i, b);
@@ -988,7 +988,8 @@ __global__ void __launch_bounds__(kBlock, UG_I_MIN_BLOCKS) k_interval_i_x(NetDev
 // bodies' code live on every SM and ran 11 % slower (instruction fetch).
 template <class R>
 __global__ void __launch_bounds__(kBlock, UG_RA_MIN_BLOCKS) k_interval_x(NetDev<R> n, BatchDev<R> bt, int q, int s0,
-                                                                       int s1, RAStep<R> rc, IStep<R> ic, unsigned nb_ra)
+                                                                       int s1, RAStep<R> rc,
+                                                                       const __grid_constant__ IStep<R> ic, unsigned nb_ra)
 {
     int u, b;
     if (blockIdx.x < nb_ra) {
