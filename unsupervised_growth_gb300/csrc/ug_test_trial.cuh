@@ -42,14 +42,13 @@ __device__ __forceinline__ unsigned load_acquire(const unsigned* p)
     return v;
 }
 
-// The warp's memory operations so far, then one arrival.
+// The warp's memory operations so far, then one arrival (a release, not a full fence: one
+// 2000/550 trial 26.3 -> 25.3 ms).
 __device__ __forceinline__ void unit_arrive(unsigned* count)
 {
     __syncwarp();
-    if ((threadIdx.x & 31) == 0) {
-        __threadfence();
-        atomicAdd(count, 1u);
-    }
+    if ((threadIdx.x & 31) == 0)
+        asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(count), "r"(1u) : "memory");
 }
 
 // Waits until count[0] >= want0 and count[kCtlWords / 2] >= want1 (each lane of two polls one
