@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(32 * kRowWarps) kl_growth_rows(const GroupMemb
         }
         const GroupMember<R>& m = M[w];
         const int b = it.y / m.n.n_ra, i = it.y - b * m.n.n_ra;
-        g_row(m.g, m.n, m.bt, soma_slice(m.bt, m.n, q), b, i, s0, s1, sh_T, sh, lane);
+        g_row(m.g, m.n, m.bt, (uint32_t)soma_slice(m.bt, m.n, q)[it.y], b, i, s0, s1, sh_T, sh, lane);
         __syncwarp();
     }
 }

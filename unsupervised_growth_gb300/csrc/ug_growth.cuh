@@ -44,6 +44,9 @@ struct SynParams {
     // both thresholds either way), so its only floating-point operation is the decay.
     int int_thresholds;
     long long act_bits, sup_bits;   // the thresholds' bit patterns
+    // LTD leaves a weight of +0 at +0 (its parameters are finite and its time constants
+    // positive), so the delivery of an event onto such a pair needs none of the post events.
+    int zero_stays;
 };
 
 // Device state of the RA->RA synapses of B growing networks of n neurons.
@@ -304,65 +307,129 @@ struct RowShared {
     int rtr[kMaxStreams];      // the run stopped at its quota with more due events behind
 };
 
+// Times as integers of the same order (no time is -0 or NaN).  A double-precision operation,
+// a comparison too, holds a lone warp for 64 cycles however few lanes take part, and a row's
+// delivery is made of comparisons: with integer ones, with the events' loads together and
+// without the LTD of zero weights the deliveries of an interval of a growing 2000 HVC(RA)
+// network took 20 us, 27 before.
+__device__ __forceinline__ long long time_key(double t)
+{
+    const long long b = __double_as_longlong(t);
+    return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+
+// A row's delivery streams in the warp's registers: lane l holds slot l of the stream ring
+// (step and time of the spike, targets delivered so far, length as in st_len).
+struct RowStreams {
+    int S, C, L;
+    double T;
+    template <class R>
+    __device__ __forceinline__ void load(const NetDev<R>& n, const int* stS, const int* stC, const int* stL, int head,
+                                         int num, int lane)
+    {
+        // the whole ring at once, whatever is open: the loads do not wait for head and num
+        S = stS[lane];
+        C = stC[lane];
+        L = stL[lane];
+        const bool open = ((lane - head) & (kMaxStreams - 1)) < num;
+        if (!open) S = C = L = 0;
+        T = open ? n.T[S] : 0.0;
+    }
+};
+static_assert(kMaxStreams == 32, "a lane per slot of the stream ring");
+
 // Gathers the events of row i due by Tlim, at most `quota` per stream: each
 // stream's due events are a prefix of its remaining targets (delivery times
 // rise along a stream), so a run is that prefix, cut at the quota.  Cursors
 // are not moved here.  Returns the event count; nrun runs, truncated = some
 // run stopped at its quota with more due events behind it.
+// A row is a chain of dependent loads (target, then its delay), so kGatherLoads pieces of 32
+// events are loaded together: of one stream, or the first pieces of several.
+constexpr int kGatherLoads = 4;
 template <class R>
-__device__ __forceinline__ int g_gather(const NetDev<R>& n, double Tlim, int head, int num, const int* stS,
-                                        const int* stC, const int* stL, const int* stT, const int* perm,
-                                        const double* Drow, RowShared& sh, int lane, int quota, int& nrun,
-                                        bool& truncated)
+__device__ __forceinline__ int g_gather(const NetDev<R>& n, double Tlim, int head, int num, const RowStreams& st,
+                                        const int* stT, const int* perm, const double* Drow, RowShared& sh, int lane,
+                                        int quota, int& nrun, bool& truncated)
 {
     int total = 0;
     nrun = 0;
     truncated = false;
-    for (int q = 0; q < num; ++q) {
-        const int slot = (head + q) % kMaxStreams;
-        const int L = stL[slot];
-        const int len = L < 0 ? -L : L;
-        const int c = stC[slot];
-        const int spk = stS[slot];
-        const double Tsp = n.T[spk];
-        const int start = total;
-        int taken = 0;
-        while (c + taken < len && taken < quota) {
-            const int k = taken + lane;
-            const int idx = c + k;
-            bool due = false;
-            double td = 0.0;
-            int t = 0;
-            if (idx < len && k < quota) {
-                t = L < 0 ? stT[slot * kMaxNss + idx] : perm[idx];
-                td = Tsp + Drow[t];
-                due = Tlim >= td;
-            }
-            const int nd = __popc(__ballot_sync(0xffffffffu, due));
-            if (due) {
-                sh.td[0][total + lane] = td;
-                sh.tgt[0][total + lane] = t;
-                sh.spk[0][total + lane] = spk;
-            }
-            total += nd;
-            taken += nd;
-            if (nd < 32) break;
+    int t[kGatherLoads];
+    double dl[kGatherLoads];
+    // targets and delays of pieces p0, p0 + 1, .. of the stream in slot
+    auto fetch = [&](int k, int slot, int off) {
+        const int L = __shfl_sync(0xffffffffu, st.L, slot), c = __shfl_sync(0xffffffffu, st.C, slot);
+        const int len = L < 0 ? -L : L, at = off + lane, idx = c + at;
+        t[k] = -1;
+        if (idx < len && at < quota) t[k] = L < 0 ? stT[slot * kMaxNss + idx] : perm[idx];
+    };
+    const int per = num == 1 ? kGatherLoads : num == 2 ? kGatherLoads / 2 : 1;   // pieces a stream per pass
+    for (int q0 = 0; q0 < num; q0 += kGatherLoads / per) {
+#pragma unroll
+        for (int k = 0; k < kGatherLoads; ++k) {
+            const int q = q0 + k / per;
+            t[k] = -1;
+            if (q < num) fetch(k, (head + q) % kMaxStreams, (k % per) * 32);
         }
-        bool trunc = false;
-        if (taken == quota && c + taken < len) {
-            const int idx = c + taken;
-            const int t = L < 0 ? stT[slot * kMaxNss + idx] : perm[idx];
-            trunc = Tlim >= Tsp + Drow[t];
-        }
-        if (taken > 0) {
-            if (lane == 0) {
-                sh.rs[nrun] = start;
-                sh.rq[nrun] = q;
-                sh.rtr[nrun] = trunc ? 1 : 0;
+#pragma unroll
+        for (int k = 0; k < kGatherLoads; ++k) dl[k] = t[k] >= 0 ? Drow[t[k]] : 0.0;
+#pragma unroll
+        for (int j = 0; j < kGatherLoads; ++j) {
+            const int q = q0 + j;
+            if (j >= kGatherLoads / per || q >= num) break;
+            const int slot = (head + q) % kMaxStreams;
+            const int L = __shfl_sync(0xffffffffu, st.L, slot), c = __shfl_sync(0xffffffffu, st.C, slot);
+            const int spk = __shfl_sync(0xffffffffu, st.S, slot), len = L < 0 ? -L : L;
+            const double Tsp = __shfl_sync(0xffffffffu, st.T, slot);
+            const int start = total;
+            int taken = 0;
+            bool more = true;
+            auto take = [&](int tk, double dk) {
+                const double td = Tsp + dk;
+                const bool due = tk >= 0 && time_key(Tlim) >= time_key(td);
+                const int nd = __popc(__ballot_sync(0xffffffffu, due));
+                if (due) {
+                    sh.td[0][total + lane] = td;
+                    sh.tgt[0][total + lane] = tk;
+                    sh.spk[0][total + lane] = spk;
+                }
+                total += nd;
+                taken += nd;
+                more = nd == 32;
+            };
+#pragma unroll
+            for (int k = 0; k < kGatherLoads; ++k)
+                if (k / per == j && more) take(t[k], dl[k]);
+            while (more && c + taken < len && taken < quota) {
+                int t2[kGatherLoads];
+                double d2[kGatherLoads];
+#pragma unroll
+                for (int k = 0; k < kGatherLoads; ++k) {
+                    const int at = taken + 32 * k + lane;
+                    t2[k] = -1;
+                    if (c + at < len && at < quota) t2[k] = L < 0 ? stT[slot * kMaxNss + c + at] : perm[c + at];
+                }
+#pragma unroll
+                for (int k = 0; k < kGatherLoads; ++k) d2[k] = t2[k] >= 0 ? Drow[t2[k]] : 0.0;
+#pragma unroll
+                for (int k = 0; k < kGatherLoads; ++k)
+                    if (more) take(t2[k], d2[k]);
             }
-            ++nrun;
+            bool trunc = false;
+            if (taken == quota && c + taken < len) {
+                const int tn = L < 0 ? stT[slot * kMaxNss + c + taken] : perm[c + taken];
+                trunc = Tlim >= Tsp + Drow[tn];
+            }
+            if (taken > 0) {
+                if (lane == 0) {
+                    sh.rs[nrun] = start;
+                    sh.rq[nrun] = q;
+                    sh.rtr[nrun] = trunc ? 1 : 0;
+                }
+                ++nrun;
+            }
+            truncated |= trunc;
         }
-        truncated |= trunc;
     }
     if (lane == 0) sh.rs[nrun] = total;
     __syncwarp();
@@ -372,7 +439,8 @@ __device__ __forceinline__ int g_gather(const NetDev<R>& n, double Tlim, int hea
 // Event order of the reference's queue: (delivery time, target), earlier spike first on a tie.
 __device__ __forceinline__ bool ev_less(double ta, int ga, int sa, double tb, int gb, int sb)
 {
-    return ta < tb || (ta == tb && (ga < gb || (ga == gb && sa < sb)));
+    const long long a = time_key(ta), b = time_key(tb);
+    return a < b || (a == b && (ga < gb || (ga == gb && sa < sb)));
 }
 
 // Ranks the gathered events into buffer 1 in queue order.  Runs are merged by
@@ -434,68 +502,85 @@ __device__ __forceinline__ bool g_rank(RowShared& sh, int total, int nrun, int l
 // desaturates).
 struct RowEv {
     bool has, changing, is_active, do_write, new_pre;
-    int t, spk, pc, sd;
+    int t, spk, pc, sd, su;
     size_t ij;
-    double wv, w2;
+    double td, wv, w2, plast, Dij;
+    short4 pre;
 };
 
-// Event (td, t, spk) of row i, delivered at the first step >= sa (Tseg = T[sa..])
-// whose time reaches td; has = false evaluates nothing.
+// The loads of event (td, t, spk) of row i, all independent of each other; has = false loads
+// nothing.
 template <class R>
-__device__ __forceinline__ void g_eval_ev(const GrowthDev& g, const NetDev<R>& n, int b, int i, int sa,
-                                          const double* Tseg, bool has, double td, int t, int spk, int rem, int sc,
-                                          RowEv& v)
+__device__ __forceinline__ void g_eval_load(const GrowthDev& g, int b, int i, bool has, double td, int t, int spk,
+                                            RowEv& v)
 {
-    const SynParams& sp = g.sp;
     v.has = has;
     v.changing = v.do_write = v.new_pre = v.is_active = false;
-    v.t = -1;
-    v.wv = v.w2 = 0.0;
-    v.pc = v.spk = 0;
-    v.sd = sa;
-    v.ij = 0;
-    if (!v.has) return;
-    v.t = t;
+    v.t = has ? t : -1;
     v.spk = spk;
-    while (Tseg[v.sd - sa] < td) ++v.sd;
-    v.ij = gidx(g, b, i, v.t);
-    // loads of the pair and the target, issued together
-    const int act = g.active[v.ij];
-    const int su = g.super[v.ij];
-    v.wv = g.W[v.ij];
-    v.pc = g.pre_cnt[v.ij];
-    const int ls = g.pre_step[v.ij * kPreRing + ((v.pc + kPreRing - 1) % kPreRing)];
-    const double plast = g.post_last[(size_t)b * g.n + v.t];
-    const double Dij = g.D[v.ij];
-    v.is_active = act == 1;
-    // new pre-synaptic event: first, or more than 30 ms after the previous one
-    v.new_pre = v.pc == 0 || td > n.T[v.pc ? ls : 0] + Dij + 30.0;
-    v.w2 = v.wv;
-    const double now = Tseg[v.sd - sa];
-    // LTD against the target's post events in [now - 100, now]; none when the newest is older
-    if (v.new_pre && (sc != sp.Nss || su == 1) && plast >= now - 100.0) {
-        const int np = post_num(g, b, v.t);
-        for (int k = 0; k < np; ++k) {
-            const double tp = n.T[post_at(g, b, v.t, k)];
-            if (!(tp >= now - 100.0)) continue;
-            g_LTD(sp, v.w2, tp - td);
-            v.do_write = true;
-            v.changing |= (v.w2 >= sp.ACTIVATION_THRESHOLD && !v.is_active && rem == 0) ||
-                          (v.w2 >= sp.SUPERSYNAPSE_THRESHOLD && su == 0 && sc < sp.Nss) ||
-                          (v.w2 < sp.SUPERSYNAPSE_THRESHOLD && su == 1) ||
-                          (v.w2 < sp.ACTIVATION_THRESHOLD && v.is_active);
-        }
+    v.td = td;
+    v.wv = v.plast = v.Dij = 0.0;
+    v.pc = v.su = 0;
+    v.pre = make_short4(0, 0, 0, 0);
+    v.ij = gidx(g, b, i, has ? t : 0);
+    if (has) {
+        v.is_active = g.active[v.ij] == 1;
+        v.su = g.super[v.ij];
+        v.wv = g.W[v.ij];
+        v.pc = g.pre_cnt[v.ij];
+        v.pre = *reinterpret_cast<const short4*>(g.pre_step + v.ij * kPreRing);   // the pair's whole ring
+        v.plast = g.post_last[(size_t)b * g.n + t];
+        v.Dij = g.D[v.ij];
     }
 }
 
+// The step that delivers a loaded event (the first >= sa, Tseg = T[sa..sb], whose time reaches
+// td), and when the pair's newest pre-synaptic event was.
 template <class R>
-__device__ __forceinline__ void g_eval(const GrowthDev& g, const NetDev<R>& n, int b, int i, int sa,
-                                       const double* Tseg, const RowShared& sh, int e, int total, int rem, int sc,
-                                       RowEv& v)
+__device__ __forceinline__ double g_eval_time(const NetDev<R>& n, int sa, int sb, const double* Tseg, RowEv& v)
 {
-    const bool has = e < total;
-    g_eval_ev(g, n, b, i, sa, Tseg, has, has ? sh.td[1][e] : 0.0, has ? sh.tgt[1][e] : -1, has ? sh.spk[1][e] : 0,
-              rem, sc, v);
+    const long long k = time_key(v.td);
+    int sd = sa;
+    for (int j = 0; j < sb - sa; ++j) sd += time_key(Tseg[j]) < k;   // T[sb] >= td
+    v.sd = sd;
+    const int lr = (v.pc + kPreRing - 1) % kPreRing;
+    const int ls = lr == 0 ? v.pre.x : lr == 1 ? v.pre.y : lr == 2 ? v.pre.z : v.pre.w;
+    return v.pc ? n.T[ls] : 0.0;
+}
+
+__device__ __forceinline__ bool g_row_changes(const SynParams& sp, double w, bool is_active, int su, int rem, int sc)
+{
+    return (w >= sp.ACTIVATION_THRESHOLD && !is_active && rem == 0) ||
+           (w >= sp.SUPERSYNAPSE_THRESHOLD && su == 0 && sc < sp.Nss) || (w < sp.SUPERSYNAPSE_THRESHOLD && su == 1) ||
+           (w < sp.ACTIVATION_THRESHOLD && is_active);
+}
+
+// The decision on a loaded event; tprev from g_eval_time.
+template <class R>
+__device__ __forceinline__ void g_eval_decide(const GrowthDev& g, const NetDev<R>& n, int b, int sa,
+                                              const double* Tseg, double tprev, int rem, int sc, RowEv& v)
+{
+    const SynParams& sp = g.sp;
+    v.w2 = v.wv;
+    if (!v.has) return;
+    // new pre-synaptic event: first, or more than 30 ms after the previous one
+    v.new_pre = v.pc == 0 || time_key(v.td) > time_key(tprev + v.Dij + 30.0);
+    if (!v.new_pre || (sc == sp.Nss && v.su != 1)) return;
+    // LTD against the target's post events in [now - 100, now]; none when the newest is older
+    const double now = Tseg[v.sd - sa], from = now - 100.0;
+    if (time_key(v.plast) < time_key(from)) return;
+    if (sp.zero_stays && __double_as_longlong(v.wv) == 0) {   // stays 0 whatever the events are
+        v.changing = g_row_changes(sp, 0.0, v.is_active, v.su, rem, sc);
+        return;
+    }
+    const int np = post_num(g, b, v.t);
+    for (int k = 0; k < np; ++k) {
+        const double tp = n.T[post_at(g, b, v.t, k)];
+        if (!(tp >= from)) continue;
+        g_LTD(sp, v.w2, tp - v.td);
+        v.do_write = true;
+        v.changing |= g_row_changes(sp, v.w2, v.is_active, v.su, rem, sc);
+    }
 }
 
 template <class R>
@@ -525,8 +610,8 @@ constexpr int kEvPerLane = 4;   // events a lane evaluates per chunk (their load
 // target twice: it is cut to 32 events and the repeats take the exact path.
 template <class R>
 __device__ __forceinline__ void g_process(const GrowthDev& g, const NetDev<R>& n, const BatchDev<R>& bt, int b, int i,
-                                          size_t r, int sa, const double* Tseg, int total, const RowShared& sh,
-                                          int lane)
+                                          size_t r, int sa, int sb, const double* Tseg, int total,
+                                          const RowShared& sh, int lane)
 {
     int base = 0;
     while (base < total) {
@@ -541,9 +626,17 @@ __device__ __forceinline__ void g_process(const GrowthDev& g, const NetDev<R>& n
         }
         const int slices = __all_sync(0xffffffffu, one) ? kEvPerLane : 1;
         RowEv v[kEvPerLane];
+        double tprev[kEvPerLane];
 #pragma unroll
-        for (int k = 0; k < kEvPerLane; ++k)
-            g_eval(g, n, b, i, sa, Tseg, sh, k < slices ? base + k * 32 + lane : total, total, rem, sc, v[k]);
+        for (int k = 0; k < kEvPerLane; ++k) {
+            const int e = base + k * 32 + lane;
+            const bool has = k < slices && e < total;
+            g_eval_load<R>(g, b, i, has, has ? sh.td[1][e] : 0.0, has ? sh.tgt[1][e] : -1, has ? sh.spk[1][e] : 0, v[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < kEvPerLane; ++k) tprev[k] = g_eval_time(n, sa, sb, Tseg, v[k]);
+#pragma unroll
+        for (int k = 0; k < kEvPerLane; ++k) g_eval_decide(g, n, b, sa, Tseg, tprev[k], rem, sc, v[k]);
         if (slices == 1) {
             const unsigned same = __match_any_sync(0xffffffffu, v[0].has ? v[0].t : -1 - lane);
             if (v[0].has && __popc(same) > 1 && lane != __ffs(same) - 1) v[0].changing = true;
@@ -579,15 +672,15 @@ __device__ __forceinline__ void g_process(const GrowthDev& g, const NetDev<R>& n
 
 // One warp, row i of instance b, steps from..to of the interval s0..s1
 // (sh_T holds T[s0..s1]); a spike at `from` has already opened its stream
-// when opened_at_from is set.  head / num: the row's stream ring.
+// when opened_at_from is set.  bits: the row's somatic spikes of the interval; head / num:
+// its stream ring, st: the ring's slots (cursors are written back at the end).
 template <class R>
 __device__ __forceinline__ void g_row_range(const GrowthDev& g, const NetDev<R>& n, const BatchDev<R>& bt,
-                                            const int* soma, int b, int i, int s0, int from, int to,
+                                            uint32_t bits, int b, int i, int s0, int from, int to,
                                             bool opened_at_from, const double* sh_T, RowShared& sh, int lane,
-                                            int& head, int& num)
+                                            int& head, int& num, RowStreams& st)
 {
     const size_t r = (size_t)b * g.n + i;
-    const uint32_t bits = (uint32_t)soma[(size_t)b * n.n_ra + i];
     const int s1 = to;
     int* stS = g.st_step + r * kMaxStreams;
     int* stC = g.st_cursor + r * kMaxStreams;
@@ -598,9 +691,12 @@ __device__ __forceinline__ void g_row_range(const GrowthDev& g, const NetDev<R>&
     int sa = from;
     while (sa <= s1) {
         if (((bits >> (sa - s0)) & 1u) && !(opened_at_from && sa == from)) {
+            stC[lane] = st.C;
+            __syncwarp();
             if (lane == 0) num = g_open_stream(g, r, sa, sh_T[sa - s0], Drow, head, num, stS, stC, stL, stT);
             num = __shfl_sync(0xffffffffu, num, 0);
             __syncwarp();
+            st.load(n, stS, stC, stL, head, num, lane);
         }
         const uint32_t later = (sa - s0 + 1) < 32 ? bits >> (sa - s0 + 1) : 0u;
         const int sb = later ? min(sa + __ffs(later) - 1, s1) : s1;
@@ -613,17 +709,19 @@ __device__ __forceinline__ void g_row_range(const GrowthDev& g, const NetDev<R>&
         while (num > 0) {
             int nrun = 0;
             bool trunc = false;
-            const int total = g_gather(n, sh_T[sb - s0], head, num, stS, stC, stL, stT, perm, Drow, sh, lane, quota,
-                                       nrun, trunc);
+            const int total = g_gather(n, sh_T[sb - s0], head, num, st, stT, perm, Drow, sh, lane, quota, nrun, trunc);
             if (total == 0) break;
             const bool sorted = g_rank(sh, total, nrun, lane);
             if (!sorted && trunc) {
                 // a stream whose (delay, target) order differs from its queue
                 // order and does not fit: deliver step by step, one event at a time
+                stC[lane] = st.C;
+                __syncwarp();
                 for (int s = sa; s <= sb; ++s) {
                     if (lane == 0) g_drain_seq(g, n, bt, b, i, s, sh_T[s - s0], head, num, stS, stC, stL, stT, perm, Drow);
                     __syncwarp();
                 }
+                st.load(n, stS, stC, stL, head, num, lane);
                 break;
             }
             // the cut: smallest last key among the truncated runs
@@ -651,11 +749,12 @@ __device__ __forceinline__ void g_row_range(const GrowthDev& g, const NetDev<R>&
                 }
                 P = lo;
             }
-            g_process(g, n, bt, b, i, r, sa, sh_T + (sa - s0), P, sh, lane);
+            g_process(g, n, bt, b, i, r, sa, sb, sh_T + (sa - s0), P, sh, lane);
             // advance each stream past its processed prefix
+            int adv = 0;
             if (lane < nrun) {
                 const int a0 = sh.rs[lane], a1 = sh.rs[lane + 1];
-                int adv = a1 - a0;
+                adv = a1 - a0;
                 if (trunc) {
                     int lo = a0, hi = a1;
                     while (lo < hi) {
@@ -665,34 +764,39 @@ __device__ __forceinline__ void g_row_range(const GrowthDev& g, const NetDev<R>&
                     }
                     adv = lo - a0;
                 }
-                stC[(head + sh.rq[lane]) % kMaxStreams] += adv;
+            }
+            for (int k = 0; k < nrun; ++k) {
+                const int ak = __shfl_sync(0xffffffffu, adv, k);
+                if (lane == (head + sh.rq[k]) % kMaxStreams) st.C += ak;
             }
             __syncwarp();
             if (!trunc) break;
         }
         // retire exhausted streams at the head of the ring
         while (num > 0) {
-            const int L = stL[head];
-            if (stC[head] < (L < 0 ? -L : L)) break;
+            const int L = __shfl_sync(0xffffffffu, st.L, head);
+            if (__shfl_sync(0xffffffffu, st.C, head) < (L < 0 ? -L : L)) break;
             head = (head + 1) % kMaxStreams;
             --num;
         }
-        __syncwarp();
         sa = sb + 1;
     }
+    stC[lane] = st.C;
+    __syncwarp();
 }
 
-// One warp, row i of instance b over the whole interval s0..s1.  Returns the
-// row's live streams after it.
+// One warp, row i of instance b over the whole interval s0..s1, its somatic spikes of the
+// interval in bits.  Returns the row's live streams after it.
 template <class R>
-__device__ __forceinline__ int g_row(const GrowthDev& g, const NetDev<R>& n, const BatchDev<R>& bt, const int* soma,
+__device__ __forceinline__ int g_row(const GrowthDev& g, const NetDev<R>& n, const BatchDev<R>& bt, uint32_t bits,
                                      int b, int i, int s0, int s1, const double* sh_T, RowShared& sh, int lane)
 {
     const size_t r = (size_t)b * g.n + i;
-    const uint32_t bits = (uint32_t)soma[(size_t)b * n.n_ra + i];
     int head = g.st_head[r], num = g.st_num[r];
     if (bits == 0 && num == 0) return 0;
-    g_row_range(g, n, bt, soma, b, i, s0, s0, s1, false, sh_T, sh, lane, head, num);
+    RowStreams st;
+    st.load(n, g.st_step + r * kMaxStreams, g.st_cursor + r * kMaxStreams, g.st_len + r * kMaxStreams, head, num, lane);
+    g_row_range(g, n, bt, bits, b, i, s0, s0, s1, false, sh_T, sh, lane, head, num, st);
     if (lane == 0) {
         g.st_head[r] = head;
         g.st_num[r] = num;
@@ -745,8 +849,11 @@ __device__ __forceinline__ void g_row_heavy(const GrowthDev& g, const NetDev<R>&
         int head = g.st_head[r], num = g.st_num[r];
         int mode = 1;
         if (bits) {
-            if (from > s0 && num > 0)
-                g_row_range(g, n, bt, soma, b, i, s0, s0, from - 1, false, sh_T, sh, lane, head, num);
+            if (from > s0 && num > 0) {
+                RowStreams st;
+                st.load(n, stS, stC, stL, head, num, lane);
+                g_row_range(g, n, bt, bits, b, i, s0, s0, from - 1, false, sh_T, sh, lane, head, num, st);
+            }
             if (lane == 0) {
                 const int before = num;
                 num = g_open_stream(g, r, from, sh_T[from - s0], Drow, head, num, stS, stC, stL, stT);
@@ -800,27 +907,30 @@ __device__ __forceinline__ void g_row_heavy(const GrowthDev& g, const NetDev<R>&
         for (int p = 0;; p ^= 1) {
             const int rem = g.remodeled[r], sc = g.sup_cnt[r];
             RowEv v[kEvPerLane];
-            double tdk[kEvPerLane];
+            double tprev[kEvPerLane];
+            int t[kEvPerLane];
 #pragma unroll
             for (int k = 0; k < kEvPerLane; ++k) {
                 const int idx = cur + w * 32 * kEvPerLane + k * 32 + lane;
-                int t = -1;
-                double td = 0.0;
-                bool due = false;
-                if (idx < len) {
-                    t = perm[idx];
-                    td = Tsp + Drow[t];
-                    due = Tlim >= td;
-                }
-                tdk[k] = td;
-                g_eval_ev(g, n, b, i, from, Tseg, due, td, t, spk, rem, sc, v[k]);
+                t[k] = idx < len ? perm[idx] : -1;
             }
+#pragma unroll
+            for (int k = 0; k < kEvPerLane; ++k) tprev[k] = t[k] >= 0 ? Drow[t[k]] : 0.0;
+#pragma unroll
+            for (int k = 0; k < kEvPerLane; ++k) {
+                const double td = Tsp + tprev[k];
+                g_eval_load<R>(g, b, i, t[k] >= 0 && time_key(Tlim) >= time_key(td), td, t[k], spk, v[k]);
+            }
+#pragma unroll
+            for (int k = 0; k < kEvPerLane; ++k) tprev[k] = g_eval_time(n, from, s1, Tseg, v[k]);
+#pragma unroll
+            for (int k = 0; k < kEvPerLane; ++k) g_eval_decide(g, n, b, from, Tseg, tprev[k], rem, sc, v[k]);
             int due_here = 0;
 #pragma unroll
             for (int k = 0; k < kEvPerLane; ++k) {
                 const int e = w * 32 * kEvPerLane + k * 32 + lane;   // position in the pass
                 if (v[k].has) {
-                    hs.td[p][e] = tdk[k];
+                    hs.td[p][e] = v[k].td;
                     hs.tgt[p][e] = v[k].t;
                     ++due_here;
                 }
@@ -836,7 +946,7 @@ __device__ __forceinline__ void g_row_heavy(const GrowthDev& g, const NetDev<R>&
             for (int e = threadIdx.x; e < ndue; e += blockDim.x) {
                 const double ta = e ? hs.td[p][e - 1] : prev_td;
                 const int ga = e ? hs.tgt[p][e - 1] : prev_t;
-                if (!(ta < hs.td[p][e] || (ta == hs.td[p][e] && ga < hs.tgt[p][e]))) hs.unsorted[p] = 1;
+                if (!ev_less(ta, ga, 0, hs.td[p][e], hs.tgt[p][e], 0)) hs.unsorted[p] = 1;
             }
             if (threadIdx.x == 0) {   // the next pass's reductions (last read a pass ago)
                 hs.first[p ^ 1] = kHeavyChunk;
@@ -877,7 +987,9 @@ __device__ __forceinline__ void g_row_heavy(const GrowthDev& g, const NetDev<R>&
     __syncthreads();
     if (w == 0) {
         int head = hs.head, num = hs.num;
-        g_row_range(g, n, bt, soma, b, i, s0, from, s1, bits != 0, sh_T, sh, lane, head, num);
+        RowStreams st;
+        st.load(n, stS, stC, stL, head, num, lane);
+        g_row_range(g, n, bt, bits, b, i, s0, from, s1, bits != 0, sh_T, sh, lane, head, num, st);
         if (lane == 0) {
             g.st_head[r] = head;
             g.st_num[r] = num;
@@ -910,7 +1022,8 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_growth_rows(GrowthDev g, Net
         if (lane == 0) atomicOr(g.error, kErrEventCapacity);
         return;
     }
-    g_row(g, n, bt, soma_slice(bt, n, q), b, i, s0, s1, sh_T, reinterpret_cast<RowShared*>(row_smem)[w], lane);
+    g_row(g, n, bt, (uint32_t)soma_slice(bt, n, q)[(size_t)b * n.n_ra + i], b, i, s0, s1, sh_T,
+          reinterpret_cast<RowShared*>(row_smem)[w], lane);
 }
 
 // New post-synaptic events of the interval in the reference's order: steps

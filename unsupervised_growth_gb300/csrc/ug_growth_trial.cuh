@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(kTrialThreads, 1)
         const int nrows = min(bt.act_cnt[q & 1], bt.act_cap);
         const int2* rows = bt.act_rows + (size_t)(q & 1) * bt.act_cap;
         for (int e = blk * kTrialWarps + w; e < nrows; e += gridDim.x * kTrialWarps) {
-            g_row(g, n, bt, soma_slice(bt, n, q), 0, rows[e].y, s0, s1, sh_T, sh, lane);
+            g_row(g, n, bt, (uint32_t)soma_slice(bt, n, q)[rows[e].y], 0, rows[e].y, s0, s1, sh_T, sh, lane);
             __syncwarp();
         }
         if (!grid_barrier_bounded(L.bar, ++passed, g.error, kErrTimeout)) return;

@@ -1013,6 +1013,8 @@ ug_status NetImpl<R>::growth_init(cudaStream_t st)
     g.sp.int_thresholds = (h.syn.ACTIVATION_THRESHOLD > 0.0 && h.syn.SUPERSYNAPSE_THRESHOLD > 0.0 &&
                            std::isfinite(h.syn.ACTIVATION_THRESHOLD) && std::isfinite(h.syn.SUPERSYNAPSE_THRESHOLD))
                               ? 1 : 0;
+    g.sp.zero_stays = (std::isfinite(h.syn.A_D) && std::isfinite(h.syn.T_0) && std::isfinite(h.syn.T_D) && h.syn.T_D > 0.0 &&
+                       std::isfinite(h.syn.TAU_D) && h.syn.TAU_D > 0.0) ? 1 : 0;
     std::memcpy(&g.sp.act_bits, &h.syn.ACTIVATION_THRESHOLD, sizeof(double));
     std::memcpy(&g.sp.sup_bits, &h.syn.SUPERSYNAPSE_THRESHOLD, sizeof(double));
     UG_CUDA(ug::epilogue_bulk_grid<R>(n, 1, &g.epi_blocks));
