@@ -22,7 +22,11 @@
 namespace ug {
 
 constexpr int kUnitWarps = 4;    // warps (units) per block, one per SM scheduler
-constexpr int kCtlWords = 64;    // arrival counters of an instance: HVC(RA) at 0, HVC(I) at kCtlWords / 2
+// Arrival counters of an instance, a 128-byte line each: HVC(RA), and HVC(I) apart for even and
+// odd intervals.  An HVC(RA) warp waits for both kinds, so none is a whole interval ahead of
+// another; an interneuron warp waits for the HVC(RA) warps only and can finish an interval
+// before a slower one has finished the last, which one common count would take for it.
+constexpr int kCtlWords = 96, kCtlInter = 32;
 
 // The launch's part of the trial: intervals q0 .. q1 - 1 (Q: the steps after the last sync).
 struct TestLoop {
@@ -34,6 +38,9 @@ struct TestLoop {
 };
 
 __device__ __forceinline__ unsigned* unit_ctl(const TestLoop& L, int b) { return L.ctl + (size_t)b * kCtlWords; }
+
+// The interneurons' counter of interval q; it reaches (q / 2 + 1) times their warps.
+__device__ __forceinline__ unsigned* inter_ctl(unsigned* ctl, int q) { return ctl + kCtlInter * (1 + (q & 1)); }
 
 __device__ __forceinline__ unsigned load_acquire(const unsigned* p)
 {
@@ -51,13 +58,14 @@ __device__ __forceinline__ void unit_arrive(unsigned* count)
         asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(count), "r"(1u) : "memory");
 }
 
-// Waits until count[0] >= want0 and count[kCtlWords / 2] >= want1 (each lane of two polls one
-// of them); false if the wait, or another warp's, gave up.
-__device__ __forceinline__ bool unit_wait(const unsigned* count, unsigned want0, unsigned want1, int* error)
+// Waits until *count >= want0 and *inter >= want1 (each lane of two polls one of them); false
+// if the wait, or another warp's, gave up.
+__device__ __forceinline__ bool unit_wait(const unsigned* count, unsigned want0, const unsigned* inter, unsigned want1,
+                                          int* error)
 {
     const int lane = threadIdx.x & 31;
     const unsigned want = lane == 0 ? want0 : lane == 1 ? want1 : 0u;
-    const unsigned* p = count + (lane == 1 ? kCtlWords / 2 : 0);
+    const unsigned* p = lane == 1 ? inter : count;
     uint64_t t0 = 0;
     for (unsigned k = 0;; ++k) {
         const bool here = want == 0u || load_acquire(p) >= want;
@@ -98,7 +106,9 @@ __global__ void __launch_bounds__(32 * kUnitWarps, Lanes<V>::n == 1 ? 1 : 4)
             for (int k = 0; k < N; ++k) u.valid[k] = false;
         int s0 = first;
         for (int q = L.q0; q < L.q1; ++q) {
-            if (q > L.q0 && !unit_wait(ctl, (unsigned)q * L.ra_units, (unsigned)q * L.i_units, bt.error)) return;
+            if (q > L.q0 && !unit_wait(ctl, (unsigned)q * L.ra_units, inter_ctl(ctl, q - 1),
+                                       (unsigned)((q - 1) / 2 + 1) * L.i_units, bt.error))
+                return;
             if (q > 0) u.sync_kicks(n, bt, q - 1);
             if (q == L.Q) break;
             const int s1 = L.sync_end[q];
@@ -122,7 +132,7 @@ __global__ void __launch_bounds__(32 * kUnitWarps, Lanes<V>::n == 1 ? 1 : 4)
         IUnit u(n, bt, any ? i : 0, b, L.q0 > 0);
         int s0 = L.q0 == 0 ? 1 : L.sync_end[L.q0 - 1] + 1;
         for (int q = L.q0; q < L.q1; ++q) {
-            if (q > L.q0 && !unit_wait(ctl, (unsigned)q * L.ra_units, 0u, bt.error)) return;
+            if (q > L.q0 && !unit_wait(ctl, (unsigned)q * L.ra_units, ctl, 0u, bt.error)) return;
             if (q > 0 && any) u.sync_kicks(n, bt, q - 1);
             if (q == L.Q) break;
             const int s1 = L.sync_end[q];
@@ -130,7 +140,7 @@ __global__ void __launch_bounds__(32 * kUnitWarps, Lanes<V>::n == 1 ? 1 : 4)
             u.template steps<false>(n, bt, ic, s0, s1, i, b, fired);
             if (!any) fired = 0;
             i_scatter(n, bt, fired, i, b, s0);
-            unit_arrive(ctl + kCtlWords / 2);
+            unit_arrive(inter_ctl(ctl, q));
             u.spike_stats(bt, i, b, s0, fired);
             s0 = s1 + 1;
         }
