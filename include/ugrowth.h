@@ -154,19 +154,20 @@ ug_status ug_run_group(ug_ctx* ctx, ug_group_item* items, int32_t n_items);
 ug_status ug_set_group_launch(ug_ctx* ctx, int32_t ra_blocks_per_sm, int32_t i_blocks_per_sm, int32_t overlap);
 /* Launch shape of single-network growth trials (ug_run_growth_trials), no counterpart in the
  * reference, whose loop over sync intervals is NetworkGrowthSimulator.cpp:8923-9564.
- * one_launch 1 (the default): each trial's intervals run in one cooperative kernel with
- * bounded grid barriers between phases, when the network's blocks can all be resident at
+ * one_launch 1 (the default): each trial's intervals run in one cooperative kernel, with
+ * bounded grid barriers between phases (double build) or bounded waits of each role on what
+ * it reads (single build), when the network's blocks can all be resident at
  * once (else, and while recording traces or inhibition, the per-interval launches run);
- * a barrier not reached within about a second ends the trial with UG_ETIMEOUT.
+ * a barrier or wait not satisfied within about a second ends the trial with UG_ETIMEOUT.
  * 0: the per-interval launches (several kernels per sync interval).  Results are the
  * same bits either way. */
 ug_status ug_set_growth_launch(ug_ctx* ctx, int32_t one_launch);
 /* Block shape of the one-launch growth trial, no counterpart in the reference (its neurons
  * step one after another in each rank's loop, NetworkGrowthSimulator.cpp:8923-8950):
- * integrating threads per block of the HVC(RA) and of the HVC(I) role, each 0 (the default,
- * 32: one integrating warp per block; the single build's RA threads step two neurons each)
+ * integrating threads per block of the HVC(RA) and of the HVC(I) role, each 0 (the default:
+ * one integrating warp per block, in the single build more where the network's size needs it)
  * or a multiple of 32 in [32, 256].  Wider roles put a network's neurons on fewer SMs, with
- * more integrating warps sharing an SM scheduler between two grid barriers.
+ * more integrating warps sharing an SM scheduler.
  * Results are the same bits for every shape; a shape whose blocks cannot all be resident
  * runs the per-interval launches.  UG_EINVAL for other widths. */
 ug_status ug_set_growth_trial_shape(ug_ctx* ctx, int32_t ra_threads, int32_t i_threads);

@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(256) kl_growth_reset(const GroupMember<R>* mem
 
 // One warp per queued row of interval q (the warp path).  T = the group's time grid.
 template <class R>
-__global__ void __launch_bounds__(32 * kRowWarps) kl_growth_rows(const GroupMember<R>* members, const int2* rows,
+__global__ void __launch_bounds__(32 * kRowWarps, 1) kl_growth_rows(const GroupMember<R>* members, const int2* rows,
                                                                  const int* act_cnt, int act_cap, const double* T,
                                                                  int q, int s0, int s1)
 {

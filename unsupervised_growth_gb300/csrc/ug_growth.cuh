@@ -443,23 +443,21 @@ __device__ __forceinline__ bool ev_less(double ta, int ga, int sa, double tb, in
     return a < b || (a == b && (ga < gb || (ga == gb && sa < sb)));
 }
 
-// Ranks the gathered events into buffer 1 in queue order.  Runs are merged by
+// Ranks the gathered events in queue order: into buffer 1, or, where the gathered order is
+// the queue's already (one run), as they lie in buffer 0; `buf`: which.  Runs are merged by
 // binary search; a run whose (time, target) order differs from its (delay,
 // target) order (delivery times that round equal) takes the quadratic rank.
-__device__ __forceinline__ bool g_rank(RowShared& sh, int total, int nrun, int lane)
+__device__ __forceinline__ bool g_rank(RowShared& sh, int total, int nrun, int lane, int& buf)
 {
     bool sorted = true;
+    buf = 1;
     for (int e = lane; e + 1 < total; e += 32)
         if (sh.spk[0][e] == sh.spk[0][e + 1] &&
             !ev_less(sh.td[0][e], sh.tgt[0][e], 0, sh.td[0][e + 1], sh.tgt[0][e + 1], 0))
             sorted = false;
     sorted = __all_sync(0xffffffffu, sorted);
     if (sorted && nrun == 1) {
-        for (int e = lane; e < total; e += 32) {
-            sh.td[1][e] = sh.td[0][e];
-            sh.tgt[1][e] = sh.tgt[0][e];
-            sh.spk[1][e] = sh.spk[0][e];
-        }
+        buf = 0;
     } else if (sorted) {
         int run = 0;
         for (int e = lane; e < total; e += 32) {
@@ -534,18 +532,37 @@ __device__ __forceinline__ void g_eval_load(const GrowthDev& g, int b, int i, bo
     }
 }
 
-// The step that delivers a loaded event (the first >= sa, Tseg = T[sa..sb], whose time reaches
-// td), and when the pair's newest pre-synaptic event was.
+// When the pair's newest pre-synaptic event was (its spike's time), of a loaded event.
 template <class R>
-__device__ __forceinline__ double g_eval_time(const NetDev<R>& n, int sa, int sb, const double* Tseg, RowEv& v)
+__device__ __forceinline__ double g_eval_prev(const NetDev<R>& n, const RowEv& v)
 {
-    const long long k = time_key(v.td);
-    int sd = sa;
-    for (int j = 0; j < sb - sa; ++j) sd += time_key(Tseg[j]) < k;   // T[sb] >= td
-    v.sd = sd;
     const int lr = (v.pc + kPreRing - 1) % kPreRing;
     const int ls = lr == 0 ? v.pre.x : lr == 1 ? v.pre.y : lr == 2 ? v.pre.z : v.pre.w;
     return v.pc ? n.T[ls] : 0.0;
+}
+
+// The steps that deliver N loaded events: the first >= sa (Tseg = T[sa..sb]) whose time reaches
+// td.  Counts the earlier steps, eight at a time and for all the events together, so that the
+// segment's times are read once and without waiting for one another.
+template <int N>
+__device__ __forceinline__ void g_eval_steps(int sa, int sb, const double* Tseg, RowEv (&v)[N])
+{
+    long long key[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        key[k] = time_key(v[k].td);
+        v[k].sd = sa;
+    }
+    const int len = sb - sa;   // T[sb] >= td
+    for (int j0 = 0; j0 < len; j0 += 8) {
+        long long t[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) t[j] = j0 + j < len ? time_key(Tseg[j0 + j]) : 0x7fffffffffffffffll;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+            for (int k = 0; k < N; ++k) v[k].sd += t[j] < key[k];
+    }
 }
 
 __device__ __forceinline__ bool g_row_changes(const SynParams& sp, double w, bool is_active, int su, int rem, int sc)
@@ -555,7 +572,7 @@ __device__ __forceinline__ bool g_row_changes(const SynParams& sp, double w, boo
            (w < sp.ACTIVATION_THRESHOLD && is_active);
 }
 
-// The decision on a loaded event; tprev from g_eval_time.
+// The decision on a loaded event; tprev from g_eval_prev, v.sd from g_eval_steps.
 template <class R>
 __device__ __forceinline__ void g_eval_decide(const GrowthDev& g, const NetDev<R>& n, int b, int sa,
                                               const double* Tseg, double tprev, int rem, int sc, RowEv& v)
@@ -611,18 +628,18 @@ constexpr int kEvPerLane = 4;   // events a lane evaluates per chunk (their load
 template <class R>
 __device__ __forceinline__ void g_process(const GrowthDev& g, const NetDev<R>& n, const BatchDev<R>& bt, int b, int i,
                                           size_t r, int sa, int sb, const double* Tseg, int total,
-                                          const RowShared& sh, int lane)
+                                          const RowShared& sh, int buf, int lane)
 {
     int base = 0;
     while (base < total) {
         const int rem = g.remodeled[r];
         const int sc = g.sup_cnt[r];
-        const int spk0 = sh.spk[1][base];
+        const int spk0 = sh.spk[buf][base];
         bool one = true;
 #pragma unroll
         for (int k = 0; k < kEvPerLane; ++k) {
             const int e = base + k * 32 + lane;
-            if (e < total && sh.spk[1][e] != spk0) one = false;
+            if (e < total && sh.spk[buf][e] != spk0) one = false;
         }
         const int slices = __all_sync(0xffffffffu, one) ? kEvPerLane : 1;
         RowEv v[kEvPerLane];
@@ -631,10 +648,11 @@ __device__ __forceinline__ void g_process(const GrowthDev& g, const NetDev<R>& n
         for (int k = 0; k < kEvPerLane; ++k) {
             const int e = base + k * 32 + lane;
             const bool has = k < slices && e < total;
-            g_eval_load<R>(g, b, i, has, has ? sh.td[1][e] : 0.0, has ? sh.tgt[1][e] : -1, has ? sh.spk[1][e] : 0, v[k]);
+            g_eval_load<R>(g, b, i, has, has ? sh.td[buf][e] : 0.0, has ? sh.tgt[buf][e] : -1, has ? sh.spk[buf][e] : 0, v[k]);
         }
 #pragma unroll
-        for (int k = 0; k < kEvPerLane; ++k) tprev[k] = g_eval_time(n, sa, sb, Tseg, v[k]);
+        for (int k = 0; k < kEvPerLane; ++k) tprev[k] = g_eval_prev(n, v[k]);
+        g_eval_steps(sa, sb, Tseg, v);
 #pragma unroll
         for (int k = 0; k < kEvPerLane; ++k) g_eval_decide(g, n, b, sa, Tseg, tprev[k], rem, sc, v[k]);
         if (slices == 1) {
@@ -661,7 +679,7 @@ __device__ __forceinline__ void g_process(const GrowthDev& g, const NetDev<R>& n
                 const int x = __shfl_sync(0xffffffffu, v[k].sd, lf);
                 if (k == kf) sdf = x;
             }
-            if (lane == 0) g_deliver(g, n, bt, b, i, sh.tgt[1][base + f], sdf, sh.spk[1][base + f], sh.td[1][base + f]);
+            if (lane == 0) g_deliver(g, n, bt, b, i, sh.tgt[buf][base + f], sdf, sh.spk[buf][base + f], sh.td[buf][base + f]);
             __syncwarp();
             base += f + 1;
         } else {
@@ -711,7 +729,8 @@ __device__ __forceinline__ void g_row_range(const GrowthDev& g, const NetDev<R>&
             bool trunc = false;
             const int total = g_gather(n, sh_T[sb - s0], head, num, st, stT, perm, Drow, sh, lane, quota, nrun, trunc);
             if (total == 0) break;
-            const bool sorted = g_rank(sh, total, nrun, lane);
+            int buf;
+            const bool sorted = g_rank(sh, total, nrun, lane, buf);
             if (!sorted && trunc) {
                 // a stream whose (delay, target) order differs from its queue
                 // order and does not fit: deliver step by step, one event at a time
@@ -744,12 +763,12 @@ __device__ __forceinline__ void g_row_range(const GrowthDev& g, const NetDev<R>&
                 int lo = 0, hi = total;   // ranked events not after the cut
                 while (lo < hi) {
                     const int mid = (lo + hi) >> 1;
-                    if (!ev_less(ct, cg, cs, sh.td[1][mid], sh.tgt[1][mid], sh.spk[1][mid])) lo = mid + 1;
+                    if (!ev_less(ct, cg, cs, sh.td[buf][mid], sh.tgt[buf][mid], sh.spk[buf][mid])) lo = mid + 1;
                     else hi = mid;
                 }
                 P = lo;
             }
-            g_process(g, n, bt, b, i, r, sa, sb, sh_T + (sa - s0), P, sh, lane);
+            g_process(g, n, bt, b, i, r, sa, sb, sh_T + (sa - s0), P, sh, buf, lane);
             // advance each stream past its processed prefix
             int adv = 0;
             if (lane < nrun) {
@@ -786,22 +805,59 @@ __device__ __forceinline__ void g_row_range(const GrowthDev& g, const NetDev<R>&
 }
 
 // One warp, row i of instance b over the whole interval s0..s1, its somatic spikes of the
-// interval in bits.  Returns the row's live streams after it.
+// interval in bits; head, num, st: the row's stream ring after it.
 template <class R>
-__device__ __forceinline__ int g_row(const GrowthDev& g, const NetDev<R>& n, const BatchDev<R>& bt, uint32_t bits,
-                                     int b, int i, int s0, int s1, const double* sh_T, RowShared& sh, int lane)
+__device__ __forceinline__ void g_row(const GrowthDev& g, const NetDev<R>& n, const BatchDev<R>& bt, uint32_t bits,
+                                      int b, int i, int s0, int s1, const double* sh_T, RowShared& sh, int lane,
+                                      int& head, int& num, RowStreams& st)
 {
     const size_t r = (size_t)b * g.n + i;
-    int head = g.st_head[r], num = g.st_num[r];
-    if (bits == 0 && num == 0) return 0;
-    RowStreams st;
+    head = g.st_head[r];
+    num = g.st_num[r];
+    if (bits == 0 && num == 0) return;
     st.load(n, g.st_step + r * kMaxStreams, g.st_cursor + r * kMaxStreams, g.st_len + r * kMaxStreams, head, num, lane);
     g_row_range(g, n, bt, bits, b, i, s0, s0, s1, false, sh_T, sh, lane, head, num, st);
     if (lane == 0) {
         g.st_head[r] = head;
         g.st_num[r] = num;
     }
-    return num;
+}
+
+template <class R>
+__device__ __forceinline__ void g_row(const GrowthDev& g, const NetDev<R>& n, const BatchDev<R>& bt, uint32_t bits,
+                                      int b, int i, int s0, int s1, const double* sh_T, RowShared& sh, int lane)
+{
+    int head, num;
+    RowStreams st;
+    g_row(g, n, bt, bits, b, i, s0, s1, sh_T, sh, lane, head, num, st);
+}
+
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+// Brings what row i's next deliveries read into L2: the pair states of the next targets of its
+// newest stream.  (The pairs of a network of 2000 HVC(RA) fill the L2 by themselves, and a
+// delivery that finds them in memory waits for it twice.)
+__device__ __forceinline__ void g_row_prefetch(const GrowthDev& g, int b, int i, int head, int num,
+                                               const RowStreams& st, int lane)
+{
+    if (num == 0) return;
+    const int slot = (head + num - 1) % kMaxStreams;
+    const int L = __shfl_sync(0xffffffffu, st.L, slot), c = __shfl_sync(0xffffffffu, st.C, slot);
+    if (L <= 0) return;   // a saturated row's few
+    const int* perm = g.perm + ((size_t)b * g.n + i) * (g.n - 1);
+#pragma unroll
+    for (int k = 0; k < kGatherLoads; ++k) {
+        const int idx = c + 32 * k + lane;
+        if (idx < L) {
+            const size_t ij = gidx(g, b, i, perm[idx]);
+            prefetch_l2(g.D + ij);
+            prefetch_l2(g.W + ij);
+            prefetch_l2(g.pre_step + ij * kPreRing);
+            prefetch_l2(g.pre_cnt + ij);
+            prefetch_l2(g.active + ij);
+            prefetch_l2(g.super + ij);
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -922,7 +978,8 @@ __device__ __forceinline__ void g_row_heavy(const GrowthDev& g, const NetDev<R>&
                 g_eval_load<R>(g, b, i, t[k] >= 0 && time_key(Tlim) >= time_key(td), td, t[k], spk, v[k]);
             }
 #pragma unroll
-            for (int k = 0; k < kEvPerLane; ++k) tprev[k] = g_eval_time(n, from, s1, Tseg, v[k]);
+            for (int k = 0; k < kEvPerLane; ++k) tprev[k] = g_eval_prev(n, v[k]);
+            g_eval_steps(from, s1, Tseg, v);
 #pragma unroll
             for (int k = 0; k < kEvPerLane; ++k) g_eval_decide(g, n, b, from, Tseg, tprev[k], rem, sc, v[k]);
             int due_here = 0;
@@ -1007,7 +1064,7 @@ __device__ __forceinline__ const int* soma_slice(const BatchDev<R>& bt, const Ne
 }
 
 template <class R>
-__global__ void __launch_bounds__(32 * kRowWarps) k_growth_rows(GrowthDev g, NetDev<R> n, BatchDev<R> bt, int q, int s0,
+__global__ void __launch_bounds__(32 * kRowWarps, 1) k_growth_rows(GrowthDev g, NetDev<R> n, BatchDev<R> bt, int q, int s0,
                                                                 int s1)
 {
     extern __shared__ __align__(16) unsigned char row_smem[];
@@ -1035,55 +1092,91 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_growth_rows(GrowthDev g, Net
 // does not matter), and the block sorts the entries by (step, neuron).
 constexpr int kNewpostCap = 4096;   // entries per interval and instance
 
+// The shared memory of the block that lists the new post events.
+struct NewpostShared {
+    int cnt;
+    unsigned keys[kNewpostCap];   // step offset << 27 | neuron
+};
+
+// Neuron i's new post events among its somatic spikes `bits` of the interval.
 template <class R>
-__device__ __forceinline__ void g_newpost_body(const GrowthDev& g, const NetDev<R>& n, const int* soma, int b,
-                                               int s0, int s1)
+__device__ __forceinline__ void g_newpost_neuron(const GrowthDev& g, const NetDev<R>& n, NewpostShared& sh, uint32_t bits,
+                                                 int i, int b, int s0, int s1, double Tsync)
 {
-    __shared__ int cnt;
-    __shared__ unsigned keys[kNewpostCap];   // step offset << 27 | neuron
-    if (threadIdx.x == 0) cnt = 0;
-    __syncthreads();
-    const double Tsync = n.T[s1];
-    for (int i = threadIdx.x; i < g.n; i += blockDim.x) {
-        const uint32_t bits = (uint32_t)soma[(size_t)b * n.n_ra + i];
-        if (!bits) continue;
-        const size_t ri = (size_t)b * g.n + i;
-        const double pl = g.post_last[ri];   // -1e300 when the neuron has no post event yet
-        uint32_t mask = 0;
-        for (uint32_t m = bits; m; m &= m - 1) {
-            const int k = __ffs(m) - 1;
-            if (n.T[s0 + k] > pl + 30.0) mask |= 1u << k;
-        }
-        if (!mask) continue;
-        const int c = __popc(mask);
-        int pos = atomicAdd(&cnt, c);
-        for (uint32_t m = mask; m; m &= m - 1) {
-            if (pos < kNewpostCap) keys[pos] = ((unsigned)(__ffs(m) - 1) << 27) | (unsigned)i;
-            ++pos;
-        }
-        for (int e = 0; e < c; ++e) {
-            g.post_step[ri * kPostRing + (g.post_cnt[ri] % kPostRing)] = s1;
-            g.post_cnt[ri] += 1;
-        }
-        g.post_last[ri] = Tsync;
+    const size_t ri = (size_t)b * g.n + i;
+    const double pl = g.post_last[ri];   // -1e300 when the neuron has no post event yet
+    uint32_t mask = 0;
+    for (uint32_t m = bits; m; m &= m - 1) {
+        const int k = __ffs(m) - 1;
+        if (n.T[s0 + k] > pl + 30.0) mask |= 1u << k;
     }
+    if (!mask) return;
+    const int c = __popc(mask);
+    int pos = atomicAdd(&sh.cnt, c);
+    for (uint32_t m = mask; m; m &= m - 1) {
+        if (pos < kNewpostCap) sh.keys[pos] = ((unsigned)(__ffs(m) - 1) << 27) | (unsigned)i;
+        ++pos;
+    }
+    for (int e = 0; e < c; ++e) {
+        g.post_step[ri * kPostRing + (g.post_cnt[ri] % kPostRing)] = s1;
+        g.post_cnt[ri] += 1;
+    }
+    g.post_last[ri] = Tsync;
+}
+
+// The listed events in order; returns their count (0 when they do not fit).
+__device__ __forceinline__ int g_newpost_sort(const GrowthDev& g, NewpostShared& sh, int b)
+{
     __syncthreads();
-    const int K = cnt;
+    const int K = sh.cnt;
     if (K > kNewpostCap || K > g.n * 16) {
         if (threadIdx.x == 0) {
             atomicOr(g.error, kErrPostCapacity);
             g.newpost_cnt[b] = 0;
         }
-        return;
+        return 0;
     }
     // rank sort (the keys are distinct)
     for (int e = threadIdx.x; e < K; e += blockDim.x) {
-        const unsigned key = keys[e];
+        const unsigned key = sh.keys[e];
         int rank = 0;
-        for (int j = 0; j < K; ++j) rank += keys[j] < key;
+        for (int j = 0; j < K; ++j) rank += sh.keys[j] < key;
         g.newpost[(size_t)b * g.n * 16 + rank] = (int)(key & ((1u << 27) - 1u));
     }
     if (threadIdx.x == 0) g.newpost_cnt[b] = K;
+    return K;
+}
+
+template <class R>
+__device__ __forceinline__ void g_newpost_body(const GrowthDev& g, const NetDev<R>& n, const int* soma, int b,
+                                               int s0, int s1)
+{
+    __shared__ NewpostShared sh;
+    if (threadIdx.x == 0) sh.cnt = 0;
+    __syncthreads();
+    const double Tsync = n.T[s1];
+    for (int i = threadIdx.x; i < g.n; i += blockDim.x) {
+        const uint32_t bits = (uint32_t)soma[(size_t)b * n.n_ra + i];
+        if (bits) g_newpost_neuron(g, n, sh, bits, i, b, s0, s1, Tsync);
+    }
+    g_newpost_sort(g, sh, b);
+}
+
+// The same from the interval's queued rows (row, spike bits), which hold every neuron that
+// spiked; row(e) for e < count, of instance 0.
+template <class R, class F>
+__device__ __forceinline__ int g_newpost_rows(const GrowthDev& g, const NetDev<R>& n, unsigned count, F&& row, int s0,
+                                              int s1)
+{
+    __shared__ NewpostShared sh;
+    if (threadIdx.x == 0) sh.cnt = 0;
+    __syncthreads();
+    const double Tsync = n.T[s1];
+    for (unsigned e = threadIdx.x; e < count; e += blockDim.x) {
+        const int2 r = row(e);
+        if (r.y) g_newpost_neuron(g, n, sh, (uint32_t)r.y, r.x, 0, s0, s1, Tsync);
+    }
+    return g_newpost_sort(g, sh, 0);
 }
 
 template <class R>

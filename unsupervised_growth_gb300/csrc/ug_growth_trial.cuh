@@ -1,4 +1,5 @@
-// One growth trial of one network in one cooperative launch: every sync interval of
+// One growth trial of one network in one cooperative launch, double build (the single build's
+// is ug_growth_units.cuh): every sync interval of
 // trial_1stSoma_pre_1stSoma_post_delays_fixedSpread (NetworkGrowthSimulator.cpp:8923-9564)
 // runs inside k_growth_trial, with bounded grid barriers where the per-interval path
 // (launch_interval + launch_growth_sync) has kernel boundaries.
@@ -29,31 +30,17 @@ namespace ug {
 constexpr int kTrialThreads = 256;
 constexpr int kTrialWarps = kTrialThreads / 32;
 
-// Threads per block of the integrating roles (whole warps, at most kTrialThreads).  The
-// single build's packed integrator steps two HVC(RA) neurons per thread, its interneuron
-// integrator one; the double build one neuron per thread.  A trial is a chain of
-// intervals whose length is set by the slowest integrating warp, so by default one warp
-// per block integrates (one integrating warp per SM), and a trial spreads over as many
-// SMs as it has integrating warps; wider roles put several integrating warps on one SM
-// scheduler (on the 2000 + 550 network: 98.7 ms per trial at 256 threads, 81.9 ms at 32).
-template <class R>
-struct TrialShape;
-template <>
-struct TrialShape<float> {
-    static constexpr int ra_w = 32, i_w = 32, ra_per_thread = 2;
-};
-template <>
-struct TrialShape<double> {
-    static constexpr int ra_w = 32, i_w = 32, ra_per_thread = 1;
-};
+// Threads per block of the integrating roles (whole warps, at most kTrialThreads): by default
+// one integrating warp per block, so that a trial spreads over as many SMs as it has
+// integrating warps; wider roles put several integrating warps on one SM scheduler.
+constexpr int kRoleThreads = 32;
 
 // The role widths of a request (0: the default); false unless each is a multiple of 32
 // in [32, kTrialThreads].
-template <class R>
 __host__ __device__ inline bool trial_widths(int req_ra, int req_i, int* ra_w, int* i_w)
 {
-    *ra_w = req_ra ? req_ra : TrialShape<R>::ra_w;
-    *i_w = req_i ? req_i : TrialShape<R>::i_w;
+    *ra_w = req_ra ? req_ra : kRoleThreads;
+    *i_w = req_i ? req_i : kRoleThreads;
     for (int w : {*ra_w, *i_w})
         if (w < 32 || w > kTrialThreads || w % 32) return false;
     return true;
@@ -70,12 +57,10 @@ struct TrialLoop {
 
 // Grid size of k_growth_trial for a network: the three roles, one sync block per
 // kTrialThreads rows.
-template <class R>
 __host__ __device__ inline void trial_roles(int n_ra, int n_i, int ra_w, int i_w, int* nb_ra, int* nb_i,
                                             int* nb_sync)
 {
-    const int ra = TrialShape<R>::ra_per_thread * ra_w;
-    *nb_ra = (n_ra + ra - 1) / ra;
+    *nb_ra = (n_ra + ra_w - 1) / ra_w;
     *nb_i = (n_i + i_w - 1) / i_w;
     *nb_sync = (n_ra + kTrialThreads - 1) / kTrialThreads;
 }
@@ -84,24 +69,14 @@ template <class R>
 __device__ __forceinline__ void trial_ra_part(const NetDev<R>& n, const BatchDev<R>& bt, int q, int s0, int s1,
                                               const RAStep<R>& rc, int k, int ra_w)
 {
-    if (threadIdx.x >= ra_w) return;
-    if constexpr (sizeof(R) == 4) {
-        interval_ra_v_body<f2, R>(n, bt, q, s0, s1, rc, k * ra_w + (int)threadIdx.x, 0);   // pairs [ra_w k, ra_w (k + 1))
-    } else {
-        interval_ra_body<R>(n, bt, q, s0, s1, rc, k, 0, ra_w);
-    }
+    if (threadIdx.x < ra_w) interval_ra_body<R>(n, bt, q, s0, s1, rc, k, 0, ra_w);
 }
 
 template <class R>
 __device__ __forceinline__ void trial_i_part(const NetDev<R>& n, const BatchDev<R>& bt, int q, int s0, int s1,
                                              const IStep<R>& ic, int k, int i_w)
 {
-    if (threadIdx.x >= i_w) return;
-    if constexpr (sizeof(R) == 4) {
-        interval_i_x_body<R>(n, bt, q, s0, s1, ic, k * i_w + (int)threadIdx.x, 0);   // interneurons [i_w k, i_w (k + 1))
-    } else {
-        interval_i_body<R>(n, bt, q, s0, s1, ic, k, 0, i_w);
-    }
+    if (threadIdx.x < i_w) interval_i_body<R>(n, bt, q, s0, s1, ic, k, 0, i_w);
 }
 
 template <class R>

@@ -362,8 +362,8 @@ private:
     // the one-launch growth trial (ug_growth_trial.cuh)
     DevMem gTrialCtl_, gActRows_;  // barrier and queue words, row queue
     bool trial_fits_ = false;      // every sync interval fits the trial's segment buffers
-    int trial_key_ = -1;           // the launch mode and role widths trial_blocks_ was sized for
-    int trial_blocks_ = 0;         // its grid (0: the network's blocks cannot all be resident)
+    int trial_key_ = -1;           // the launch mode and role widths trial_plan_ was sized for
+    ug::GrowthPlan trial_plan_;    // its grid (no blocks: they cannot all be resident)
     int gloop_trial_launch_ = -1;  // the trial_key_ the loop graph was captured with
     static int trial_key(const ug::LaunchCtx& lc)
     {
@@ -375,18 +375,17 @@ private:
         const int key = trial_key(lc);
         if (key == trial_key_) return UG_OK;
         trial_key_ = -1;
-        trial_blocks_ = 0;
-        int ra_w = 0, i_w = 0;
-        if (key && trial_fits_ && ug::trial_widths<R>(lc.trial_ra_w, lc.trial_i_w, &ra_w, &i_w))
-            UG_CUDA(ug::growth_trial_grid<R>(h.n_ra, h.n_i, ra_w, i_w, &trial_blocks_));
+        trial_plan_ = ug::GrowthPlan();
+        if (key && trial_fits_)
+            UG_CUDA(ug::growth_trial_plan<R>(h.n_ra, h.n_i, lc.trial_ra_w, lc.trial_i_w, &trial_plan_));
         trial_key_ = key;
         return UG_OK;
     }
-    // trial_grid(lc) has sized trial_blocks_ before any use of this
+    // trial_grid(lc) has sized trial_plan_ before any use of this
     bool one_launch(const ug::LaunchCtx& lc) const
     {
-        return lc.trial_launch && !lc.timer && trial_key_ == trial_key(lc) && trial_blocks_ > 0 && bd_.B == 1 && !bd_.trace_ra && !bd_.trace_i &&
-               !bd_.ginh_slot;
+        return lc.trial_launch && !lc.timer && trial_key_ == trial_key(lc) && trial_plan_.blocks > 0 && bd_.B == 1 &&
+               !bd_.trace_ra && !bd_.trace_i && !bd_.ginh_slot;
     }
     DevMem gTrRaSlot_, gTrISlot_, gTrRaBuf_, gTrIBuf_;   // per-neuron traces
     void apply_recording()
@@ -1044,9 +1043,9 @@ ug_status NetImpl<R>::growth_init(cudaStream_t st)
     UG_TRY(gLoop_.alloc(ug::kLoopWords * sizeof(int)));
     if (!hloop_) UG_CUDA(cudaMallocHost(&hloop_, ug::kLoopWords * sizeof(int)));
     // the one-launch trial: barrier and queue words, the row queue
-    UG_TRY(gTrialCtl_.alloc(8 * sizeof(unsigned)));
+    UG_TRY(gTrialCtl_.alloc(ug::kGrowthCtlWords * sizeof(unsigned long long)));
     UG_TRY(gActRows_.alloc(4 * (size_t)n * sizeof(int2)));
-    trial_blocks_ = 0;
+    trial_plan_ = ug::GrowthPlan();
     trial_key_ = -1;
     bool fits = !sync_steps.empty();
     for (size_t q = 0; q < sync_steps.size(); ++q) {
@@ -1141,25 +1140,9 @@ ug_status NetImpl<R>::issue_growth_trial(const ug::LaunchCtx& lc, int64_t* launc
     ++cnt;
     const int Q = (int)sync_steps.size();
     if (one_launch(lc)) {
-        // every interval in one cooperative launch; its queue of rows with deliveries
-        unsigned* ctl = gTrialCtl_.as<unsigned>();
-        UG_CUDA(cudaMemsetAsync(ctl, 0, gTrialCtl_.bytes(), lc.main));
-        ug::BatchDev<R> b = bd_;
-        b.act_rows = gActRows_.as<int2>();
-        b.act_cnt = reinterpret_cast<int*>(ctl + 4);
-        b.act_cap = h.n_ra;
-        b.member = 0;
-        b.live_streams = gd_.st_num;
-        b.heavy = 0;
-        ug::TrialLoop L;
-        L.sync_end = dSyncEnd_.as<int>();
-        L.Q = Q;
-        int nb_sync = 0;
-        ug::trial_widths<R>(lc.trial_ra_w, lc.trial_i_w, &L.ra_w, &L.i_w);   // checked by trial_grid
-        ug::trial_roles<R>(h.n_ra, h.n_i, L.ra_w, L.i_w, &L.nb_ra, &L.nb_i, &nb_sync);
-        L.bar = ctl;
-        L.posted = ctl + 1;
-        UG_CUDA(ug::launch_growth_trial<R>(gd_, nd_, b, rc_, ic_, L, trial_blocks_, lc.main));
+        // every interval in one cooperative launch
+        UG_CUDA(ug::launch_growth_trial<R>(gd_, nd_, bd_, rc_, ic_, trial_plan_, dSyncEnd_.as<int>(), Q,
+                                           gTrialCtl_.as<unsigned long long>(), gActRows_.as<int2>(), lc.main));
         cnt += 1;
     } else {
         bool tail_open = false;

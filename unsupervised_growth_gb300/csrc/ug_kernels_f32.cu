@@ -12,9 +12,10 @@ template cudaError_t launch_growth_epilogue<float>(const GrowthDev&, const Launc
 template cudaError_t launch_growth_remove<float>(const GrowthDev&, const int*, int, cudaStream_t);
 template cudaError_t launch_check_bad<float>(const NetDev<float>&, const BatchDev<float>&, int*, cudaStream_t);
 template cudaError_t epilogue_bulk_grid<float>(int, int, int*);
-template cudaError_t growth_trial_grid<float>(int, int, int, int, int*);
-template cudaError_t launch_growth_trial<float>(const GrowthDev&, const NetDev<float>&, const BatchDev<float>&,
-                                             const RAStep<float>&, const IStep<float>&, const TrialLoop&, int, cudaStream_t);
+template cudaError_t growth_trial_plan<float>(int, int, int, int, GrowthPlan*);
+template cudaError_t launch_growth_trial<float>(const GrowthDev&, const NetDev<float>&, BatchDev<float>, const RAStep<float>&,
+                                              const IStep<float>&, const GrowthPlan&, const int*, int,
+                                              unsigned long long*, int2*, cudaStream_t);
 template cudaError_t launch_growth_head<float>(const TailDev<float>&, int*, cudaStream_t);
 template cudaError_t launch_growth_tail<float>(const TailDev<float>&, cudaStream_t);
 template cudaError_t group_grids<float>(GroupDev&, int, int);

@@ -291,33 +291,72 @@ cudaError_t launch_growth_epilogue(const GrowthDev& g, const LaunchCtx& lc)
 // Dynamic shared memory of k_growth_trial: one row buffer per warp.
 constexpr size_t kTrialSmem = (size_t)kTrialWarps * sizeof(RowShared);
 
-template <class R>
-cudaError_t growth_trial_grid(int n_ra, int n_i, int ra_w, int i_w, int* blocks)
+inline cudaError_t units_attributes(const void* kernel)
 {
-    *blocks = 0;
-    cudaError_t e =
-        cudaFuncSetAttribute(k_growth_trial<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrialSmem);
-    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrialSmem);
+}
+
+// Single build: one HVC(RA) neuron per thread where the roles fit the SMs, a block each, else
+// two.  The rows take what the other roles leave, up to kRowBlocks blocks.
+template <class R>
+cudaError_t growth_trial_plan(int n_ra, int n_i, int req_ra, int req_i, GrowthPlan* plan)
+{
+    *plan = GrowthPlan();
     int dev = 0, sms = 0, per_sm = 0, coop = 0;
-    e = cudaGetDevice(&dev);
+    cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-    if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_growth_trial<R>, kTrialThreads, kTrialSmem);
-    if (e != cudaSuccess) return e;
-    int nb_ra = 0, nb_i = 0, nb_sync = 0;
-    trial_roles<R>(n_ra, n_i, ra_w, i_w, &nb_ra, &nb_i, &nb_sync);
-    const long long total = (long long)nb_ra + nb_i + nb_sync;
-    if (coop && per_sm > 0 && total <= (long long)per_sm * sms) *blocks = (int)total;
-    return cudaSuccess;
+    int ra_w = 0, i_w = 0;
+    if (e != cudaSuccess || !coop || !trial_widths(req_ra, req_i, &ra_w, &i_w)) return e;
+    if constexpr (sizeof(R) == 4) {
+        for (int lanes = 1; lanes <= 2 && plan->blocks == 0; ++lanes) {
+            e = units_attributes(lanes == 1 ? (const void*)k_growth_units<float> : (const void*)k_growth_units<f2>);
+            if (e != cudaSuccess) return e;
+            // by default as few warps to a block as leave the rows enough blocks
+            for (int per = 1; per <= kTrialWarps && plan->blocks == 0; per *= 2) {
+                UnitsLoop u{};
+                u.ra_units = (n_ra + 32 * lanes - 1) / (32 * lanes);
+                u.i_units = (n_i + 31) / 32;
+                u.ra_per = req_ra ? ra_w / 32 : per;
+                u.i_per = req_i ? i_w / 32 : per;
+                u.nb_ra = (u.ra_units + u.ra_per - 1) / u.ra_per;
+                u.nb_i = (u.i_units + u.i_per - 1) / u.i_per;
+                u.nb_sync = std::min(kSyncBlocks, (n_ra + kTrialThreads - 1) / kTrialThreads);
+                u.nb_row = std::min(kRowBlocks, sms - u.nb_ra - u.nb_i - u.nb_sync);
+                if (u.nb_row < (per < kTrialWarps ? kEnoughRowBlocks : kMinRowBlocks)) continue;
+                plan->lanes = lanes;
+                plan->units = u;
+                plan->blocks = u.nb_ra + u.nb_i + u.nb_sync + u.nb_row;
+            }
+        }
+        return cudaSuccess;
+    } else {
+        e = units_attributes((const void*)k_growth_trial<R>);
+        if (e == cudaSuccess)
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_growth_trial<R>, kTrialThreads, kTrialSmem);
+        if (e != cudaSuccess) return e;
+        int nb_sync = 0;
+        plan->trial.ra_w = ra_w;
+        plan->trial.i_w = i_w;
+        trial_roles(n_ra, n_i, ra_w, i_w, &plan->trial.nb_ra, &plan->trial.nb_i, &nb_sync);
+        const long long total = (long long)plan->trial.nb_ra + plan->trial.nb_i + nb_sync;
+        if (per_sm > 0 && total <= (long long)per_sm * sms) plan->blocks = (int)total;
+        return cudaSuccess;
+    }
 }
 
 template <class R>
-cudaError_t launch_growth_trial(const GrowthDev& g, const NetDev<R>& n, const BatchDev<R>& b, const RAStep<R>& rc,
-                                const IStep<R>& ic, const TrialLoop& L, int blocks, cudaStream_t st)
+cudaError_t launch_growth_trial(const GrowthDev& g, const NetDev<R>& n, BatchDev<R> b, const RAStep<R>& rc,
+                                const IStep<R>& ic, const GrowthPlan& plan, const int* sync_end, int Q,
+                                unsigned long long* ctl, int2* act_rows, cudaStream_t st)
 {
+    cudaError_t e = cudaMemsetAsync(ctl, 0, kGrowthCtlWords * sizeof(unsigned long long), st);
+    if (e != cudaSuccess) return e;
+    b.member = 0;
+    b.live_streams = g.st_num;
+    b.heavy = 0;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.gridDim = dim3((unsigned)plan.blocks);
     cfg.blockDim = dim3(kTrialThreads);
     cfg.dynamicSmemBytes = kTrialSmem;
     cfg.stream = st;
@@ -326,7 +365,27 @@ cudaError_t launch_growth_trial(const GrowthDev& g, const NetDev<R>& n, const Ba
     at[0].val.cooperative = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_growth_trial<R>, g, n, b, rc, ic, L);
+    if constexpr (sizeof(R) == 4) {
+        UnitsLoop L = plan.units;
+        L.sync_end = sync_end;
+        L.Q = Q;
+        L.ctl = ctl;
+        L.rows = act_rows;
+        L.rows_cap = 2 * n.n_ra;
+        b.soma_bits = nullptr;   // the spike bits travel with the queued rows
+        return plan.lanes == 1 ? cudaLaunchKernelEx(&cfg, k_growth_units<float>, g, n, b, rc, ic, L)
+                               : cudaLaunchKernelEx(&cfg, k_growth_units<f2>, g, n, b, rc, ic, L);
+    } else {
+        TrialLoop L = plan.trial;
+        L.sync_end = sync_end;
+        L.Q = Q;
+        L.bar = reinterpret_cast<unsigned*>(ctl);
+        L.posted = L.bar + 1;
+        b.act_rows = act_rows;
+        b.act_cnt = reinterpret_cast<int*>(ctl) + 4;
+        b.act_cap = n.n_ra;
+        return cudaLaunchKernelEx(&cfg, k_growth_trial<R>, g, n, b, rc, ic, L);
+    }
 }
 
 // Grid of the bulk-copy epilogue for B networks of n neurons (0: rows not 16-byte aligned

@@ -12,6 +12,7 @@
 #include "ug_group.cuh"
 #include "ug_test_trial.cuh"
 #include "ug_growth_trial.cuh"
+#include "ug_growth_units.cuh"
 #include "ug_tail.cuh"
 
 namespace ug {
@@ -163,11 +164,20 @@ template <class R>
 cudaError_t launch_growth_epilogue(const GrowthDev& g, const LaunchCtx& lc);
 // The one-launch growth trial (ug_growth_trial.cuh): its grid for a network (0 when the
 // blocks cannot all be resident at once), and the cooperative launch.
+struct GrowthPlan {
+    int blocks = 0;   // 0: the network's blocks cannot all be resident, per-interval launches
+    int lanes = 1;    // single build: HVC(RA) neurons per thread
+    TrialLoop trial{};   // double build (k_growth_trial)
+    UnitsLoop units{};   // single build (k_growth_units)
+};
+// The grid for a network and a request of role widths (0: the default).
 template <class R>
-cudaError_t growth_trial_grid(int n_ra, int n_i, int ra_w, int i_w, int* blocks);
+cudaError_t growth_trial_plan(int n_ra, int n_i, int req_ra, int req_i, GrowthPlan* plan);
+// ctl: kGrowthCtlWords 64-bit words, cleared here; act_rows: room for 4 n_ra queued rows.
 template <class R>
-cudaError_t launch_growth_trial(const GrowthDev& g, const NetDev<R>& n, const BatchDev<R>& b, const RAStep<R>& rc,
-                                const IStep<R>& ic, const TrialLoop& L, int blocks, cudaStream_t st);
+cudaError_t launch_growth_trial(const GrowthDev& g, const NetDev<R>& n, BatchDev<R> b, const RAStep<R>& rc,
+                                const IStep<R>& ic, const GrowthPlan& plan, const int* sync_end, int Q,
+                                unsigned long long* ctl, int2* act_rows, cudaStream_t st);
 template <class R>
 cudaError_t launch_growth_remove(const GrowthDev& g, const int* rep, int nrep, cudaStream_t st);
 template <class R>
