@@ -142,10 +142,10 @@ __global__ void __launch_bounds__(32 * kRowWarps, 1) kl_growth_rows(const GroupM
                                                                  int q, int s0, int s1)
 {
     extern __shared__ __align__(16) unsigned char row_smem[];
-    __shared__ double sh_T[kSegSteps];
+    __shared__ double sh_T[2 * kSegSteps];
     __shared__ GroupMember<R> M[kRowWarps];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int k = threadIdx.x; k <= s1 - s0 && k < kSegSteps; k += blockDim.x) sh_T[k] = T[s0 + k];
+    g_stage_times(sh_T, T, s0, s1);
     __syncthreads();
     if (s1 - s0 >= kSegSteps) return;   // the host never builds such an interval
     const int nrows = min(act_cnt[q & 1], act_cap);
@@ -174,9 +174,9 @@ __global__ void __launch_bounds__(32 * kHeavyWarps, 1) kl_growth_rows_heavy(cons
                                                                          int s1)
 {
     extern __shared__ __align__(16) unsigned char heavy_smem[];
-    __shared__ double sh_T[kSegSteps];
+    __shared__ double sh_T[2 * kSegSteps];
     __shared__ GroupMember<R> M;
-    for (int k = threadIdx.x; k <= s1 - s0 && k < kSegSteps; k += blockDim.x) sh_T[k] = T[s0 + k];
+    g_stage_times(sh_T, T, s0, s1);
     __syncthreads();
     if (s1 - s0 >= kSegSteps) return;
     RowShared& sh = *reinterpret_cast<RowShared*>(heavy_smem);

@@ -47,6 +47,12 @@ struct SynParams {
     // LTD leaves a weight of +0 at +0 (its parameters are finite and its time constants
     // positive), so the delivery of an event onto such a pair needs none of the post events.
     int zero_stays;
+    int zero_active, zero_super;    // 0 >= ACTIVATION_THRESHOLD, 0 >= SUPERSYNAPSE_THRESHOLD
+    // g_row_changes for a weight of 0
+    __device__ __forceinline__ bool zero_changes(bool is_active, int su, int rem, int sc) const
+    {
+        return (zero_active ? !is_active && rem == 0 : is_active) || (zero_super ? su == 0 && sc < Nss : su == 1);
+    }
 };
 
 // Device state of the RA->RA synapses of B growing networks of n neurons.
@@ -71,6 +77,7 @@ struct GrowthDev {
     double* spike_last;     // [B][n] time of the row's newest somatic spike (-1e300: none this trial)
     double max_delay;       // bound on every RA->RA delay the network can have
     int* st_step;           // [B][n][kMaxStreams] spike step of each live stream
+    double* st_time;        // [B][n][kMaxStreams] and its time
     int* st_cursor;         // [B][n][kMaxStreams]
     int* st_len;            // [B][n][kMaxStreams] targets in the stream (n-1, or the snapshot size)
     int* st_tgt;            // [B][n][kMaxStreams][kMaxNss] snapshot of a saturated spike's targets
@@ -228,12 +235,14 @@ static __device__ __noinline__ void g_deliver(const GrowthDev& g, const NetDev<R
 __device__ __forceinline__ int g_open_stream(const GrowthDev& g, size_t r, int s, double Ts, const double* Drow,
                                              int head, int num, int* stS, int* stC, int* stL, int* stT)
 {
+    double* stTm = g.st_time + r * kMaxStreams;
     if (num >= kMaxStreams) {
         atomicOr(g.error, kErrEventCapacity);
         return num;
     }
     const int slot = (head + num) % kMaxStreams;
     stS[slot] = s;
+    stTm[slot] = Ts;
     g.spike_last[r] = Ts;
     stC[slot] = 0;
     const int sc = g.sup_cnt[r];
@@ -297,6 +306,16 @@ constexpr int kRowWarps = 2;    // rows (warps) per block (2 x RowShared stays u
 constexpr int kDueCap = 512;    // due events merged per segment in shared memory
 constexpr int kSegSteps = 32;   // longest interval the row kernel handles
 
+// The block's copy of an interval's times: T[s0..s1], and from kSegSteps on the starts of the
+// STDP windows of those steps (100 ms before).
+__device__ __forceinline__ void g_stage_times(double* sh_T, const double* T, int s0, int s1)
+{
+    for (int k = threadIdx.x; k <= s1 - s0 && k < kSegSteps; k += blockDim.x) {
+        sh_T[k] = T[s0 + k];
+        sh_T[kSegSteps + k] = T[s0 + k] - 100.0;
+    }
+}
+
 // Per-warp shared buffers of the row kernel.
 struct RowShared {
     double td[2][kDueCap];     // gathered / ranked delivery times
@@ -323,17 +342,13 @@ __device__ __forceinline__ long long time_key(double t)
 struct RowStreams {
     int S, C, L;
     double T;
-    template <class R>
-    __device__ __forceinline__ void load(const NetDev<R>& n, const int* stS, const int* stC, const int* stL, int head,
-                                         int num, int lane)
+    // Row r's whole ring, open or not: the loads do not wait for head and num.
+    __device__ __forceinline__ void load(const GrowthDev& g, size_t r, int lane)
     {
-        // the whole ring at once, whatever is open: the loads do not wait for head and num
-        S = stS[lane];
-        C = stC[lane];
-        L = stL[lane];
-        const bool open = ((lane - head) & (kMaxStreams - 1)) < num;
-        if (!open) S = C = L = 0;
-        T = open ? n.T[S] : 0.0;
+        S = g.st_step[r * kMaxStreams + lane];
+        C = g.st_cursor[r * kMaxStreams + lane];
+        L = g.st_len[r * kMaxStreams + lane];
+        T = g.st_time[r * kMaxStreams + lane];
     }
 };
 static_assert(kMaxStreams == 32, "a lane per slot of the stream ring");
@@ -499,46 +514,55 @@ __device__ __forceinline__ bool g_rank(RowShared& sh, int total, int nrun, int l
 // deactivation or supersynapse change -- which is also the only way the row
 // desaturates).
 struct RowEv {
-    bool has, changing, is_active, do_write, new_pre;
-    int t, spk, pc, sd, su;
+    bool has, changing, do_write, new_pre;
+    int t, spk, pc, sd, act, su;
     size_t ij;
     double td, wv, w2, plast, Dij;
     short4 pre;
+    __device__ __forceinline__ bool is_active() const { return act == 1; }
 };
 
-// The loads of event (td, t, spk) of row i, all independent of each other; has = false loads
-// nothing.
-template <class R>
+// The loads of event (td, t, spk) of row i, all independent of each other; has = false: an
+// event that does nothing (it loads the pair (i, 0)).  No value is looked at here and nothing
+// branches on `has`, so that the loads of several events are in flight together.
 __device__ __forceinline__ void g_eval_load(const GrowthDev& g, int b, int i, bool has, double td, int t, int spk,
                                             RowEv& v)
 {
     v.has = has;
-    v.changing = v.do_write = v.new_pre = v.is_active = false;
+    v.changing = v.do_write = v.new_pre = false;
     v.t = has ? t : -1;
     v.spk = spk;
     v.td = td;
-    v.wv = v.plast = v.Dij = 0.0;
-    v.pc = v.su = 0;
-    v.pre = make_short4(0, 0, 0, 0);
-    v.ij = gidx(g, b, i, has ? t : 0);
-    if (has) {
-        v.is_active = g.active[v.ij] == 1;
-        v.su = g.super[v.ij];
-        v.wv = g.W[v.ij];
-        v.pc = g.pre_cnt[v.ij];
-        v.pre = *reinterpret_cast<const short4*>(g.pre_step + v.ij * kPreRing);   // the pair's whole ring
-        v.plast = g.post_last[(size_t)b * g.n + t];
-        v.Dij = g.D[v.ij];
-    }
+    const int j = has ? t : 0;
+    v.ij = gidx(g, b, i, j);
+    v.act = g.active[v.ij];
+    v.su = g.super[v.ij];
+    v.wv = g.W[v.ij];
+    v.pc = g.pre_cnt[v.ij];
+    v.pre = *reinterpret_cast<const short4*>(g.pre_step + v.ij * kPreRing);   // the pair's whole ring
+    v.plast = g.post_last[(size_t)b * g.n + j];
+    v.Dij = g.D[v.ij];
 }
 
-// When the pair's newest pre-synaptic event was (its spike's time), of a loaded event.
+// An event that is not there, without loads.
+__device__ __forceinline__ void g_eval_none(RowEv& v)
+{
+    v.has = v.changing = v.do_write = v.new_pre = false;
+    v.t = -1;
+    v.spk = v.pc = v.act = v.su = 0;
+    v.ij = 0;
+    v.td = v.wv = v.plast = v.Dij = 0.0;
+    v.pre = make_short4(0, 0, 0, 0);
+}
+
+// When the pair's newest pre-synaptic event was (its spike's time), of a loaded event; not
+// looked at for a pair without one.
 template <class R>
 __device__ __forceinline__ double g_eval_prev(const NetDev<R>& n, const RowEv& v)
 {
     const int lr = (v.pc + kPreRing - 1) % kPreRing;
     const int ls = lr == 0 ? v.pre.x : lr == 1 ? v.pre.y : lr == 2 ? v.pre.z : v.pre.w;
-    return v.pc ? n.T[ls] : 0.0;
+    return n.T[v.has && v.pc ? ls : 0];
 }
 
 // The steps that deliver N loaded events: the first >= sa (Tseg = T[sa..sb]) whose time reaches
@@ -572,22 +596,24 @@ __device__ __forceinline__ bool g_row_changes(const SynParams& sp, double w, boo
            (w < sp.ACTIVATION_THRESHOLD && is_active);
 }
 
-// The decision on a loaded event; tprev from g_eval_prev, v.sd from g_eval_steps.
+// The decision on a loaded event; tprev from g_eval_prev (looked at when the pair has had an
+// event), v.sd from g_eval_steps.  Tfrom: the start of the STDP window of each step of Tseg.
 template <class R>
 __device__ __forceinline__ void g_eval_decide(const GrowthDev& g, const NetDev<R>& n, int b, int sa,
-                                              const double* Tseg, double tprev, int rem, int sc, RowEv& v)
+                                              const double* Tfrom, double tprev, int rem, int sc, RowEv& v)
 {
     const SynParams& sp = g.sp;
     v.w2 = v.wv;
     if (!v.has) return;
     // new pre-synaptic event: first, or more than 30 ms after the previous one
-    v.new_pre = v.pc == 0 || time_key(v.td) > time_key(tprev + v.Dij + 30.0);
+    v.new_pre = v.pc == 0;
+    if (v.pc != 0) v.new_pre = time_key(v.td) > time_key(tprev + v.Dij + 30.0);
     if (!v.new_pre || (sc == sp.Nss && v.su != 1)) return;
     // LTD against the target's post events in [now - 100, now]; none when the newest is older
-    const double now = Tseg[v.sd - sa], from = now - 100.0;
+    const double from = Tfrom[v.sd - sa];
     if (time_key(v.plast) < time_key(from)) return;
     if (sp.zero_stays && __double_as_longlong(v.wv) == 0) {   // stays 0 whatever the events are
-        v.changing = g_row_changes(sp, 0.0, v.is_active, v.su, rem, sc);
+        v.changing = sp.zero_changes(v.is_active(), v.su, rem, sc);
         return;
     }
     const int np = post_num(g, b, v.t);
@@ -596,7 +622,7 @@ __device__ __forceinline__ void g_eval_decide(const GrowthDev& g, const NetDev<R
         if (!(tp >= from)) continue;
         g_LTD(sp, v.w2, tp - v.td);
         v.do_write = true;
-        v.changing |= g_row_changes(sp, v.w2, v.is_active, v.su, rem, sc);
+        v.changing |= g_row_changes(sp, v.w2, v.is_active(), v.su, rem, sc);
     }
 }
 
@@ -604,7 +630,7 @@ template <class R>
 __device__ __forceinline__ void g_commit(const GrowthDev& g, const NetDev<R>& n, const BatchDev<R>& bt, int b,
                                          const RowEv& v)
 {
-    if (v.is_active) {
+    if (v.is_active()) {
         // update_Ge_RA[target] += w, applied at the sync closing the delivery step
         const size_t slot = (size_t)(n.syncidx[v.sd] % n.ring) * bt.B * n.n_ra + (size_t)b * n.n_ra + v.t;
         atomicAdd((unsigned long long*)&bt.ring_ra_exc[slot], (unsigned long long)llrint(v.wv * kFixScale));
@@ -627,7 +653,8 @@ constexpr int kEvPerLane = 4;   // events a lane evaluates per chunk (their load
 // target twice: it is cut to 32 events and the repeats take the exact path.
 template <class R>
 __device__ __forceinline__ void g_process(const GrowthDev& g, const NetDev<R>& n, const BatchDev<R>& bt, int b, int i,
-                                          size_t r, int sa, int sb, const double* Tseg, int total,
+                                          size_t r, int sa, int sb, const double* Tseg,
+                                          const double* Tfrom, int total,
                                           const RowShared& sh, int buf, int lane)
 {
     int base = 0;
@@ -644,17 +671,20 @@ __device__ __forceinline__ void g_process(const GrowthDev& g, const NetDev<R>& n
         const int slices = __all_sync(0xffffffffu, one) ? kEvPerLane : 1;
         RowEv v[kEvPerLane];
         double tprev[kEvPerLane];
+        const int have = min(slices * 32, total - base);   // events of this chunk
 #pragma unroll
         for (int k = 0; k < kEvPerLane; ++k) {
-            const int e = base + k * 32 + lane;
-            const bool has = k < slices && e < total;
-            g_eval_load<R>(g, b, i, has, has ? sh.td[buf][e] : 0.0, has ? sh.tgt[buf][e] : -1, has ? sh.spk[buf][e] : 0, v[k]);
+            const int e = base + k * 32 + lane, at = min(e, total - 1);
+            if (k * 32 < have)
+                g_eval_load(g, b, i, e < total, sh.td[buf][at], sh.tgt[buf][at], sh.spk[buf][at], v[k]);
+            else
+                g_eval_none(v[k]);
         }
 #pragma unroll
-        for (int k = 0; k < kEvPerLane; ++k) tprev[k] = g_eval_prev(n, v[k]);
+        for (int k = 0; k < kEvPerLane; ++k) tprev[k] = k * 32 < have ? g_eval_prev(n, v[k]) : 0.0;
         g_eval_steps(sa, sb, Tseg, v);
 #pragma unroll
-        for (int k = 0; k < kEvPerLane; ++k) g_eval_decide(g, n, b, sa, Tseg, tprev[k], rem, sc, v[k]);
+        for (int k = 0; k < kEvPerLane; ++k) g_eval_decide(g, n, b, sa, Tfrom, tprev[k], rem, sc, v[k]);
         if (slices == 1) {
             const unsigned same = __match_any_sync(0xffffffffu, v[0].has ? v[0].t : -1 - lane);
             if (v[0].has && __popc(same) > 1 && lane != __ffs(same) - 1) v[0].changing = true;
@@ -689,7 +719,7 @@ __device__ __forceinline__ void g_process(const GrowthDev& g, const NetDev<R>& n
 }
 
 // One warp, row i of instance b, steps from..to of the interval s0..s1
-// (sh_T holds T[s0..s1]); a spike at `from` has already opened its stream
+// (sh_T: g_stage_times); a spike at `from` has already opened its stream
 // when opened_at_from is set.  bits: the row's somatic spikes of the interval; head / num:
 // its stream ring, st: the ring's slots (cursors are written back at the end).
 template <class R>
@@ -714,7 +744,7 @@ __device__ __forceinline__ void g_row_range(const GrowthDev& g, const NetDev<R>&
             if (lane == 0) num = g_open_stream(g, r, sa, sh_T[sa - s0], Drow, head, num, stS, stC, stL, stT);
             num = __shfl_sync(0xffffffffu, num, 0);
             __syncwarp();
-            st.load(n, stS, stC, stL, head, num, lane);
+            st.load(g, r, lane);
         }
         const uint32_t later = (sa - s0 + 1) < 32 ? bits >> (sa - s0 + 1) : 0u;
         const int sb = later ? min(sa + __ffs(later) - 1, s1) : s1;
@@ -740,7 +770,7 @@ __device__ __forceinline__ void g_row_range(const GrowthDev& g, const NetDev<R>&
                     if (lane == 0) g_drain_seq(g, n, bt, b, i, s, sh_T[s - s0], head, num, stS, stC, stL, stT, perm, Drow);
                     __syncwarp();
                 }
-                st.load(n, stS, stC, stL, head, num, lane);
+                st.load(g, r, lane);
                 break;
             }
             // the cut: smallest last key among the truncated runs
@@ -768,7 +798,7 @@ __device__ __forceinline__ void g_row_range(const GrowthDev& g, const NetDev<R>&
                 }
                 P = lo;
             }
-            g_process(g, n, bt, b, i, r, sa, sb, sh_T + (sa - s0), P, sh, buf, lane);
+            g_process(g, n, bt, b, i, r, sa, sb, sh_T + (sa - s0), sh_T + kSegSteps + (sa - s0), P, sh, buf, lane);
             // advance each stream past its processed prefix
             int adv = 0;
             if (lane < nrun) {
@@ -812,10 +842,10 @@ __device__ __forceinline__ void g_row(const GrowthDev& g, const NetDev<R>& n, co
                                       int& head, int& num, RowStreams& st)
 {
     const size_t r = (size_t)b * g.n + i;
+    st.load(g, r, lane);
     head = g.st_head[r];
     num = g.st_num[r];
     if (bits == 0 && num == 0) return;
-    st.load(n, g.st_step + r * kMaxStreams, g.st_cursor + r * kMaxStreams, g.st_len + r * kMaxStreams, head, num, lane);
     g_row_range(g, n, bt, bits, b, i, s0, s0, s1, false, sh_T, sh, lane, head, num, st);
     if (lane == 0) {
         g.st_head[r] = head;
@@ -884,7 +914,7 @@ struct HeavyShared {
     int mode, slot, spk, head, num, cur, len;
 };
 
-// Block: queued row i of instance b in the interval s0..s1 (sh_T = T[s0..s1]).
+// Block: queued row i of instance b in the interval s0..s1 (sh_T: g_stage_times).
 template <class R>
 __device__ __forceinline__ void g_row_heavy(const GrowthDev& g, const NetDev<R>& n, const BatchDev<R>& bt,
                                             const int* soma, int b, int i, int s0, int s1, const double* sh_T,
@@ -907,7 +937,7 @@ __device__ __forceinline__ void g_row_heavy(const GrowthDev& g, const NetDev<R>&
         if (bits) {
             if (from > s0 && num > 0) {
                 RowStreams st;
-                st.load(n, stS, stC, stL, head, num, lane);
+                st.load(g, r, lane);
                 g_row_range(g, n, bt, bits, b, i, s0, s0, from - 1, false, sh_T, sh, lane, head, num, st);
             }
             if (lane == 0) {
@@ -926,7 +956,7 @@ __device__ __forceinline__ void g_row_heavy(const GrowthDev& g, const NetDev<R>&
                 const int c = stC[sq];
                 if (c >= len) continue;
                 const int t = L < 0 ? stT[sq * kMaxNss + c] : perm[c];
-                if (Tlim >= n.T[stS[sq]] + Drow[t]) {
+                if (Tlim >= g.st_time[r * kMaxStreams + sq] + Drow[t]) {
                     slot = sq;
                     ++ndue;
                 }
@@ -975,13 +1005,13 @@ __device__ __forceinline__ void g_row_heavy(const GrowthDev& g, const NetDev<R>&
 #pragma unroll
             for (int k = 0; k < kEvPerLane; ++k) {
                 const double td = Tsp + tprev[k];
-                g_eval_load<R>(g, b, i, t[k] >= 0 && time_key(Tlim) >= time_key(td), td, t[k], spk, v[k]);
+                g_eval_load(g, b, i, t[k] >= 0 && time_key(Tlim) >= time_key(td), td, t[k], spk, v[k]);
             }
 #pragma unroll
             for (int k = 0; k < kEvPerLane; ++k) tprev[k] = g_eval_prev(n, v[k]);
             g_eval_steps(from, s1, Tseg, v);
 #pragma unroll
-            for (int k = 0; k < kEvPerLane; ++k) g_eval_decide(g, n, b, from, Tseg, tprev[k], rem, sc, v[k]);
+            for (int k = 0; k < kEvPerLane; ++k) g_eval_decide(g, n, b, from, Tseg + kSegSteps, tprev[k], rem, sc, v[k]);
             int due_here = 0;
 #pragma unroll
             for (int k = 0; k < kEvPerLane; ++k) {
@@ -1045,7 +1075,7 @@ __device__ __forceinline__ void g_row_heavy(const GrowthDev& g, const NetDev<R>&
     if (w == 0) {
         int head = hs.head, num = hs.num;
         RowStreams st;
-        st.load(n, stS, stC, stL, head, num, lane);
+        st.load(g, r, lane);
         g_row_range(g, n, bt, bits, b, i, s0, from, s1, bits != 0, sh_T, sh, lane, head, num, st);
         if (lane == 0) {
             g.st_head[r] = head;
@@ -1068,10 +1098,10 @@ __global__ void __launch_bounds__(32 * kRowWarps, 1) k_growth_rows(GrowthDev g, 
                                                                 int s1)
 {
     extern __shared__ __align__(16) unsigned char row_smem[];
-    __shared__ double sh_T[kSegSteps];
+    __shared__ double sh_T[2 * kSegSteps];
     const int b = blockIdx.y;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int k = threadIdx.x; k <= s1 - s0 && k < kSegSteps; k += blockDim.x) sh_T[k] = n.T[s0 + k];
+    g_stage_times(sh_T, n.T, s0, s1);
     __syncthreads();
     const int i = blockIdx.x * kRowWarps + w;
     if (i >= g.n) return;

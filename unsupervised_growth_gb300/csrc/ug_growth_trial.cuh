@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(kTrialThreads, 1)
                    const __grid_constant__ IStep<R> ic, TrialLoop L)
 {
     extern __shared__ __align__(16) unsigned char trial_smem[];
-    __shared__ double sh_T[kSegSteps];
+    __shared__ double sh_T[2 * kSegSteps];
     const int blk = blockIdx.x, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     RowShared& sh = reinterpret_cast<RowShared*>(trial_smem)[w];
     unsigned passed = 0;   // grid barriers passed
@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(kTrialThreads, 1)
         if (last) break;
         if (!grid_barrier_bounded(L.bar, ++passed, g.error, kErrTimeout)) return;
         // phase 2: the queued rows of interval q, a warp each
-        for (int k = threadIdx.x; k <= s1 - s0 && k < kSegSteps; k += blockDim.x) sh_T[k] = n.T[s0 + k];
+        g_stage_times(sh_T, n.T, s0, s1);
         __syncthreads();
         const int nrows = min(bt.act_cnt[q & 1], bt.act_cap);
         const int2* rows = bt.act_rows + (size_t)(q & 1) * bt.act_cap;

@@ -209,7 +209,7 @@ __device__ __forceinline__ bool block_wait(int* error, F&& ready)
 __device__ __forceinline__ void units_rows(const GrowthDev& g, const NetDev<float>& n, const BatchDev<float>& bt,
                                            const UnitsLoop& L, int k, RowShared* row_smem)
 {
-    __shared__ double sh_T[2][kSegSteps];
+    __shared__ double sh_T[2][2 * kSegSteps];
     __shared__ unsigned s_queued;
     __shared__ int s_ok;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -217,7 +217,7 @@ __device__ __forceinline__ void units_rows(const GrowthDev& g, const NetDev<floa
     for (int q = 0; q < L.Q; ++q) {
         const int s0 = q == 0 ? 1 : L.sync_end[q - 1] + 1, s1 = L.sync_end[q];
         double* T = sh_T[q & 1];
-        for (int j = threadIdx.x; j <= s1 - s0 && j < kSegSteps; j += blockDim.x) T[j] = n.T[s0 + j];
+        g_stage_times(T, n.T, s0, s1);
         const unsigned before = (q & 1) ? queued_to[1] : queued_to[0];
         // The interval's rows are known once the HVC(RA) warps are through with it; if this block
         // has any, sync q - 1 must be closed: its post events, and where it had any, every

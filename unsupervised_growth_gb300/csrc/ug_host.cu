@@ -350,7 +350,7 @@ private:
     bool rara_dirty_ = false;       // device synapse lists changed since the static lists were built
     ug::GrowthDev gd_{};
     DevMem gW_, gD_, gPerm_, gActive_, gSuper_, gActList_, gActCnt_, gSupList_, gSupCnt_, gRemod_, gPreStep_,
-        gPreCnt_, gPostStep_, gPostCnt_, gPostLast_, gSpikeLast_, gStStep_, gStCur_, gStLen_, gStTgt_, gStHead_, gStNum_, gNewpost_,
+        gPreCnt_, gPostStep_, gPostCnt_, gPostLast_, gSpikeLast_, gStStep_, gStTime_, gStCur_, gStLen_, gStTgt_, gStHead_, gStNum_, gNewpost_,
         gNewpostCnt_, gSomaBits_, gBad_, gRep_;
     cudaGraphExec_t ggraph_ = nullptr;
     int ggraph_training_ = -1;
@@ -805,7 +805,7 @@ size_t NetImpl<R>::device_bytes() const
                             &mean_inj_, &test_ctl_, &dSyncEnd_})
         t += m->bytes();
     for (const DevMem* m : {&gW_, &gD_, &gPerm_, &gActive_, &gSuper_, &gActList_, &gActCnt_, &gSupList_, &gSupCnt_,
-                            &gRemod_, &gPreStep_, &gPreCnt_, &gPostStep_, &gPostCnt_, &gPostLast_, &gSpikeLast_, &gStStep_, &gStCur_, &gStLen_,
+                            &gRemod_, &gPreStep_, &gPreCnt_, &gPostStep_, &gPostCnt_, &gPostLast_, &gSpikeLast_, &gStStep_, &gStTime_, &gStCur_, &gStLen_,
                             &gStTgt_, &gStHead_, &gStNum_, &gNewpost_, &gNewpostCnt_, &gSomaBits_, &gBad_, &gRep_,
                             &gHist_, &gHead_, &gHsum_, &gHact_, &gFrl_, &gScale_, &gMatf_, &gRest_, &gGca_, &gMature_,
                             &gTar_, &gRepCnt_, &gLoop_})
@@ -830,7 +830,7 @@ size_t NetImpl<R>::footprint(int kind, int B) const
     t += (size_t)ring * 8 * (2 * bra + bi) + (size_t)B * (cap * 8 + 16);
     if (kind == 1) {
         const size_t nn = nra * nra;
-        t += 35 * nn + nra * (4 + 4 * ug::kMaxNss + 12 + 4 * ug::kPostRing + 4 + 16 + 3 * 4 * ug::kMaxStreams +
+        t += 35 * nn + nra * (4 + 4 * ug::kMaxNss + 12 + 4 * ug::kPostRing + 4 + 16 + (3 * 4 + 8) * ug::kMaxStreams +
                               4 * ug::kMaxStreams * ug::kMaxNss + 8 + 64 + 8 + 4 + 4) + 8;
         // per-trial bookkeeping (activity history ring, maturation state)
         t += nra * (4 * (size_t)std::max(h.mat.RATE_WINDOW_LONG, 0) + 8 + 4 + 5 * 8 + 4 + 4) + 32;
@@ -991,6 +991,7 @@ ug_status NetImpl<R>::growth_init(cudaStream_t st)
     UG_TRY(gSpikeLast_.alloc((size_t)n * sizeof(double)));
     if (n >= (1 << 27)) return fail(UG_EINVAL, "growth networks are limited to 2^27 HVC(RA) neurons");
     UG_TRY(gStStep_.alloc((size_t)n * ug::kMaxStreams * sizeof(int)));
+    UG_TRY(gStTime_.alloc((size_t)n * ug::kMaxStreams * sizeof(double)));
     UG_TRY(gStCur_.alloc((size_t)n * ug::kMaxStreams * sizeof(int)));
     UG_TRY(gStLen_.alloc((size_t)n * ug::kMaxStreams * sizeof(int)));
     UG_TRY(gStTgt_.alloc((size_t)n * ug::kMaxStreams * ug::kMaxNss * sizeof(int)));
@@ -1013,7 +1014,10 @@ ug_status NetImpl<R>::growth_init(cudaStream_t st)
                            std::isfinite(h.syn.ACTIVATION_THRESHOLD) && std::isfinite(h.syn.SUPERSYNAPSE_THRESHOLD))
                               ? 1 : 0;
     g.sp.zero_stays = (std::isfinite(h.syn.A_D) && std::isfinite(h.syn.T_0) && std::isfinite(h.syn.T_D) && h.syn.T_D > 0.0 &&
-                       std::isfinite(h.syn.TAU_D) && h.syn.TAU_D > 0.0) ? 1 : 0;
+                       std::isfinite(h.syn.TAU_D) && h.syn.TAU_D > 0.0 &&
+                       !std::isnan(h.syn.ACTIVATION_THRESHOLD) && !std::isnan(h.syn.SUPERSYNAPSE_THRESHOLD)) ? 1 : 0;
+    g.sp.zero_active = 0.0 >= h.syn.ACTIVATION_THRESHOLD ? 1 : 0;
+    g.sp.zero_super = 0.0 >= h.syn.SUPERSYNAPSE_THRESHOLD ? 1 : 0;
     std::memcpy(&g.sp.act_bits, &h.syn.ACTIVATION_THRESHOLD, sizeof(double));
     std::memcpy(&g.sp.sup_bits, &h.syn.SUPERSYNAPSE_THRESHOLD, sizeof(double));
     UG_CUDA(ug::epilogue_bulk_grid<R>(n, 1, &g.epi_blocks));
@@ -1025,7 +1029,7 @@ ug_status NetImpl<R>::growth_init(cudaStream_t st)
     g.post_step = gPostStep_.as<int>(); g.post_cnt = gPostCnt_.as<int>(); g.post_last = gPostLast_.as<double>();
     g.spike_last = gSpikeLast_.as<double>();
     g.max_delay = max_delay_;
-    g.st_step = gStStep_.as<int>(); g.st_cursor = gStCur_.as<int>(); g.st_len = gStLen_.as<int>();
+    g.st_step = gStStep_.as<int>(); g.st_time = gStTime_.as<double>(); g.st_cursor = gStCur_.as<int>(); g.st_len = gStLen_.as<int>();
     g.st_tgt = gStTgt_.as<int>(); g.st_head = gStHead_.as<int>(); g.st_num = gStNum_.as<int>();
     g.newpost = gNewpost_.as<int>(); g.newpost_cnt = gNewpostCnt_.as<int>();
     g.error = error_.as<int>();
