@@ -1,4 +1,5 @@
 // Double-precision kernels (the parity build).  Compiled with -fmad=false.
+#define UG_DOUBLE_UNIT   // the double-precision launchers and their kernels belong to this unit alone
 #include "ug_kernels_inst.cuh"
 
 namespace ug {

@@ -1,6 +1,9 @@
 // Shared body of the per-precision launcher translation units.
 #pragma once
 #include "ug_launch.h"
+#ifdef UG_DOUBLE_UNIT
+#include "ug_f64_lanes.cuh"
+#endif
 
 namespace ug {
 
@@ -30,15 +33,34 @@ inline void launch_noise_events(const NetDev<float>& n, const BatchDev<float>& b
     if (lc.timer) lc.timer->end(lc.main);
 }
 
+#ifdef UG_DOUBLE_UNIT
 // Threads per block of the double-precision integrators: one warp per block for small
 // batches, so that a single trial spreads over as many SMs as it has warps (GB300's FP64
 // pipe is narrow, and a trial of 2000 neurons is only 63 + 18 warps).
 inline int dp_block(int B) { return B < 16 ? 32 : kBlock; }
 
+// Batches up to these many neurons go to the kernels with eight lanes per neuron.  They make
+// eight times the warps with a fifth of the operations each, so they are the faster ones until
+// the FP64 pipes of all sub-partitions are busy.  Measured, one interval of both kernels:
+// 602 HVC(RA) / 150 HVC(I) 2.40 -> 0.41 ms, 4800 / 1200 2.41 -> 0.72, 9600 / 2400 3.57 -> 1.29
+// (general HVC(RA) beside lanes for HVC(I): 0.88, 0.88, 1.40); 16 000 / 4000: lanes for both
+// 2.19, general HVC(RA) 1.67; 40 000 / 10 000 6.21 -> 5.65 with lanes for HVC(I); 16 000 / 16 000
+// 3.62 general, 4.10 with lanes for HVC(I).  Blocks of one warp spread over the SMs: 4 warps of
+// one SM take 76 cycles an operation instead of 64 (602 / 150: blocks of 128 threads 0.44 ms).
+// Recorded neurons (traces, inhibition tracking) stay with the general kernels.
+constexpr int kLanesMaxRA = 10000, kLanesMaxI = 12000, kLanesBlock = 32;
+inline bool dp_lanes(long long neurons, int most) { return neurons <= most; }
+inline unsigned dp_lanes_grid(long long neurons) { return (unsigned)((neurons * kLanes + kLanesBlock - 1) / kLanesBlock); }
+
 inline void launch_i(const NetDev<double>& n, const BatchDev<double>& b, int q, int s0, int s1,
                      const IStep<double>& ic, cudaStream_t st, const LaunchCtx& lc)
 {
     if (lc.timer) lc.timer->begin("k_interval_i", lc.main);
+    if (!b.trace_i && dp_lanes((long long)b.B * n.n_i, kLanesMaxI)) {
+        k_interval_i_lanes<<<dp_lanes_grid((long long)b.B * n.n_i), kLanesBlock, 0, st>>>(n, b, q, s0, s1, ic);
+        if (lc.timer) lc.timer->end(lc.main);
+        return;
+    }
     const int t = dp_block(b.B);
     const dim3 g((n.n_i + t - 1) / t, b.B);
     if (b.trace_i)
@@ -47,6 +69,7 @@ inline void launch_i(const NetDev<double>& n, const BatchDev<double>& b, int q, 
         k_interval_i<double><<<g, t, 0, st>>>(n, b, q, s0, s1, ic);
     if (lc.timer) lc.timer->end(lc.main);
 }
+#endif
 
 inline void launch_i(const NetDev<float>& n, const BatchDev<float>& b, int q, int s0, int s1, const IStep<float>& ic,
                      cudaStream_t st, const LaunchCtx& lc)
@@ -166,18 +189,22 @@ cudaError_t launch_test_trial(const NetDev<R>& n, const BatchDev<R>& b, const RA
 
 // HVC(RA) interval kernel: the double build steps one neuron per thread, the
 // single build two neurons per thread with packed f32x2 arithmetic.
+#ifdef UG_DOUBLE_UNIT
 inline void launch_ra(const NetDev<double>& n, const BatchDev<double>& b, int q, int s0, int s1,
                       const RAStep<double>& rc, const LaunchCtx& lc)
 {
     const int t = dp_block(b.B);
     const dim3 g((n.n_ra + t - 1) / t, b.B);
     if (lc.timer) lc.timer->begin("k_interval_ra", lc.main);
-    if (b.ginh_slot || b.trace_ra)
+    if (!b.ginh_slot && !b.trace_ra && dp_lanes((long long)b.B * n.n_ra, kLanesMaxRA))
+        k_interval_ra_lanes<<<dp_lanes_grid((long long)b.B * n.n_ra), kLanesBlock, 0, lc.main>>>(n, b, q, s0, s1, rc);
+    else if (b.ginh_slot || b.trace_ra)
         k_interval_ra<double, true><<<g, t, 0, lc.main>>>(n, b, q, s0, s1, rc);
     else
         k_interval_ra<double><<<g, t, 0, lc.main>>>(n, b, q, s0, s1, rc);
     if (lc.timer) lc.timer->end(lc.main);
 }
+#endif
 
 inline void launch_ra(const NetDev<float>& n, const BatchDev<float>& b, int q, int s0, int s1, const RAStep<float>& rc,
                       const LaunchCtx& lc)
