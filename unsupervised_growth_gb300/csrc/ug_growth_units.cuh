@@ -114,7 +114,7 @@ __device__ __forceinline__ bool ra_wait(const UnitsLoop& L, int q, int* error)
     return ok;
 }
 
-template <class V>
+template <class V, bool kTrack>
 __device__ __forceinline__ void units_ra(const NetDev<float>& n, const BatchDev<float>& bt, const RAStep<float>& rc,
                                          const UnitsLoop& L, int unit)
 {
@@ -138,7 +138,7 @@ __device__ __forceinline__ void units_ra(const NetDev<float>& n, const BatchDev<
         for (int k = 0; k < N; ++k) live[k] = u.valid[k] ? __ldcg(&bt.live_streams[u.ent[k]]) : 0;
         const int s1 = L.sync_end[q];
         uint32_t soma[N] = {}, dend[N] = {};
-        u.template steps<false>(n, bt, rc, s0, s1, soma, dend);
+        u.template steps<kTrack>(n, bt, rc, s0, s1, soma, dend);
         unsigned queued = 0;
 #pragma unroll
         for (int k = 0; k < N; ++k) {
@@ -164,6 +164,7 @@ __device__ __forceinline__ void units_ra(const NetDev<float>& n, const BatchDev<
     u.store(n, bt);
 }
 
+template <bool kTrack>
 __device__ __forceinline__ void units_i(const NetDev<float>& n, const BatchDev<float>& bt, const IStep<float>& ic,
                                         const UnitsLoop& L, int unit)
 {
@@ -184,7 +185,7 @@ __device__ __forceinline__ void units_i(const NetDev<float>& n, const BatchDev<f
         if (q == L.Q) break;
         const int s1 = L.sync_end[q];
         uint32_t fired = 0;
-        u.template steps<false>(n, bt, ic, s0, s1, i, 0, fired);
+        u.template steps<kTrack>(n, bt, ic, s0, s1, i, any ? 0 : 1, fired);   // traces are of instance 0
         if (!any) fired = 0;
         i_scatter(n, bt, fired, i, 0, s0);
         __syncwarp();
@@ -329,8 +330,11 @@ __device__ __forceinline__ void units_sync(const GrowthDev& g, const NetDev<floa
     }
 }
 
-// V: the lane type of the HVC(RA) warps.
-template <class V>
+// V: the lane type of the HVC(RA) warps.  kTrack: traces of the listed neurons and inhibition
+// tracking (a kernel of its own, as for the interval kernels: 450 / 113 with every neuron's
+// inhibition at 1 ms, a trial with its weights read back 116 -> 31.6 ms against five
+// launches per interval).
+template <class V, bool kTrack>
 __global__ void __launch_bounds__(kTrialThreads, 1)
     k_growth_units(GrowthDev g, NetDev<float> n, BatchDev<float> bt, RAStep<float> rc,
                    const __grid_constant__ IStep<float> ic, UnitsLoop L)
@@ -340,13 +344,13 @@ __global__ void __launch_bounds__(kTrialThreads, 1)
     const int w = (int)(threadIdx.x >> 5);
     if (blk < L.nb_ra) {
         const int unit = blk * L.ra_per + w;
-        if (w < L.ra_per && unit < L.ra_units) units_ra<V>(n, bt, rc, L, unit);
+        if (w < L.ra_per && unit < L.ra_units) units_ra<V, kTrack>(n, bt, rc, L, unit);
         return;
     }
     blk -= L.nb_ra;
     if (blk < L.nb_i) {
         const int unit = blk * L.i_per + w;
-        if (w < L.i_per && unit < L.i_units) units_i(n, bt, ic, L, unit);
+        if (w < L.i_per && unit < L.i_units) units_i<kTrack>(n, bt, ic, L, unit);
         return;
     }
     blk -= L.nb_i;

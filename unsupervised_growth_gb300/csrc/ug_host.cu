@@ -384,8 +384,9 @@ private:
     // trial_grid(lc) has sized trial_plan_ before any use of this
     bool one_launch(const ug::LaunchCtx& lc) const
     {
+        const bool recording = bd_.trace_ra || bd_.trace_i || bd_.ginh_slot;   // the double build's trial has no such form
         return lc.trial_launch && !lc.timer && trial_key_ == trial_key(lc) && trial_plan_.blocks > 0 && bd_.B == 1 &&
-               !bd_.trace_ra && !bd_.trace_i && !bd_.ginh_slot;
+               (sizeof(R) == 4 || !recording);
     }
     DevMem gTrRaSlot_, gTrISlot_, gTrRaBuf_, gTrIBuf_;   // per-neuron traces
     void apply_recording()

@@ -337,8 +337,11 @@ cudaError_t growth_trial_plan(int n_ra, int n_i, int req_ra, int req_i, GrowthPl
     if (e != cudaSuccess || !coop || !trial_widths(req_ra, req_i, &ra_w, &i_w)) return e;
     if constexpr (sizeof(R) == 4) {
         for (int lanes = 1; lanes <= 2 && plan->blocks == 0; ++lanes) {
-            e = units_attributes(lanes == 1 ? (const void*)k_growth_units<float> : (const void*)k_growth_units<f2>);
-            if (e != cudaSuccess) return e;
+            for (const void* f : {lanes == 1 ? (const void*)k_growth_units<float, false> : (const void*)k_growth_units<f2, false>,
+                                  lanes == 1 ? (const void*)k_growth_units<float, true> : (const void*)k_growth_units<f2, true>}) {
+                e = units_attributes(f);
+                if (e != cudaSuccess) return e;
+            }
             // by default as few warps to a block as leave the rows enough blocks
             for (int per = 1; per <= kTrialWarps && plan->blocks == 0; per *= 2) {
                 UnitsLoop u{};
@@ -400,8 +403,11 @@ cudaError_t launch_growth_trial(const GrowthDev& g, const NetDev<R>& n, BatchDev
         L.rows = act_rows;
         L.rows_cap = 2 * n.n_ra;
         b.soma_bits = nullptr;   // the spike bits travel with the queued rows
-        return plan.lanes == 1 ? cudaLaunchKernelEx(&cfg, k_growth_units<float>, g, n, b, rc, ic, L)
-                               : cudaLaunchKernelEx(&cfg, k_growth_units<f2>, g, n, b, rc, ic, L);
+        if (b.trace_ra || b.trace_i || b.ginh_slot)
+            return plan.lanes == 1 ? cudaLaunchKernelEx(&cfg, k_growth_units<float, true>, g, n, b, rc, ic, L)
+                                   : cudaLaunchKernelEx(&cfg, k_growth_units<f2, true>, g, n, b, rc, ic, L);
+        return plan.lanes == 1 ? cudaLaunchKernelEx(&cfg, k_growth_units<float, false>, g, n, b, rc, ic, L)
+                               : cudaLaunchKernelEx(&cfg, k_growth_units<f2, false>, g, n, b, rc, ic, L);
     } else {
         TrialLoop L = plan.trial;
         L.sync_end = sync_end;
