@@ -439,7 +439,17 @@ struct Gauss {
     float inv2s2;   // 1 / (2 sigma^2)
     float rel;      // relative half-width of the band decided in double precision
     int exact;      // 1: every pair below wA in double precision
+    float near_[33];   // by the leading zeros of the pair's word: the closeness a connection needs
 };
+
+// How close two points are in single precision: the dot product (sphere) or minus the squared
+// distance (square), the larger the closer.
+__device__ inline float closeness32(const Geo& g, float4 a, float4 b)
+{
+    if (g.sphere) return __fmaf_rn(a.z, b.z, __fmaf_rn(a.y, b.y, __fmul_rn(a.x, b.x)));
+    const float dx = __fsub_rn(a.x, b.x), dy = __fsub_rn(a.y, b.y);
+    return -__fmaf_rn(dy, dy, __fmul_rn(dx, dx));
+}
 
 // the reference's test (:651-652): random(1) < A exp(-d^2 / (2 sigma^2)), in double precision
 __device__ inline bool connect_exact(const Geo& g, const Gauss& q, const double* a, const double* b, uint32_t w)
@@ -475,41 +485,73 @@ __device__ inline bool connect(const Geo& g, const Gauss& q, float4 a32, float4 
 }
 
 // RA->I or I->RA decisions (:649-690) as bit words of 32 targets, and the per-row counts.
-// A lane decides four targets from one Philox block, 128 targets per warp pass.
+// A lane decides four targets from one Philox block, 128 targets per warp pass.  A word with c
+// leading zeros is at least 2^(31 - c), so it connects only within the distance at which
+// A exp(-d^2 / 2 sigma^2) falls to 2^-(c + 1): one comparison of the closeness with near_[c]
+// leaves about twice the pairs that connect (some thousandths; the word alone left a tenth, at
+// least one lane of every warp), and a warp takes them up one per lane and round.
+// The block's eight rows share tiles of target coordinates in shared memory (a lane reads its
+// four targets as three vectors; the same loads from the L1 cache, 64 bytes apart, took more
+// cycles than the Philox rounds, which are what is left).  20 000 x 5000: 0.46 ms for both directions,
+// 1.0 ms with the word alone as the filter.
+constexpr int kConnTile = 1024;
 __global__ void __launch_bounds__(kRowThreads) k_conn_decide(Geo g, Gauss q, const double* src, const float4* src32,
                                                              int n_src, const double* dst, const float4* dst32,
                                                              int n_dst, uint32_t part, unsigned* bits, int nw,
                                                              int* rowcnt)
 {
+    __shared__ __align__(16) float s_xyz[3][kConnTile];
+    __shared__ float s_near[33];
+    if (threadIdx.x < 33) s_near[threadIdx.x] = q.near_[threadIdx.x];
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * (kRowThreads / 32) + (threadIdx.x >> 5);
-    if (row >= n_src) return;
-    const double* a = src + 3 * row;
-    const float4 a32 = src32[row];
+    const bool mine = row < n_src;
+    const double* a = src + 3 * (mine ? row : 0);
+    const float4 a32 = src32[mine ? row : 0];
     const ug::StreamId s = ug::make_stream(g.seed, ug::kNoiseTopology, g.net, (uint32_t)row, part);
     int cnt = 0;
-    for (int c0 = 0; c0 < n_dst; c0 += 128) {
-        const int j0 = c0 + 4 * lane;
-        unsigned m = 0;
-        if (j0 < n_dst) {
-            const ug::Philox4 b = ug::stream_block(s, (uint32_t)(j0 >> 2));
-            const uint32_t w[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int j = j0 + c;
-                if (j < n_dst && (long long)w[c] < q.wA && connect(g, q, a32, dst32[j], a, dst + 3 * j, w[c]))
-                    m |= 1u << c;
-            }
+    for (int t0 = 0; t0 < n_dst; t0 += kConnTile) {
+        const int tn = min(kConnTile, n_dst - t0);
+        __syncthreads();
+        for (int k = threadIdx.x; k < tn; k += kRowThreads) {
+            const float4 p = dst32[t0 + k];
+            s_xyz[0][k] = p.x;
+            s_xyz[1][k] = p.y;
+            s_xyz[2][k] = p.z;
         }
-        // lanes 8k .. 8k+7 make word k of this pass
-        unsigned v = m << (4 * (lane & 7));
-        v |= __shfl_xor_sync(0xffffffffu, v, 1);
-        v |= __shfl_xor_sync(0xffffffffu, v, 2);
-        v |= __shfl_xor_sync(0xffffffffu, v, 4);
-        const int wi = (c0 >> 5) + (lane >> 3);
-        if ((lane & 7) == 0 && wi < nw) bits[(size_t)row * nw + wi] = v;
-        cnt += __popc(m);
+        __syncthreads();
+        if (!mine) continue;
+        for (int c0 = t0; c0 < t0 + tn; c0 += 128) {
+            const int j0 = c0 + 4 * lane;
+            unsigned m = 0, maybe = 0;
+            const ug::Philox4 b = ug::stream_block(s, (uint32_t)(j0 >> 2));
+            const float4 x = *reinterpret_cast<const float4*>(&s_xyz[0][j0 - t0]);   // past the tile's end: old values
+            const float4 y = *reinterpret_cast<const float4*>(&s_xyz[1][j0 - t0]);
+            const float4 z = *reinterpret_cast<const float4*>(&s_xyz[2][j0 - t0]);
+            maybe |= (unsigned)!(closeness32(g, a32, make_float4(x.x, y.x, z.x, 0.f)) < s_near[__clz((int)b.x)]);
+            maybe |= (unsigned)!(closeness32(g, a32, make_float4(x.y, y.y, z.y, 0.f)) < s_near[__clz((int)b.y)]) << 1;
+            maybe |= (unsigned)!(closeness32(g, a32, make_float4(x.z, y.z, z.z, 0.f)) < s_near[__clz((int)b.z)]) << 2;
+            maybe |= (unsigned)!(closeness32(g, a32, make_float4(x.w, y.w, z.w, 0.f)) < s_near[__clz((int)b.w)]) << 3;
+            if (j0 + 4 > n_dst) maybe &= j0 < n_dst ? (1u << (n_dst - j0)) - 1u : 0u;
+            while (__any_sync(0xffffffffu, maybe != 0)) {
+                if (maybe) {
+                    const int c = __ffs(maybe) - 1, j = j0 + c;
+                    const uint32_t w = c == 0 ? b.x : c == 1 ? b.y : c == 2 ? b.z : b.w;
+                    if ((long long)w < q.wA && connect(g, q, a32, dst32[j], a, dst + 3 * j, w)) m |= 1u << c;
+                    maybe &= maybe - 1;
+                }
+            }
+            // lanes 8k .. 8k+7 make word k of this pass
+            unsigned v = m << (4 * (lane & 7));
+            v |= __shfl_xor_sync(0xffffffffu, v, 1);
+            v |= __shfl_xor_sync(0xffffffffu, v, 2);
+            v |= __shfl_xor_sync(0xffffffffu, v, 4);
+            const int wi = (c0 >> 5) + (lane >> 3);
+            if ((lane & 7) == 0 && wi < nw) bits[(size_t)row * nw + wi] = v;
+            cnt += __popc(m);
+        }
     }
+    if (!mine) return;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
     if (lane == 0) rowcnt[row] = cnt;
@@ -531,15 +573,13 @@ __global__ void __launch_bounds__(1024) k_scan(const int* cnt, int n, int* off)
     if (threadIdx.x == 0) off[n] = carry;
 }
 
-// targets and lengths of the kept pairs, by source then target
-__global__ void __launch_bounds__(kRowThreads) k_conn_fill(Geo g, const double* src, int n_src, const double* dst,
-                                                           const unsigned* bits, int nw, const int* off, int* tgt,
-                                                           double* len)
+// targets of the kept pairs, by source then target, and the source of each
+__global__ void __launch_bounds__(kRowThreads) k_conn_fill(int n_src, const unsigned* bits, int nw, const int* off,
+                                                           int* tgt, int* from)
 {
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * (kRowThreads / 32) + (threadIdx.x >> 5);
     if (row >= n_src) return;
-    const double* a = src + 3 * row;
     int base = off[row];
     for (int w0 = 0; w0 < nw; w0 += 32) {
         const int wi = w0 + lane;
@@ -553,14 +593,24 @@ __global__ void __launch_bounds__(kRowThreads) k_conn_fill(Geo g, const double* 
         }
         int pos = base + incl - c;
         while (m) {
-            const int j = 32 * wi + __ffs(m) - 1;
+            tgt[pos] = 32 * wi + __ffs(m) - 1;
+            from[pos] = row;
             m &= m - 1;
-            tgt[pos] = j;
-            len[pos] = dist(g, a, dst + 3 * j) * kExpDist / g.model;
             ++pos;
         }
         base += __shfl_sync(0xffffffffu, incl, 31);
     }
+}
+
+// The lengths of the connections, a thread each: the double-precision arc cosine is a chain of
+// operations that hold a warp 64 cycles however few lanes take part, and a row's connections
+// come to few lanes at a time (in the fill itself, 20 000 x 5000: both fills 238 us,
+// now 29 and 18 here).
+__global__ void __launch_bounds__(kRowThreads) k_conn_lengths(Geo g, const double* src, const double* dst, const int* from,
+                                                              const int* tgt, int n, double* len)
+{
+    const int e = blockIdx.x * kRowThreads + threadIdx.x;
+    if (e < n) len[e] = dist(g, src + 3 * from[e], dst + 3 * tgt[e]) * kExpDist / g.model;
 }
 
 // ------------------------------------------------------------------ host side
@@ -653,6 +703,19 @@ Gauss make_gauss(const Geo& g, double A, double sigma)
     q.logA = A > 0 ? (float)std::log(A) : 0.f;
     q.scale = (float)scale;
     q.inv2s2 = q.exact ? 0.f : (float)inv;
+    // random(1) of a word with c leading zeros is at least 2^-(c + 1), so a connection needs
+    // x < log(A) + (c + 1) log(2); the word 0, and `exact`, filter nothing.  The copies' dot product
+    // is off by less than 3e-7 (the margin: 2e-6), their distance by 5e-7 (1e-5 d^2 + 2e-6 of d^2).
+    for (int c = 0; c < 33; ++c) {
+        q.near_[c] = -8.f;
+        if (q.exact || c == 32) continue;
+        const double x = std::max(0.0, std::log(A) + (c + 1) * std::log(2.0)) + 1e-3;
+        const double d = std::sqrt(x / inv) / scale;   // on the unit sphere or square
+        if (g.sphere)
+            q.near_[c] = d < kPi ? (float)(std::cos(d) - 2e-6) : -8.f;
+        else
+            q.near_[c] = (float)(-d * d * (1 + 1e-5) - 2e-6);
+    }
     q.rel = (float)(g.sphere ? 0.02 + 8e-7 / (g.too_close * std::sin(g.too_close)) : 0.02 + 2e-6 / g.too_close);
     return q;
 }
@@ -825,11 +888,22 @@ ug_status generate(ug_ctx* ctx, const ug_topology_params& p, int n_ra, int n_i, 
     TCUDA(mem.get(&tgt_ir, totals[1]));
     TCUDA(mem.get(&len_ri, totals[0]));
     TCUDA(mem.get(&len_ir, totals[1]));
-    k_conn_fill<<<(n_ra + rows - 1) / rows, kRowThreads, 0, st>>>(g, ra, n_ra, ii, bits_ri, nw_ri, off_ri, tgt_ri,
-                                                                 len_ri);
-    k_conn_fill<<<(n_i + rows - 1) / rows, kRowThreads, 0, st>>>(g, ii, n_i, ra, bits_ir, nw_ir, off_ir, tgt_ir,
-                                                                len_ir);
+    int *from_ri = nullptr, *from_ir = nullptr;
+    TCUDA(mem.get(&from_ri, totals[0]));
+    TCUDA(mem.get(&from_ir, totals[1]));
+    k_conn_fill<<<(n_ra + rows - 1) / rows, kRowThreads, 0, st>>>(n_ra, bits_ri, nw_ri, off_ri, tgt_ri, from_ri);
+    k_conn_fill<<<(n_i + rows - 1) / rows, kRowThreads, 0, st>>>(n_i, bits_ir, nw_ir, off_ir, tgt_ir, from_ir);
     launches += 2;
+    if (totals[0]) {
+        k_conn_lengths<<<(totals[0] + kRowThreads - 1) / kRowThreads, kRowThreads, 0, st>>>(g, ra, ii, from_ri, tgt_ri,
+                                                                                         totals[0], len_ri);
+        ++launches;
+    }
+    if (totals[1]) {
+        k_conn_lengths<<<(totals[1] + kRowThreads - 1) / kRowThreads, kRowThreads, 0, st>>>(g, ii, ra, from_ir, tgt_ir,
+                                                                                         totals[1], len_ir);
+        ++launches;
+    }
     TCUDA(cudaGetLastError());
     TCUDA(cudaEventRecord(ev1, st));
     t.ra_xyz.resize(3 * (size_t)n_ra);
