@@ -196,8 +196,8 @@ __global__ void __launch_bounds__(kBlock, 1) k_interval_ra_lanes(NetDev<double> 
         spikes |= (uint32_t)(c == 2 ? !fl && high : fl && low) << (st - s0);
         fl = fl ? !low : high;
         const Philox4 w = stream_block(sid, (uint32_t)st - 1);
-        ra_debrabant_lane(k, s, G, rc.dt, e1, e2, ra_point(point_index(c == 2 ? w.z : w.x), 0.0),
-                          ra_point(point_index(c == 2 ? w.w : w.y), 0.0));
+        ra_debrabant_lane(k, s, G, rc.dt, e1, e2, ra_point(point_index(c == 2 ? w.z : w.x)),
+                          ra_point(point_index(c == 2 ? w.w : w.y)));
     }
     const uint32_t dend = __shfl_sync(0xffffffffu, spikes, 2, kLanes);
     const int fd = __shfl_sync(0xffffffffu, fl, 2, kLanes);
@@ -280,7 +280,7 @@ __device__ __forceinline__ double i_rhs_lane(const ILanes& k, double y, double G
     return c == 0 ? kV : c <= 3 ? kk : c == 4 ? kw : 1.0;
 }
 
-// One DP8 step of the lane's component (i_dp8<double>); d: the decay factors of the lane's G.
+// One DP8 step of the lane's component (i_dp8); d: the decay factors of the lane's G.
 __device__ __forceinline__ void i_dp8_lane(const ILanes& ln, double& s, double& G, double dt, const double* d)
 {
     const DPT B7[] = {UG_DP_B7}, B8[] = {UG_DP_B8}, B9[] = {UG_DP_B9}, B10[] = {UG_DP_B10}, B11[] = {UG_DP_B11},

@@ -1,4 +1,5 @@
-// Neuron integrators of the trial path, one neuron per thread.
+// Neuron integrators of the double build, one neuron per thread, and the neuron
+// constants and states of both builds.
 //
 //  * HVC(RA): two-compartment Hodgkin-Huxley neuron (c++/include/HH2_test.h,
 //    c++/src/HH2_test.cpp) advanced by the 4-stage Debrabant weak-order-3
@@ -7,12 +8,10 @@
 //    c++/src/HHI_buffer.cpp) advanced by the 12-stage Dormand-Prince 8 step
 //    (HHI_buffer.cpp:426-690) with Poisson conductance noise.
 //
-// The double instantiation follows the reference's operation order term by
-// term (the translation unit is compiled without multiply-add contraction), so
-// it reproduces the reference's double-precision results up to the last-bit
-// differences of the device exp().  The float instantiation computes the same
-// equations with SFU exponentials and merged reciprocals (8 ex2 + 7 rcp per RA
-// stage, 7 ex2 + 4 rcp per I stage).
+// They follow the reference's operation order term by term (the translation unit
+// is compiled without multiply-add contraction), so they reproduce the reference's
+// double-precision results up to the last-bit differences of the device exp().
+// ug_ra_f32.cuh and ug_i_f32.cuh hold the single build's forms.
 //
 // RA somatic conductances are not carried: on the trial path HVC(RA) neurons
 // get no Poisson noise (set_noise, NetworkGrowthSimulator.cpp:2061-2075) and
@@ -72,15 +71,10 @@ inline void philox_key_schedule(uint64_t seed, uint32_t* ks)
     }
 }
 
-__device__ __forceinline__ double ra_point(int idx, double)
+__device__ __forceinline__ double ra_point(int idx)
 {
     const double s6 = 2.449489742783178098197284;  // sqrt(6) (the reference computes sqrt(6) in double)
     return idx == 0 ? s6 : idx == 1 ? -s6 : idx <= 10 ? 1.0 : idx <= 19 ? -1.0 : 0.0;
-}
-__device__ __forceinline__ float ra_point(int idx, float)
-{
-    const float s6 = 2.4494897f;
-    return idx == 0 ? s6 : idx == 1 ? -s6 : idx <= 10 ? 1.0f : idx <= 19 ? -1.0f : 0.0f;
 }
 
 // ------------------------------------------------------------ RA, double
@@ -154,111 +148,24 @@ __device__ __forceinline__ void ra_debrabant(RAState<double>& s, double EL, doub
     s.Gi = s.Gi * p.e1;
 }
 
-// ------------------------------------------------------------- RA, float
-struct RAKf { float Vs, Vd, n, l, h, r, c, Ca; };
-
-__device__ __forceinline__ float fexp(float x) { return __expf(x); }
-__device__ __forceinline__ float frcp(float x) { return __fdividef(1.0f, x); }
-
-__device__ __forceinline__ RAKf ra_rhs_f(float vs, float vd, float n, float h, float l, float r, float c, float ca,
-                                        float Ge_d, float Gi_d, float EL, float GdCa, float mu_term_s, float mu_term_d)
-{
-    typedef RAConst K;
-    RAKf k;
-    const float m = frcp(1.0f + fexp((vs + 30.0f) * (-1.0f / 9.5f)));
-    const float m3 = m * m * m;
-    const float n2 = n * n;
-    const float n4 = n2 * n2;
-    const float coup_s = (vd - vs) * (float)(100000.0 / (K::Rc * K::As));
-    k.Vs = -(float)K::GsL * (vs - EL) - (float)K::GsNa * m3 * h * (vs - (float)K::EsNa)
-           - ((float)K::GsK * n4 + (float)K::GsKLT * l) * (vs - (float)K::EsK) + mu_term_s + coup_s;
-    // GdCaK (vd - EdK) c / (1 + 6/ca) = GdCaK (vd - EdK) c ca / (ca + 6)
-    const float cak = (float)K::GdCaK * (vd - (float)K::EdK) * c * ca * frcp(ca + 6.0f);
-    k.Vd = -(float)K::GdL * (vd - EL) - GdCa * r * r * (vd - (float)K::EdCa) - cak - Ge_d * vd
-           - Gi_d * (vd - (float)K::Egaba) + mu_term_d + (vs - vd) * (float)(100000.0 / (K::Rc * K::Ad));
-    // kn = (nInf - n) / tauN with nInf = 1/(1+En), tauN = 0.1 + 0.5/(1+Et): one reciprocal
-    {
-        const float En = fexp((vs + 35.0f) * -0.1f);
-        const float Et = fexp((vs + 27.0f) * (1.0f / 15.0f));
-        const float a = 1.0f + En, b = 1.0f + Et;
-        k.n = (1.0f - n * a) * b * frcp(a * (0.1f * b + 0.5f));
-    }
-    k.l = (frcp(1.0f + fexp((vs + 40.0f) * -0.2f)) - l) * 0.1f;
-    {
-        const float Eh = fexp((vs + 45.0f) * (1.0f / 7.0f));
-        const float Et = fexp((vs + 40.5f) * (1.0f / 6.0f));
-        const float a = 1.0f + Eh, b = 1.0f + Et;
-        k.h = (1.0f - h * a) * b * frcp(a * (0.1f * b + 0.75f));
-    }
-    k.r = frcp(1.0f + fexp((vd + 5.0f) * -0.1f)) - r;
-    k.c = (frcp(1.0f + fexp((vd - 10.0f) * (-1.0f / 7.0f))) - c) * (1.0f / 15.0f);
-    k.Ca = (-0.1f * GdCa) * r * r * (vd - (float)K::EdCa) - 0.02f * ca;
-    return k;
-}
-
-__device__ __forceinline__ void ra_debrabant(RAState<float>& s, float EL, float GdCa, const RAStep<float>& p,
-                                             float J1s, float J2s, float J1d, float J2d)
-{
-    typedef RAConst K;
-    const float dt = p.dt;
-    const float ns = p.sq * p.sig_s * (float)(1.0 / (K::As * K::cm));
-    const float nd = p.sq * p.sig_d * (float)(1.0 / (K::Ad * K::cm));
-    const float mus = (float)(100000.0 / K::As) * p.mu_s, mud = (float)(100000.0 / K::Ad) * p.mu_d;
-    const float Ge1 = s.Ge * p.e1, Gi1 = s.Gi * p.e1, Ge2 = s.Ge * p.e2, Gi2 = s.Gi * p.e2;
-
-    const RAKf a1 = ra_rhs_f(s.Vs + ns * (-0.01844540496323970f * J1s - 0.1866426386543421f * J2s),
-                             s.Vd + nd * (-0.01844540496323970f * J1d - 0.1866426386543421f * J2d), s.n, s.h, s.l, s.r,
-                             s.c, s.Ca, s.Ge, s.Gi, EL, GdCa, mus, mud);
-    const RAKf a2 = ra_rhs_f(s.Vs + dt * a1.Vs + ns * (0.8017012756521233f * J1s - 0.8575745885712401f * J2s),
-                             s.Vd + dt * a1.Vd + nd * (0.8017012756521233f * J1d - 0.8575745885712401f * J2d),
-                             s.n + dt * a1.n, s.h + dt * a1.h, s.l + dt * a1.l, s.r + dt * a1.r, s.c + dt * a1.c,
-                             s.Ca + dt * a1.Ca, Ge1, Gi1, EL, GdCa, mus, mud);
-    const float d8 = dt * 0.125f;
-    const RAKf a3 = ra_rhs_f(s.Vs + d8 * (3.0f * a1.Vs + a2.Vs) + ns * (0.5092227024816198f * J1s - 0.4723392695015512f * J2s),
-                             s.Vd + d8 * (3.0f * a1.Vd + a2.Vd) + nd * (0.5092227024816198f * J1d - 0.4723392695015512f * J2d),
-                             s.n + d8 * (3.0f * a1.n + a2.n), s.h + d8 * (3.0f * a1.h + a2.h), s.l + d8 * (3.0f * a1.l + a2.l),
-                             s.r + d8 * (3.0f * a1.r + a2.r), s.c + d8 * (3.0f * a1.c + a2.c), s.Ca + d8 * (3.0f * a1.Ca + a2.Ca),
-                             Ge2, Gi2, EL, GdCa, mus, mud);
-    const float b1 = -0.4526683126055039f, b2 = -0.4842227708685013f, b3 = 1.9368910834740051f;
-#define UG_H4(f) (s.f + dt * (b1 * a1.f + b2 * a2.f + b3 * a3.f))
-    const RAKf a4 = ra_rhs_f(UG_H4(Vs) + ns * (0.9758794209767762f * J1s + 0.3060354860326548f * J2s),
-                             UG_H4(Vd) + nd * (0.9758794209767762f * J1d + 0.3060354860326548f * J2d), UG_H4(n), UG_H4(h),
-                             UG_H4(l), UG_H4(r), UG_H4(c), UG_H4(Ca), Ge1, Gi1, EL, GdCa, mus, mud);
-#undef UG_H4
-    const float q1 = 1.0f / 6.0f, q2 = -0.005430430675258792f, q3 = 2.0f / 3.0f, q4 = 0.1720970973419255f;
-#define UG_UPD(f) (s.f + dt * (q1 * a1.f + q2 * a2.f + q3 * a3.f + q4 * a4.f))
-    s.Vs = UG_UPD(Vs) + ns * 100000.0f * J1s;
-    s.Vd = UG_UPD(Vd) + nd * 100000.0f * J1d;
-    s.Ca = UG_UPD(Ca);
-    s.n = UG_UPD(n);
-    s.l = UG_UPD(l);
-    s.h = UG_UPD(h);
-    s.r = UG_UPD(r);
-    s.c = UG_UPD(c);
-#undef UG_UPD
-    s.Ge = Ge1;
-    s.Gi = Gi1;
-}
-
 // Spike detection on the state before the step (HH2_test::state_check,
 // HH2_test.cpp:561-594).  flags bit0 = soma flag, bit1 = dendrite flag.
-template <class R>
-__device__ __forceinline__ void ra_state_check(const RAState<R>& s, int& flags, bool& fired_soma, bool& fired_dend)
+__device__ __forceinline__ void ra_state_check(const RAState<double>& s, int& flags, bool& fired_soma, bool& fired_dend)
 {
     const int fs = flags & 1, fd = (flags >> 1) & 1;
     int nfs = fs, nfd = fd;
     fired_soma = false;
     fired_dend = false;
-    if (fs == 1 && s.Vs < R(-35.0)) {
+    if (fs == 1 && s.Vs < -35.0) {
         nfs = 0;
         fired_soma = true;
-    } else if (fs == 0 && s.Vs > R(-30.0)) {
+    } else if (fs == 0 && s.Vs > -30.0) {
         nfs = 1;
     }
-    if (fd == 0 && s.Vd >= R(-30.0)) {
+    if (fd == 0 && s.Vd >= -30.0) {
         nfd = 1;
         fired_dend = true;
-    } else if (fd == 1 && s.Vd < R(-35.0)) {
+    } else if (fd == 1 && s.Vd < -35.0) {
         nfd = 0;
     }
     flags = (flags & ~3) | nfs | (nfd << 1);
@@ -267,14 +174,13 @@ __device__ __forceinline__ void ra_state_check(const RAState<R>& s, int& flags, 
 // One trial-path RA step: check, draw the step's 4 point indices (block
 // `step-1` of the neuron's stream, in the order ind1s, ind2s, ind1d, ind2d,
 // HH2_test.cpp:640-643), integrate.
-template <class R>
-__device__ __forceinline__ void ra_step(RAState<R>& s, int& flags, bool& fired_soma, bool& fired_dend, R EL, R GdCa,
-                                        const RAStep<R>& p, const StreamId& sid, uint32_t step)
+__device__ __forceinline__ void ra_step(RAState<double>& s, int& flags, bool& fired_soma, bool& fired_dend, double EL,
+                                        double GdCa, const RAStep<double>& p, const StreamId& sid, uint32_t step)
 {
     ra_state_check(s, flags, fired_soma, fired_dend);
     const Philox4 w = stream_block(sid, step - 1);
-    ra_debrabant(s, EL, GdCa, p, ra_point(point_index(w.x), R(0)), ra_point(point_index(w.y), R(0)),
-                 ra_point(point_index(w.z), R(0)), ra_point(point_index(w.w), R(0)));
+    ra_debrabant(s, EL, GdCa, p, ra_point(point_index(w.x)), ra_point(point_index(w.y)),
+                 ra_point(point_index(w.z)), ra_point(point_index(w.w)));
 }
 
 // -------------------------------------------------------------- I, DP8
@@ -329,33 +235,7 @@ __device__ __forceinline__ IKd i_rhs_d(double v, double h, double w, double m3, 
     return k;
 }
 
-struct IKf { float V, n, m, h, w; };
-
-// x / (1 - exp(-x/10)) with its removable singularity at x = 0 handled by the series 10 (1 + x/20 + x^2/1200)
-__device__ __forceinline__ float i_vtrap(float x)
-{
-    if (fabsf(x) < 1e-3f) return 10.0f + x * (0.5f + x * (1.0f / 120.0f));
-    return __fdividef(x, 1.0f - __expf(x * -0.1f));
-}
-
-__device__ __forceinline__ IKf i_rhs_f(float v, float h, float w, float m3, float n4, float n, float m, float Ge, float Gi)
-{
-    typedef IConst K;
-    IKf k;
-    k.V = -(float)K::gL * (v - (float)K::El) - (float)K::gNa * h * m3 * (v - (float)K::Ena)
-          - ((float)K::gKdr * n4 + (float)K::gKHT * w) * (v - (float)K::Ek) - Ge * v - Gi * (v - (float)K::Ei);
-    k.n = 0.15f * i_vtrap(v + 15.0f) * (1.0f - n) - 0.2f * __expf((v + 25.0f) * (-1.0f / 80.0f)) * n;
-    k.m = i_vtrap(v + 22.0f) * (1.0f - m) - 40.0f * __expf((v + 47.0f) * (-1.0f / 18.0f)) * m;
-    k.h = 0.7f * __expf((v + 34.0f) * -0.05f) * (1.0f - h) - 10.0f * __fdividef(h, 1.0f + __expf((v + 4.0f) * -0.1f));
-    k.w = __fdividef(1.0f, 1.0f + __expf(v * -0.2f)) - w;
-    return k;
-}
-
-template <class R>
-__device__ __forceinline__ void i_dp8(IStateR<R>& s, const IStep<R>& p);
-
-template <>
-__device__ __forceinline__ void i_dp8<double>(IStateR<double>& s, const IStep<double>& p)
+__device__ __forceinline__ void i_dp8(IStateR<double>& s, const IStep<double>& p)
 {
     const DPT B7[] = {UG_DP_B7}, B8[] = {UG_DP_B8}, B9[] = {UG_DP_B9}, B10[] = {UG_DP_B10}, B11[] = {UG_DP_B11},
               B12[] = {UG_DP_B12}, BO[] = {UG_DP_OUT};
@@ -439,83 +319,14 @@ __device__ __forceinline__ void i_dp8<double>(IStateR<double>& s, const IStep<do
     s.Gi = s.Gi * p.gi[11];
 }
 
-template <>
-__device__ __forceinline__ void i_dp8<float>(IStateR<float>& s, const IStep<float>& p)
-{
-    // Same tableau; coefficients folded to num/den in float at compile time.
-    const DPT B7[] = {UG_DP_B7}, B8[] = {UG_DP_B8}, B9[] = {UG_DP_B9}, B10[] = {UG_DP_B10}, B11[] = {UG_DP_B11},
-              B12[] = {UG_DP_B12}, BO[] = {UG_DP_OUT};
-    const DPT* tb[6] = {B7, B8, B9, B10, B11, B12};
-    const int cnt[6] = {4, 5, 6, 7, 8, 9};
-    const int acount[5] = {1, 2, 2, 3, 3};
-    const int astage[5][3] = {{0, 0, 0}, {0, 1, 0}, {0, 2, 0}, {0, 2, 3}, {0, 3, 4}};
-    const double acoef[5][3] = {{1, 0, 0}, {1, 3, 0}, {1, 3, 0}, {20, -75, 75}, {3, 15, 12}};
-    const double aden[5] = {18, 48, 32, 64, 80};
-    const float dt = p.dt;
-    float kV[12], kn[12], km[12], kh[12], kw[12];
-#pragma unroll
-    for (int st = 0; st < 12; ++st) {
-        float v, n1, m1, h1, w1;
-        if (st == 0) {
-            v = s.V; n1 = s.n; m1 = s.m; h1 = s.h; w1 = s.w;
-        } else {
-            float sV = 0.f, sn = 0.f, sm = 0.f, sh = 0.f, sw = 0.f;
-            if (st <= 5) {
-                const int a = st - 1;
-#pragma unroll
-                for (int j = 0; j < 3; ++j) {
-                    if (j < acount[a]) {
-                        const int q = astage[a][j];
-                        const float c = (float)(acoef[a][j] / aden[a]);
-                        sV += c * kV[q]; sn += c * kn[q]; sm += c * km[q]; sh += c * kh[q]; sw += c * kw[q];
-                    }
-                }
-            } else {
-                const DPT* t = tb[st - 6];
-#pragma unroll
-                for (int j = 0; j < 9; ++j) {
-                    if (j < cnt[st - 6]) {
-                        const int q = t[j].s;
-                        const float c = (float)(t[j].num / t[j].den);
-                        sV += c * kV[q]; sn += c * kn[q]; sm += c * km[q]; sh += c * kh[q]; sw += c * kw[q];
-                    }
-                }
-            }
-            v = s.V + dt * sV;
-            n1 = s.n + dt * sn;
-            m1 = s.m + dt * sm;
-            h1 = s.h + dt * sh;
-            w1 = s.w + dt * sw;
-        }
-        const float n2 = n1 * n1;
-        const IKf k = i_rhs_f(v, h1, w1, m1 * m1 * m1, n2 * n2, n1, m1, s.Ge * p.ge[st], s.Gi * p.gi[st]);
-        kV[st] = k.V; kn[st] = k.n; km[st] = k.m; kh[st] = k.h; kw[st] = k.w;
-    }
-    float oV = 0.f, on = 0.f, om = 0.f, oh = 0.f, ow = 0.f;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const int q = BO[j].s;
-        const float c = (float)(BO[j].num / BO[j].den);
-        oV += c * kV[q]; on += c * kn[q]; om += c * km[q]; oh += c * kh[q]; ow += c * kw[q];
-    }
-    s.V = s.V + dt * oV;
-    s.n = s.n + dt * on;
-    s.m = s.m + dt * om;
-    s.h = s.h + dt * oh;
-    s.w = s.w + dt * ow;
-    s.Ge = s.Ge * p.ge[11];
-    s.Gi = s.Gi * p.gi[11];
-}
-
 // Interneuron spike detection (HHI_buffer::state_check, HHI_buffer.cpp:260-276).
-template <class R>
-__device__ __forceinline__ bool i_state_check(R V, int& flag)
+__device__ __forceinline__ bool i_state_check(double V, int& flag)
 {
-    if (flag == 1 && V < R(-25.0)) {
+    if (flag == 1 && V < -25.0) {
         flag = 0;
         return true;
     }
-    if (flag == 0 && V > R(-20.0)) flag = 1;
+    if (flag == 0 && V > -20.0) flag = 1;
     return false;
 }
 

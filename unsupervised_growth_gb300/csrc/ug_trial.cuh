@@ -211,26 +211,13 @@ __device__ __forceinline__ void scatter_warp(uint32_t bits, int src, int s0, con
     }
 }
 
-template <class R>
-__device__ __forceinline__ void load_ra_step(const NetDev<R>& n, RAStep<R>& p, int s);
-
-template <>
-__device__ __forceinline__ void load_ra_step<double>(const NetDev<double>& n, RAStep<double>& p, int s)
+__device__ __forceinline__ void load_ra_step(const NetDev<double>& n, RAStep<double>& p, int s)
 {
     p.e1 = n.ra_decay[2 * s];
     p.e2 = n.ra_decay[2 * s + 1];
 }
 
-template <>
-__device__ __forceinline__ void load_ra_step<float>(const NetDev<float>&, RAStep<float>&, int)
-{
-}
-
-template <class R>
-__device__ __forceinline__ void load_i_step(const NetDev<R>& n, IStep<R>& p, int s);
-
-template <>
-__device__ __forceinline__ void load_i_step<double>(const NetDev<double>& n, IStep<double>& p, int s)
+__device__ __forceinline__ void load_i_step(const NetDev<double>& n, IStep<double>& p, int s)
 {
     const double* d = n.i_decay + (size_t)24 * s;
 #pragma unroll
@@ -238,11 +225,6 @@ __device__ __forceinline__ void load_i_step<double>(const NetDev<double>& n, ISt
         p.ge[k] = d[k];
         p.gi[k] = d[12 + k];
     }
-}
-
-template <>
-__device__ __forceinline__ void load_i_step<float>(const NetDev<float>&, IStep<float>&, int)
-{
 }
 
 // Smallest step s >= s_from with T[s-1] > x (the step whose start time has
@@ -268,48 +250,20 @@ __device__ __forceinline__ int first_step_after(const double* T, int num_steps, 
 // HHI_buffer.cpp:278-294) at step st, whose start time has passed
 // noise_time: add the conductance kick(s), draw the next noise time, and
 // return the step at which it will be passed.  Kept out of line: it runs on
-// about 1% of neuron-steps and is the only double-precision arithmetic of
-// the single-precision integrator.
-static __device__ __noinline__ int i_noise_event_d(const double* T, int num_steps, int st, double& noise_time,
-                                                   double& G, const StreamId& sid, uint32_t& word)
+// about 1% of neuron-steps (double build; the single build draws its events beforehand).
+static __device__ __noinline__ int i_noise_event(const double* T, int num_steps, int st, double& noise_time, double& G,
+                                                 const StreamId& sid, uint32_t& word)
 {
     i_noise_check(T[st - 1], 0.02, G, noise_time, sid, word);
     return first_step_after(T, num_steps, noise_time, st + 1);
 }
 
-// single build: the kick is accumulated in float and the interval is
-// -4 log(1 - u/0xffffffff) (= 1000 * Exp(250 Hz) in ms), which rounds within an
+// single build: the noise interval is -4 log(1 - u/0xffffffff) (= 1000 * Exp(250 Hz) in ms), which rounds within an
 // ulp of the reference's form; noise times stay double, so the steps at
 // which noise arrives are the double build's.
 __device__ __forceinline__ double i_noise_interval_fast(uint32_t u)
 {
     return -4.0 * log(1.0 - (double)u * (1.0 / 4294967295.0));
-}
-
-static __device__ __noinline__ int i_noise_event_f(const double* T, int num_steps, int st, double& noise_time,
-                                                   float& G, const StreamId& sid, uint32_t& word)
-{
-    const float gscale = (float)(IConst::G_noise / 4294967295.0);
-    G += gscale * (float)stream_word(sid, word++);
-    double rnd = i_noise_interval_fast(stream_word(sid, word++));
-    while (rnd < 0.02) {
-        rnd = i_noise_interval_fast(stream_word(sid, word++));
-        G += gscale * (float)stream_word(sid, word++);
-    }
-    noise_time = noise_time + rnd;
-    return first_step_after(T, num_steps, noise_time, st + 1);
-}
-
-__device__ __forceinline__ int i_noise_event(const double* T, int num_steps, int st, double& noise_time, double& G,
-                                             const StreamId& sid, uint32_t& word)
-{
-    return i_noise_event_d(T, num_steps, st, noise_time, G, sid, word);
-}
-
-__device__ __forceinline__ int i_noise_event(const double* T, int num_steps, int st, double& noise_time, float& G,
-                                             const StreamId& sid, uint32_t& word)
-{
-    return i_noise_event_f(T, num_steps, st, noise_time, G, sid, word);
 }
 
 // Sets every neuron of every instance to the reference's rest state
