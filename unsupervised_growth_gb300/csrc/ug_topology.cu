@@ -540,10 +540,9 @@ __device__ inline bool connect(const Geo& g, const Gauss& q, float4 a32, float4 
 // A exp(-d^2 / 2 sigma^2) falls to 2^-(c + 1): one comparison of the closeness with near_[c]
 // leaves about twice the pairs that connect (some thousandths; the word alone left a tenth, at
 // least one lane of every warp), and a warp takes them up one per lane and round.
-// The block's eight rows share tiles of target coordinates in shared memory (a lane reads its
-// four targets as three vectors; the same loads from the L1 cache, 64 bytes apart, took more
-// cycles than the Philox rounds, which are what is left).  20 000 x 5000: 0.46 ms for both directions,
-// 1.0 ms with the word alone as the filter.
+// The block's eight rows share tiles of target coordinates in shared memory, which a lane reads
+// as three vectors of its four targets.  Bound by issue, the Philox rounds most of all.
+// 20 000 x 5000: 0.45 ms for both directions, 1.0 ms with the word alone as the filter.
 constexpr int kConnTile = 1024;
 __global__ void __launch_bounds__(kRowThreads) k_conn_decide(Geo g, Gauss q, const double* src, const float4* src32,
                                                              int n_src, const double* dst, const float4* dst32,
