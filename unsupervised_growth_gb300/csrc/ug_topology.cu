@@ -896,12 +896,14 @@ ug_status generate(ug_ctx* ctx, const ug_topology_params& p, int n_ra, int n_i, 
             return terr(UG_EINVAL, "HVC(RA) placement gave up after " + std::to_string(a0 - h.last_kept) +
                                        " attempts in a row too close to a placed neuron (no room at the minimum "
                                        "intersomatic distance)");
-        // next batch: the attempts still needed at the last batch's keep rate, with a margin, and
+        // next batch: twice the attempts still needed at the last batch's keep rate, which falls as
+        // the points fill up (a quarter more took 4 or 5 batches for 2000 to 20 000 neurons, twice
+        // takes 2 or 3; a batch is four launches and a synchronisation: 577 -> 470 us at 2000), and
         // about kmax attempts left open by the points already placed
         const double rate = std::max((double)h.kept / K, 1.0 / 64);
         const double open = std::max((double)h.unflagged / K, 1.0 / 64);
         const int limit = std::min(kMaxBatch, std::max(kMinBatch, round_up((long long)(kmax / open), kMinBatch)));
-        K = std::min(limit, std::max(kMinBatch, round_up((long long)((n_ra - h.count) / rate * 1.25) + 1, kMinBatch)));
+        K = std::min(limit, std::max(kMinBatch, round_up((long long)((n_ra - h.count) / rate * 2) + 1, kMinBatch)));
     }
     t.ra_attempts = h.attempts;
     t.i_retries = h.retries;
