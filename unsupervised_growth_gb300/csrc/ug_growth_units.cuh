@@ -30,20 +30,31 @@
 
 namespace ug {
 
-// Counters of the launch, each in a 128-byte line of its own, zero at the launch.  Those with
-// a step of kCtlParity are apart for even and odd intervals: warps of one interval may be
-// through with it before others have read the counts of the one before.
+// Counters of the launch, zero at the launch: words of the launch, each in a 128-byte line of
+// its own, and words of every interval, in an array per kind.  A role that no other waits for
+// may be any number of intervals behind the HVC(RA) warps: the first sync block, while they
+// integrate intervals without rows; a row block that has had no row for some time.  An
+// interval's words never change once it is complete, so such a role reads in them what the
+// others read, and takes no later interval's arrivals or rows for those of its own.
 enum GrowthCtl {
-    kCtlRA = 0,         // [parity] HVC(RA) arrivals << 32 | rows queued
-    kCtlI = 32,         // [parity] HVC(I) arrivals
-    kCtlDone = 64,      // [parity] rows delivered
-    kCtlPos = 96,       // [parity] queue positions handed out
-    kCtlPosted = 128,   // intervals whose post events are in place << 32 | those that had any;
+    kCtlPos = 0,        // queue positions handed out
+    kCtlPosted = 16,    // intervals whose post events are in place << 32 | those that had any;
                         // the word after it: the last of those that had any
-    kCtlLtp = 144,      // sync block arrivals, one each per interval that had post events
-    kGrowthCtlWords = 160,
-    kCtlParity = 16
+    kCtlLtp = 32,       // sync block arrivals, one each per interval that had post events
+    kCtlIntervals = 48  // the intervals' words: kCtlKinds arrays of ctl_stride(Q)
 };
+enum GrowthCtlKind {
+    kCtlRA,             // HVC(RA) arrivals << 32 | rows queued
+    kCtlI,              // HVC(I) arrivals
+    kCtlDone,           // rows delivered
+    kCtlKinds
+};
+// An array's words: 16 columns of whole 128-byte lines, consecutive intervals in different
+// columns, so that one interval's arrivals do not meet the polls of the one before.
+__host__ __device__ constexpr int ctl_column(int Q) { return (Q + 255) / 256 * 16; }
+__host__ __device__ constexpr int ctl_stride(int Q) { return 16 * ctl_column(Q); }
+// Words of a trial of Q sync intervals.
+__host__ __device__ constexpr size_t growth_ctl_words(int Q) { return kCtlIntervals + (size_t)kCtlKinds * ctl_stride(Q); }
 constexpr int kSyncBlocks = 16, kRowBlocks = 64;              // at most
 constexpr int kEnoughRowBlocks = 32, kMinRowBlocks = 8;       // rather than wider roles; at least
 
@@ -54,15 +65,17 @@ struct UnitsLoop {
     int ra_per, i_per;     // of them per block
     int nb_ra, nb_i, nb_sync, nb_row;
     unsigned long long* ctl;
-    int2* rows;            // [parity][rows_cap] rings of queued rows: (row, somatic spike bits)
+    // Ring of queued rows (row, somatic spike bits).  An interval's rows lie behind those of all
+    // earlier ones, as many as their words say; those of the last interval with rows may still
+    // be read (by the first sync block) while the next one's are queued, but no third one's:
+    // rows are delivered once every earlier sync is closed, and the HVC(RA) warps wait for that.
+    int2* rows;
     int rows_cap;          // at least two intervals' rows
-    __device__ __forceinline__ unsigned long long* at(int word, int q) const { return ctl + word + kCtlParity * (q & 1); }
-    // arrivals of `units` warps up to interval q on its parity's counter
-    static __device__ __forceinline__ unsigned arrivals(int q, int units) { return (unsigned)(q / 2 + 1) * (unsigned)units; }
-    __device__ __forceinline__ int2& row(int q, unsigned pos) const
+    __device__ __forceinline__ unsigned long long* at(GrowthCtlKind kind, int q) const
     {
-        return rows[(size_t)(q & 1) * rows_cap + pos % (unsigned)rows_cap];
+        return ctl + kCtlIntervals + kind * ctl_stride(Q) + (q & 15) * ctl_column(Q) + (q >> 4);
     }
+    __device__ __forceinline__ int2& row(unsigned pos) const { return rows[pos % (unsigned)rows_cap]; }
 };
 
 __device__ __forceinline__ unsigned long long load_acquire64(const unsigned long long* p)
@@ -103,7 +116,7 @@ __device__ __forceinline__ bool ra_wait(const UnitsLoop& L, int q, int* error)
 {
     const int lane = threadIdx.x & 31;
     const unsigned long long* p = L.at(lane == 0 ? kCtlRA : lane == 1 ? kCtlI : kCtlDone, q);
-    const unsigned want = UnitsLoop::arrivals(q, lane == 0 ? L.ra_units : L.i_units);
+    const unsigned want = (unsigned)(lane == 0 ? L.ra_units : L.i_units);
     const bool ok = poll_bounded(0xffffffffu, error, [&] {
         const unsigned long long v = lane < 3 ? load_acquire64(p) : 0ull;
         const unsigned queued = (unsigned)__shfl_sync(0xffffffffu, v, 0);
@@ -148,9 +161,9 @@ __device__ __forceinline__ void units_ra(const NetDev<float>& n, const BatchDev<
             const unsigned m = __ballot_sync(0xffffffffu, row);
             if (m) {
                 unsigned pos = 0;
-                if (lane == 0) pos = (unsigned)atomicAdd(L.at(kCtlPos, q), (unsigned long long)__popc(m));
+                if (lane == 0) pos = (unsigned)atomicAdd(L.ctl + kCtlPos, (unsigned long long)__popc(m));
                 pos = __shfl_sync(0xffffffffu, pos, 0) + __popc(m & ((1u << lane) - 1u));
-                if (row) L.row(q, pos) = make_int2(i0 + k, (int)soma[k]);
+                if (row) L.row(pos) = make_int2(i0 + k, (int)soma[k]);
                 queued += __popc(m);
             }
         }
@@ -174,7 +187,7 @@ __device__ __forceinline__ void units_i(const NetDev<float>& n, const BatchDev<f
     int s0 = 1;
     for (int q = 0; q <= L.Q; ++q) {
         if (q > 0) {
-            const unsigned want = UnitsLoop::arrivals(q - 1, L.ra_units);
+            const unsigned want = (unsigned)L.ra_units;
             const bool ok = poll_bounded(0xffffffffu, bt.error, [&] {
                 return lane != 0 || (unsigned)(load_acquire64(L.at(kCtlRA, q - 1)) >> 32) >= want;
             });
@@ -214,24 +227,23 @@ __device__ __forceinline__ void units_rows(const GrowthDev& g, const NetDev<floa
     __shared__ unsigned s_queued;
     __shared__ int s_ok;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    unsigned queued_to[2] = {0, 0};   // rows queued up to the last interval of each parity
+    unsigned before = 0;   // rows queued in the intervals before q
     for (int q = 0; q < L.Q; ++q) {
         const int s0 = q == 0 ? 1 : L.sync_end[q - 1] + 1, s1 = L.sync_end[q];
         double* T = sh_T[q & 1];
         g_stage_times(T, n.T, s0, s1);
-        const unsigned before = (q & 1) ? queued_to[1] : queued_to[0];
         // The interval's rows are known once the HVC(RA) warps are through with it; if this block
         // has any, sync q - 1 must be closed: its post events, and where it had any, every
         // row's LTP.  One lane of the first warp polls each.
         if (w == 0) {
-            const unsigned want = UnitsLoop::arrivals(q, L.ra_units);
+            const unsigned want = (unsigned)L.ra_units;
             const unsigned long long* p = lane == 0 ? L.at(kCtlRA, q) : L.ctl + (lane == 1 ? kCtlPosted : kCtlLtp);
             unsigned queued = 0;
             const bool ok = poll_bounded(0xffffffffu, g.error, [&] {
                 const unsigned long long v = lane < 3 ? load_acquire64(p) : 0ull;
                 queued = (unsigned)__shfl_sync(0xffffffffu, v, 0);
                 const unsigned posts = (unsigned)__shfl_sync(0xffffffffu, v, 1);
-                const bool here = (unsigned)k < queued - before;
+                const bool here = (unsigned)k < queued;
                 return lane == 0   ? (unsigned)(v >> 32) >= want
                        : lane == 1 ? !here || (unsigned)(v >> 32) >= (unsigned)q
                        : lane == 2 ? !here || v >= (unsigned long long)posts * L.nb_sync
@@ -244,14 +256,14 @@ __device__ __forceinline__ void units_rows(const GrowthDev& g, const NetDev<floa
         }
         __syncthreads();
         if (!s_ok) return;
-        const unsigned queued = s_queued, count = queued - before;
+        const unsigned count = s_queued;
         __syncthreads();   // the next interval's wait may write s_queued
         if ((unsigned)k < count) {
             // row e of the interval: block e % nb_row, so that rows spread over the SMs first
             RowStreams st;
             int head = 0, num = 0, row = -1;
             for (unsigned e = (unsigned)(k + w * L.nb_row); e < count; e += (unsigned)(L.nb_row * kTrialWarps)) {
-                const int2 r = L.row(q, before + e);
+                const int2 r = L.row(before + e);
                 row = r.x;
                 g_row(g, n, bt, (uint32_t)r.y, 0, row, s0, s1, T, row_smem[w], lane, head, num, st);
                 __syncwarp();
@@ -263,8 +275,7 @@ __device__ __forceinline__ void units_rows(const GrowthDev& g, const NetDev<floa
             }
             if (row >= 0) g_row_prefetch(g, 0, row, head, num, st, lane);
         }
-        if (q & 1) queued_to[1] = queued;
-        else queued_to[0] = queued;
+        before += count;
     }
 }
 
@@ -280,20 +291,20 @@ __device__ __forceinline__ void units_ltp(const GrowthDev& g, const NetDev<float
 __device__ __forceinline__ void units_newpost(const GrowthDev& g, const NetDev<float>& n, const UnitsLoop& L)
 {
     __shared__ unsigned s_queued;
-    unsigned queued_to[2] = {0, 0}, posts = 0;
+    unsigned before = 0, posts = 0;   // rows queued in the intervals before q; those that had post events
     for (int q = 0; q < L.Q; ++q) {
         const int s0 = q == 0 ? 1 : L.sync_end[q - 1] + 1, s1 = L.sync_end[q];
-        const unsigned want = UnitsLoop::arrivals(q, L.ra_units);
+        const unsigned want = (unsigned)L.ra_units;
         if (!block_wait(g.error, [&] {
                 const unsigned long long v = load_acquire64(L.at(kCtlRA, q));
                 s_queued = (unsigned)v;
                 return (unsigned)(v >> 32) >= want && (unsigned)load_acquire64(L.at(kCtlDone, q)) >= (unsigned)v;
             }))
             return;
-        const unsigned queued = s_queued, before = (q & 1) ? queued_to[1] : queued_to[0];
+        const unsigned count = s_queued;
         int K = 0;
-        if (queued != before) {
-            K = g_newpost_rows(g, n, queued - before, [&](unsigned e) { return L.row(q, before + e); }, s0, s1);
+        if (count) {
+            K = g_newpost_rows(g, n, count, [&](unsigned e) { return L.row(before + e); }, s0, s1);
             __syncthreads();
         }
         if (K > 0) ++posts;
@@ -302,8 +313,7 @@ __device__ __forceinline__ void units_newpost(const GrowthDev& g, const NetDev<f
             store_release64(L.ctl + kCtlPosted, ((unsigned long long)(q + 1) << 32) + posts);
         }
         if (K > 0) units_ltp(g, n, L, 0, s1);
-        if (q & 1) queued_to[1] = queued;
-        else queued_to[0] = queued;
+        before += count;
     }
 }
 

@@ -1048,7 +1048,7 @@ ug_status NetImpl<R>::growth_init(cudaStream_t st)
     UG_TRY(gLoop_.alloc(ug::kLoopWords * sizeof(int)));
     if (!hloop_) UG_CUDA(cudaMallocHost(&hloop_, ug::kLoopWords * sizeof(int)));
     // the one-launch trial: barrier and queue words, the row queue
-    UG_TRY(gTrialCtl_.alloc(ug::kGrowthCtlWords * sizeof(unsigned long long)));
+    UG_TRY(gTrialCtl_.alloc(ug::growth_ctl_words((int)sync_steps.size()) * sizeof(unsigned long long)));
     UG_TRY(gActRows_.alloc(4 * (size_t)n * sizeof(int2)));
     trial_plan_ = ug::GrowthPlan();
     trial_key_ = -1;

@@ -380,7 +380,7 @@ cudaError_t launch_growth_trial(const GrowthDev& g, const NetDev<R>& n, BatchDev
                                 const IStep<R>& ic, const GrowthPlan& plan, const int* sync_end, int Q,
                                 unsigned long long* ctl, int2* act_rows, cudaStream_t st)
 {
-    cudaError_t e = cudaMemsetAsync(ctl, 0, kGrowthCtlWords * sizeof(unsigned long long), st);
+    cudaError_t e = cudaMemsetAsync(ctl, 0, growth_ctl_words(Q) * sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
     b.member = 0;
     b.live_streams = g.st_num;

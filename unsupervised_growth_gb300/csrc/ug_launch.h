@@ -173,7 +173,7 @@ struct GrowthPlan {
 // The grid for a network and a request of role widths (0: the default).
 template <class R>
 cudaError_t growth_trial_plan(int n_ra, int n_i, int req_ra, int req_i, GrowthPlan* plan);
-// ctl: kGrowthCtlWords 64-bit words, cleared here; act_rows: room for 4 n_ra queued rows.
+// ctl: growth_ctl_words(Q) 64-bit words, cleared here; act_rows: room for 4 n_ra queued rows.
 template <class R>
 cudaError_t launch_growth_trial(const GrowthDev& g, const NetDev<R>& n, BatchDev<R> b, const RAStep<R>& rc,
                                 const IStep<R>& ic, const GrowthPlan& plan, const int* sync_end, int Q,
