@@ -157,8 +157,9 @@ ug_status ug_set_group_launch(ug_ctx* ctx, int32_t ra_blocks_per_sm, int32_t i_b
  * one_launch 1 (the default): each trial's intervals run in one cooperative kernel, with
  * bounded grid barriers between phases (double build) or bounded waits of each role on what
  * it reads (single build), when the network's blocks can all be resident at
- * once (else, and in the double build while recording traces or inhibition, the
- * per-interval launches run);
+ * once (else, for networks of more than 8000 HVC(RA) neurons in the single build, and in the
+ * double build while recording traces or inhibition, the per-interval launches run: they are
+ * the faster ones for a large network);
  * a barrier or wait not satisfied within about a second ends the trial with UG_ETIMEOUT.
  * 0: the per-interval launches (several kernels per sync interval).  Results are the
  * same bits either way. */

@@ -24,27 +24,9 @@
 // sets kErrTimeout, every block leaves, and the host reports UG_ETIMEOUT.
 #pragma once
 #include "ug_growth.cuh"
+#include "ug_plan.h"
 
 namespace ug {
-
-constexpr int kTrialThreads = 256;
-constexpr int kTrialWarps = kTrialThreads / 32;
-
-// Threads per block of the integrating roles (whole warps, at most kTrialThreads): by default
-// one integrating warp per block, so that a trial spreads over as many SMs as it has
-// integrating warps; wider roles put several integrating warps on one SM scheduler.
-constexpr int kRoleThreads = 32;
-
-// The role widths of a request (0: the default); false unless each is a multiple of 32
-// in [32, kTrialThreads].
-__host__ __device__ inline bool trial_widths(int req_ra, int req_i, int* ra_w, int* i_w)
-{
-    *ra_w = req_ra ? req_ra : kRoleThreads;
-    *i_w = req_i ? req_i : kRoleThreads;
-    for (int w : {*ra_w, *i_w})
-        if (w < 32 || w > kTrialThreads || w % 32) return false;
-    return true;
-}
 
 struct TrialLoop {
     const int* sync_end;   // [Q] last step of each sync interval

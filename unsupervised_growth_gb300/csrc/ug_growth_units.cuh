@@ -55,15 +55,9 @@ __host__ __device__ constexpr int ctl_column(int Q) { return (Q + 255) / 256 * 1
 __host__ __device__ constexpr int ctl_stride(int Q) { return 16 * ctl_column(Q); }
 // Words of a trial of Q sync intervals.
 __host__ __device__ constexpr size_t growth_ctl_words(int Q) { return kCtlIntervals + (size_t)kCtlKinds * ctl_stride(Q); }
-constexpr int kSyncBlocks = 16, kRowBlocks = 64;              // at most
-constexpr int kEnoughRowBlocks = 32, kMinRowBlocks = 8;       // rather than wider roles; at least
-
-struct UnitsLoop {
+struct UnitsLoop : UnitsShape {
     const int* sync_end;   // [Q] last step of each sync interval
     int Q;                 // sync intervals before the trailing one
-    int ra_units, i_units; // warps of the two integrating roles
-    int ra_per, i_per;     // of them per block
-    int nb_ra, nb_i, nb_sync, nb_row;
     unsigned long long* ctl;
     // Ring of queued rows (row, somatic spike bits).  An interval's rows lie behind those of all
     // earlier ones, as many as their words say; those of the last interval with rows may still

@@ -323,8 +323,6 @@ inline cudaError_t units_attributes(const void* kernel)
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrialSmem);
 }
 
-// Single build: one HVC(RA) neuron per thread where the roles fit the SMs, a block each, else
-// two.  The rows take what the other roles leave, up to kRowBlocks blocks.
 template <class R>
 cudaError_t growth_trial_plan(int n_ra, int n_i, int req_ra, int req_i, GrowthPlan* plan)
 {
@@ -336,28 +334,13 @@ cudaError_t growth_trial_plan(int n_ra, int n_i, int req_ra, int req_i, GrowthPl
     int ra_w = 0, i_w = 0;
     if (e != cudaSuccess || !coop || !trial_widths(req_ra, req_i, &ra_w, &i_w)) return e;
     if constexpr (sizeof(R) == 4) {
-        for (int lanes = 1; lanes <= 2 && plan->blocks == 0; ++lanes) {
-            for (const void* f : {lanes == 1 ? (const void*)k_growth_units<float, false> : (const void*)k_growth_units<f2, false>,
-                                  lanes == 1 ? (const void*)k_growth_units<float, true> : (const void*)k_growth_units<f2, true>}) {
-                e = units_attributes(f);
-                if (e != cudaSuccess) return e;
-            }
-            // by default as few warps to a block as leave the rows enough blocks
-            for (int per = 1; per <= kTrialWarps && plan->blocks == 0; per *= 2) {
-                UnitsLoop u{};
-                u.ra_units = (n_ra + 32 * lanes - 1) / (32 * lanes);
-                u.i_units = (n_i + 31) / 32;
-                u.ra_per = req_ra ? ra_w / 32 : per;
-                u.i_per = req_i ? i_w / 32 : per;
-                u.nb_ra = (u.ra_units + u.ra_per - 1) / u.ra_per;
-                u.nb_i = (u.i_units + u.i_per - 1) / u.i_per;
-                u.nb_sync = std::min(kSyncBlocks, (n_ra + kTrialThreads - 1) / kTrialThreads);
-                u.nb_row = std::min(kRowBlocks, sms - u.nb_ra - u.nb_i - u.nb_sync);
-                if (u.nb_row < (per < kTrialWarps ? kEnoughRowBlocks : kMinRowBlocks)) continue;
-                plan->lanes = lanes;
-                plan->units = u;
-                plan->blocks = u.nb_ra + u.nb_i + u.nb_sync + u.nb_row;
-            }
+        plan->units = units_shape(n_ra, n_i, req_ra, req_i, sms);
+        plan->blocks = plan->units.blocks();
+        const bool one = plan->units.lanes == 1;
+        for (const void* f : {one ? (const void*)k_growth_units<float, false> : (const void*)k_growth_units<f2, false>,
+                              one ? (const void*)k_growth_units<float, true> : (const void*)k_growth_units<f2, true>}) {
+            e = units_attributes(f);
+            if (e != cudaSuccess) return e;
         }
         return cudaSuccess;
     } else {
@@ -396,7 +379,8 @@ cudaError_t launch_growth_trial(const GrowthDev& g, const NetDev<R>& n, BatchDev
     cfg.attrs = at;
     cfg.numAttrs = 1;
     if constexpr (sizeof(R) == 4) {
-        UnitsLoop L = plan.units;
+        UnitsLoop L;
+        static_cast<UnitsShape&>(L) = plan.units;
         L.sync_end = sync_end;
         L.Q = Q;
         L.ctl = ctl;
@@ -404,9 +388,9 @@ cudaError_t launch_growth_trial(const GrowthDev& g, const NetDev<R>& n, BatchDev
         L.rows_cap = 2 * n.n_ra;
         b.soma_bits = nullptr;   // the spike bits travel with the queued rows
         if (b.trace_ra || b.trace_i || b.ginh_slot)
-            return plan.lanes == 1 ? cudaLaunchKernelEx(&cfg, k_growth_units<float, true>, g, n, b, rc, ic, L)
+            return L.lanes == 1 ? cudaLaunchKernelEx(&cfg, k_growth_units<float, true>, g, n, b, rc, ic, L)
                                    : cudaLaunchKernelEx(&cfg, k_growth_units<f2, true>, g, n, b, rc, ic, L);
-        return plan.lanes == 1 ? cudaLaunchKernelEx(&cfg, k_growth_units<float, false>, g, n, b, rc, ic, L)
+        return L.lanes == 1 ? cudaLaunchKernelEx(&cfg, k_growth_units<float, false>, g, n, b, rc, ic, L)
                                : cudaLaunchKernelEx(&cfg, k_growth_units<f2, false>, g, n, b, rc, ic, L);
     } else {
         TrialLoop L = plan.trial;

@@ -165,10 +165,9 @@ cudaError_t launch_growth_epilogue(const GrowthDev& g, const LaunchCtx& lc);
 // The one-launch growth trial (ug_growth_trial.cuh): its grid for a network (0 when the
 // blocks cannot all be resident at once), and the cooperative launch.
 struct GrowthPlan {
-    int blocks = 0;   // 0: the network's blocks cannot all be resident, per-interval launches
-    int lanes = 1;    // single build: HVC(RA) neurons per thread
+    int blocks = 0;   // 0: per-interval launches (the blocks cannot all be resident, or those are faster)
     TrialLoop trial{};   // double build (k_growth_trial)
-    UnitsLoop units{};   // single build (k_growth_units)
+    UnitsShape units;    // single build (k_growth_units)
 };
 // The grid for a network and a request of role widths (0: the default).
 template <class R>
