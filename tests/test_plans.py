@@ -10,9 +10,10 @@ CSRC = ROOT / "unsupervised_growth_gb300" / "csrc"
 
 SOURCE = r"""
 #include "ug_plan.h"
-extern "C" int shape(int n_ra, int n_i, int req_ra, int req_i, int sms, int* out)
+extern "C" int shape(int n_ra, int n_i, int req_ra, int req_i, int sms, int resident, int* out)
 {
-    const ug::UnitsShape u = ug::units_shape(n_ra, n_i, req_ra, req_i, sms);
+    const bool fits[2] = {(resident & 1) != 0, (resident & 2) != 0};
+    const ug::UnitsShape u = ug::units_shape(n_ra, n_i, req_ra, req_i, sms, fits);
     if (!u.lanes) return 0;
     const int v[] = {u.lanes, u.ra_units, u.i_units, u.ra_per, u.i_per, u.nb_ra, u.nb_i, u.nb_sync, u.nb_row};
     for (int k = 0; k < 9; ++k) out[k] = v[k];
@@ -30,9 +31,9 @@ def plans(tmp_path_factory):
     return ctypes.CDLL(str(d / "plans.so"))
 
 
-def units_shape(plans, n_ra, n_i, req=(0, 0), sms=152):
+def units_shape(plans, n_ra, n_i, req=(0, 0), sms=152, resident=3):
     out = (ctypes.c_int * 9)()
-    blocks = plans.shape(n_ra, n_i, *req, sms, out)
+    blocks = plans.shape(n_ra, n_i, *req, sms, resident, out)
     names = ("lanes", "ra_units", "i_units", "ra_per", "i_per", "nb_ra", "nb_i", "nb_sync", "nb_row")
     return blocks, dict(zip(names, out)) if blocks else {}
 
@@ -62,3 +63,11 @@ def test_requested_widths(plans):
     assert units_shape(plans, 3600, 40, (32, 32))[1]["lanes"] == 1
     assert units_shape(plans, 4200, 40, (32, 32))[1]["lanes"] == 2   # 132 blocks with one neuron per thread
     assert units_shape(plans, 8000, 8000, (32, 32))[0] == 0        # no blocks left for the rows
+
+
+@pytest.mark.parametrize("n_ra", [33, 2000, 8000])
+def test_a_kernel_no_sm_can_hold_is_not_planned(plans, n_ra):
+    """resident: bit 0 the form with one HVC(RA) neuron per thread, bit 1 the one with two."""
+    assert units_shape(plans, n_ra, 40, resident=0)[0] == 0
+    assert units_shape(plans, n_ra, 40, resident=1)[1]["lanes"] == 1
+    assert units_shape(plans, n_ra, 40, resident=2)[1]["lanes"] == 2

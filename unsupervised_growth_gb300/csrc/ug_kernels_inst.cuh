@@ -323,6 +323,18 @@ inline cudaError_t units_attributes(const void* kernel)
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrialSmem);
 }
 
+// Whether an SM takes a block of `kernel`, a form of k_growth_units (its shared memory is most
+// of an SM's); a device that refuses the size is no error, the per-interval launches run.
+template <class K>
+bool units_resident(K kernel)
+{
+    int per_sm = 0;
+    cudaError_t e = units_attributes((const void*)kernel);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kTrialThreads, kTrialSmem);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e == cudaSuccess && per_sm > 0;
+}
+
 template <class R>
 cudaError_t growth_trial_plan(int n_ra, int n_i, int req_ra, int req_i, GrowthPlan* plan)
 {
@@ -334,14 +346,10 @@ cudaError_t growth_trial_plan(int n_ra, int n_i, int req_ra, int req_i, GrowthPl
     int ra_w = 0, i_w = 0;
     if (e != cudaSuccess || !coop || !trial_widths(req_ra, req_i, &ra_w, &i_w)) return e;
     if constexpr (sizeof(R) == 4) {
-        plan->units = units_shape(n_ra, n_i, req_ra, req_i, sms);
+        const bool resident[2] = {units_resident(k_growth_units<float, false>) && units_resident(k_growth_units<float, true>),
+                                  units_resident(k_growth_units<f2, false>) && units_resident(k_growth_units<f2, true>)};
+        plan->units = units_shape(n_ra, n_i, req_ra, req_i, sms, resident);
         plan->blocks = plan->units.blocks();
-        const bool one = plan->units.lanes == 1;
-        for (const void* f : {one ? (const void*)k_growth_units<float, false> : (const void*)k_growth_units<f2, false>,
-                              one ? (const void*)k_growth_units<float, true> : (const void*)k_growth_units<f2, true>}) {
-            e = units_attributes(f);
-            if (e != cudaSuccess) return e;
-        }
         return cudaSuccess;
     } else {
         e = units_attributes((const void*)k_growth_trial<R>);

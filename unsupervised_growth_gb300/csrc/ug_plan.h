@@ -43,13 +43,15 @@ constexpr int kEnoughRowBlocks = 32, kMinRowBlocks = 8;       // rather than wid
 constexpr int kUnitsMaxRA = 8000;
 
 // One HVC(RA) neuron per thread where the roles fit the SMs, a block each, else two.  The rows
-// take what the other roles leave, up to kRowBlocks blocks.  req_ra, req_i as trial_widths.
-inline UnitsShape units_shape(int n_ra, int n_i, int req_ra, int req_i, int sms)
+// take what the other roles leave, up to kRowBlocks blocks.  req_ra, req_i as trial_widths;
+// resident: whether an SM takes a block of the kernel with one, with two neurons per thread.
+inline UnitsShape units_shape(int n_ra, int n_i, int req_ra, int req_i, int sms, const bool (&resident)[2])
 {
     UnitsShape none;
     int ra_w = 0, i_w = 0;
     if (n_ra > kUnitsMaxRA || !trial_widths(req_ra, req_i, &ra_w, &i_w)) return none;
     for (int lanes = 1; lanes <= 2; ++lanes) {
+        if (!resident[lanes - 1]) continue;
         // by default as few warps to a block as leave the rows enough blocks
         for (int per = 1; per <= kTrialWarps; per *= 2) {
             UnitsShape u;
