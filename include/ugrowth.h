@@ -451,12 +451,16 @@ ug_status ug_create_network_topology(ug_ctx* ctx, const char* config_file, const
 ug_status ug_calibrate_pipes(int32_t device, double* mufu_ops_per_s, double* fma_ops_per_s);
 
 /* No counterpart in the reference (failure detection).  Every wait in the library's kernels
- * (on an mbarrier of the bulk copy engine, on a flag in global memory, or at a grid barrier
- * of the one-launch growth trial) gives up after one second and raises UG_ETIMEOUT instead
- * of hanging the device.  This runs one such wait that nothing can satisfy -- which 0: a
+ * (on an mbarrier of the bulk copy engine, on a flag in global memory, at a grid barrier of
+ * the double build's one-launch growth trial, or for the arrivals of other roles in the
+ * single build's one-launch trials) gives up after one second and raises UG_ETIMEOUT instead
+ * of hanging the device; the single build's growth trial, after one second in which its
+ * deliveries did not advance.  This runs one such wait that nothing can satisfy -- which 0: a
  * global flag nothing sets; which 1: an mbarrier expecting bytes no copy delivers; which 2:
- * a grid barrier of a two-block cooperative launch that the blocks never reach -- and
- * returns UG_ETIMEOUT once it gives up; the device stays usable. */
+ * a grid barrier of a two-block cooperative launch that the blocks never reach; which 3: an
+ * arrival nothing makes; which 5: the same, with work beside it that stops advancing -- and
+ * returns UG_ETIMEOUT once it gives up; the device stays usable.  which 4: an arrival made
+ * after 1.6 s of advancing work, which returns UG_OK. */
 ug_status ug_probe_bounded_wait(int32_t device, int32_t which);
 
 #ifdef __cplusplus

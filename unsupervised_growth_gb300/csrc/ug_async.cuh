@@ -136,6 +136,38 @@ __device__ __forceinline__ bool block_wait_geq(const unsigned* word, unsigned va
     return s_ok != 0;
 }
 
+// Bounded polling by the calling thread(s) of `mask`: ready() until it holds for all of them;
+// false, with `timeout_bit` set in *error, once nothing has happened for kWaitNs or another
+// wait of the launch has given up.  beat (or null): a word that the launch's work advances
+// (advance_beat) wherever a piece of it may take long, so that a wait for much work is not
+// taken for one that nothing will satisfy.
+template <class F>
+__device__ __forceinline__ bool poll_bounded(unsigned mask, int* error, int timeout_bit, const unsigned long long* beat,
+                                             F&& ready)
+{
+    uint64_t t0 = 0;
+    unsigned long long seen = 0;
+    for (unsigned k = 0;; ++k) {
+        if (__all_sync(mask, ready())) return true;
+        if ((k & 255u) == 255u) {   // now and then: the time, progress, and whether another warp gave up
+            const uint64_t t = globaltimer_ns();
+            const unsigned long long b = beat ? *(const volatile unsigned long long*)beat : 0ull;
+            if (t0 == 0 || b != seen) {
+                t0 = t;
+                seen = b;
+            }
+            if (__any_sync(mask, t - t0 > kWaitNs || (*(volatile int*)error & timeout_bit))) {
+                atomicOr(error, timeout_bit);
+                return false;
+            }
+        }
+    }
+}
+__device__ __forceinline__ void advance_beat(unsigned long long* beat)
+{
+    asm volatile("red.relaxed.gpu.global.add.u64 [%0], 1;" ::"l"(beat) : "memory");
+}
+
 // Grid-wide barrier of a cooperative launch.  `count` counts arrivals; barrier k of the
 // launch is passed once it reaches k * gridDim.x.  Each block's writes are fenced before
 // its arrival and read after the wait, so everything written before the barrier is seen

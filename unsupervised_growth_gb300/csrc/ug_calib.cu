@@ -56,7 +56,10 @@ __global__ void k_fma_loop(float* out, int iters, float seed)
 // a global flag nothing sets; which 1 waits on an mbarrier that expects 16 bytes of
 // transactions no copy delivers; which 2 is the grid barrier of the one-launch growth
 // trial (a cooperative launch of two blocks) waiting for its second barrier, which the
-// blocks never reach.  error[0] gets 8 (the timeout flag) once it gives up.
+// blocks never reach; which 3 polls (poll_bounded, the wait of the one-launch trials' roles)
+// for a flag nothing sets; which 4 and 5 poll beside a block that advances the wait's beat:
+// for 1.6 s, then sets the flag (4: the wait holds out), or for 0.3 s and no flag (5).
+// error[0] gets 8 (the timeout flag) once a wait gives up.
 __global__ void k_wait_probe(int which, int* flag, int* error)
 {
     __shared__ uint64_t bar;
@@ -66,6 +69,20 @@ __global__ void k_wait_probe(int which, int* flag, int* error)
     } else if (which == 2) {
         // one arrival per block, but the wait is for the second barrier (2 x 2 arrivals)
         ok = ug::grid_barrier_bounded(reinterpret_cast<unsigned*>(flag), 2u, error, 8);
+    } else if (which >= 3) {
+        unsigned long long* beat = reinterpret_cast<unsigned long long*>(flag + 2);
+        ok = true;
+        if (which > 3 && blockIdx.x == 0) {
+            const uint64_t t0 = ug::globaltimer_ns(), until = which == 4 ? 1600000000ull : 300000000ull;
+            while (threadIdx.x == 0 && ug::globaltimer_ns() - t0 < until) {
+                ug::advance_beat(beat);
+                __nanosleep(100000);
+            }
+            if (threadIdx.x == 0 && which == 4) atomicExch(flag, 1);
+        } else if (threadIdx.x < 32) {
+            ok = ug::poll_bounded(0xffffffffu, error, 8, which > 3 ? beat : nullptr,
+                                  [&] { return *(volatile int*)flag != 0; });
+        }
     } else {
         if (threadIdx.x == 0) {
             ug::mbar_init(&bar, 1);
@@ -82,14 +99,14 @@ __global__ void k_wait_probe(int which, int* flag, int* error)
 
 extern "C" ug_status ug_probe_bounded_wait(int32_t device, int32_t which)
 {
-    if (which < 0 || which > 2) return UG_EINVAL;
+    if (which < 0 || which > 5) return UG_EINVAL;
     if (cudaSetDevice(device) != cudaSuccess) return UG_ECUDA;
     int* buf = nullptr;
-    if (cudaMalloc(&buf, 2 * sizeof(int)) != cudaSuccess) return UG_ENOMEM;
+    if (cudaMalloc(&buf, 4 * sizeof(int)) != cudaSuccess) return UG_ENOMEM;
     int host[2] = {0, 0};
-    cudaError_t e = cudaMemset(buf, 0, 2 * sizeof(int));
+    cudaError_t e = cudaMemset(buf, 0, 4 * sizeof(int));
     if (e == cudaSuccess) {
-        if (which == 2) {
+        if (which == 2 || which >= 4) {
             int coop = 0;
             e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
             if (e == cudaSuccess && !coop) e = cudaErrorNotSupported;
@@ -99,7 +116,7 @@ extern "C" ug_status ug_probe_bounded_wait(int32_t device, int32_t which)
             void* args[] = {&w, &f, &err};
             if (e == cudaSuccess) e = cudaLaunchCooperativeKernel((const void*)k_wait_probe, dim3(2), dim3(64), args, 0, 0);
         } else {
-            k_wait_probe<<<1, 32>>>(which, buf, buf + 1);
+            k_wait_probe<<<1, 32>>>(which, buf, buf + 1);   // a 64-bit word of beats behind the two
         }
         if (e == cudaSuccess) e = cudaDeviceSynchronize();
     }

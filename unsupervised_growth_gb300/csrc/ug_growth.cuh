@@ -87,6 +87,7 @@ struct GrowthDev {
     int* newpost_cnt;       // [B]
     int* error;
     int epi_blocks;         // blocks of the bulk-copy epilogue (0: the warp epilogue)
+    unsigned long long* beat = nullptr;   // advanced by deliveries that change a row (poll_bounded); or null
 };
 
 __device__ __forceinline__ size_t gidx(const GrowthDev& g, int b, int i, int j)
@@ -709,7 +710,10 @@ __device__ __forceinline__ void g_process(const GrowthDev& g, const NetDev<R>& n
                 const int x = __shfl_sync(0xffffffffu, v[k].sd, lf);
                 if (k == kf) sdf = x;
             }
-            if (lane == 0) g_deliver(g, n, bt, b, i, sh.tgt[buf][base + f], sdf, sh.spk[buf][base + f], sh.td[buf][base + f]);
+            if (lane == 0) {
+                g_deliver(g, n, bt, b, i, sh.tgt[buf][base + f], sdf, sh.spk[buf][base + f], sh.td[buf][base + f]);
+                if (g.beat) advance_beat(g.beat);
+            }
             __syncwarp();
             base += f + 1;
         } else {

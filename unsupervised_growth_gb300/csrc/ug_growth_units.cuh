@@ -23,7 +23,11 @@
 // give the same bits.
 //
 // Every wait is bounded (ug_async.cuh): one that gives up sets kErrTimeout, every block leaves
-// at its next wait, and the host reports UG_ETIMEOUT.
+// at its next wait, and the host reports UG_ETIMEOUT.  An interval's deliveries can take a
+// second and more (18 000 HVC(RA), 200 training neurons, fast synapses), so a wait gives up
+// when the interval's work has not advanced for a second: a warp that takes up a further row
+// or has delivered an event that changed its row, and a sync block that takes up further rows,
+// say so.
 #pragma once
 #include "ug_growth_trial.cuh"
 #include "ug_test_trial.cuh"
@@ -41,7 +45,8 @@ enum GrowthCtl {
     kCtlPosted = 16,    // intervals whose post events are in place << 32 | those that had any;
                         // the word after it: the last of those that had any
     kCtlLtp = 32,       // sync block arrivals, one each per interval that had post events
-    kCtlIntervals = 48  // the intervals' words: kCtlKinds arrays of ctl_stride(Q)
+    kCtlBeat = 48,      // advances while an interval's rows or LTP take long (poll_bounded)
+    kCtlIntervals = 64  // the intervals' words: kCtlKinds arrays of ctl_stride(Q)
 };
 enum GrowthCtlKind {
     kCtlRA,             // HVC(RA) arrivals << 32 | rows queued
@@ -87,31 +92,13 @@ __device__ __forceinline__ void store_release64(unsigned long long* p, unsigned 
     asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-// Bounded polling by the calling thread(s): ready() until it holds for the whole mask.
-template <class F>
-__device__ __forceinline__ bool poll_bounded(unsigned mask, int* error, F&& ready)
-{
-    uint64_t t0 = 0;
-    for (unsigned k = 0;; ++k) {
-        if (__all_sync(mask, ready())) return true;
-        if ((k & 255u) == 255u) {   // now and then: the time, and whether another warp gave up
-            const uint64_t t = globaltimer_ns();
-            if (t0 == 0) t0 = t;
-            if (__any_sync(mask, t - t0 > kWaitNs || (*(volatile int*)error & kErrTimeout))) {
-                atomicOr(error, kErrTimeout);
-                return false;
-            }
-        }
-    }
-}
-
 // An HVC(RA) warp after interval q: all warps' interval q, and the deliveries of its rows.
 __device__ __forceinline__ bool ra_wait(const UnitsLoop& L, int q, int* error)
 {
     const int lane = threadIdx.x & 31;
     const unsigned long long* p = L.at(lane == 0 ? kCtlRA : lane == 1 ? kCtlI : kCtlDone, q);
     const unsigned want = (unsigned)(lane == 0 ? L.ra_units : L.i_units);
-    const bool ok = poll_bounded(0xffffffffu, error, [&] {
+    const bool ok = poll_bounded(0xffffffffu, error, kErrTimeout, L.ctl + kCtlBeat, [&] {
         const unsigned long long v = lane < 3 ? load_acquire64(p) : 0ull;
         const unsigned queued = (unsigned)__shfl_sync(0xffffffffu, v, 0);
         return lane == 0 ? (unsigned)(v >> 32) >= want : lane == 1 ? (unsigned)v >= want
@@ -182,7 +169,7 @@ __device__ __forceinline__ void units_i(const NetDev<float>& n, const BatchDev<f
     for (int q = 0; q <= L.Q; ++q) {
         if (q > 0) {
             const unsigned want = (unsigned)L.ra_units;
-            const bool ok = poll_bounded(0xffffffffu, bt.error, [&] {
+            const bool ok = poll_bounded(0xffffffffu, bt.error, kErrTimeout, L.ctl + kCtlBeat, [&] {
                 return lane != 0 || (unsigned)(load_acquire64(L.at(kCtlRA, q - 1)) >> 32) >= want;
             });
             if (!ok) return;
@@ -205,11 +192,11 @@ __device__ __forceinline__ void units_i(const NetDev<float>& n, const BatchDev<f
 
 // Thread 0 waits (ready returns whether it is done, and may leave values in sh), then the block.
 template <class F>
-__device__ __forceinline__ bool block_wait(int* error, F&& ready)
+__device__ __forceinline__ bool block_wait(const UnitsLoop& L, int* error, F&& ready)
 {
     __shared__ int s_ok;
     __syncthreads();
-    if (threadIdx.x == 0) s_ok = poll_bounded(1u, error, ready) ? 1 : 0;
+    if (threadIdx.x == 0) s_ok = poll_bounded(1u, error, kErrTimeout, L.ctl + kCtlBeat, ready) ? 1 : 0;
     __syncthreads();
     return s_ok != 0;
 }
@@ -233,7 +220,7 @@ __device__ __forceinline__ void units_rows(const GrowthDev& g, const NetDev<floa
             const unsigned want = (unsigned)L.ra_units;
             const unsigned long long* p = lane == 0 ? L.at(kCtlRA, q) : L.ctl + (lane == 1 ? kCtlPosted : kCtlLtp);
             unsigned queued = 0;
-            const bool ok = poll_bounded(0xffffffffu, g.error, [&] {
+            const bool ok = poll_bounded(0xffffffffu, g.error, kErrTimeout, L.ctl + kCtlBeat, [&] {
                 const unsigned long long v = lane < 3 ? load_acquire64(p) : 0ull;
                 queued = (unsigned)__shfl_sync(0xffffffffu, v, 0);
                 const unsigned posts = (unsigned)__shfl_sync(0xffffffffu, v, 1);
@@ -257,6 +244,7 @@ __device__ __forceinline__ void units_rows(const GrowthDev& g, const NetDev<floa
             RowStreams st;
             int head = 0, num = 0, row = -1;
             for (unsigned e = (unsigned)(k + w * L.nb_row); e < count; e += (unsigned)(L.nb_row * kTrialWarps)) {
+                if (row >= 0 && lane == 0) advance_beat(L.ctl + kCtlBeat);   // the warp's last row is done
                 const int2 r = L.row(before + e);
                 row = r.x;
                 g_row(g, n, bt, (uint32_t)r.y, 0, row, s0, s1, T, row_smem[w], lane, head, num, st);
@@ -276,7 +264,10 @@ __device__ __forceinline__ void units_rows(const GrowthDev& g, const NetDev<floa
 // LTP, LTD and remodeling of this sync block's share of the rows, at the sync of step s1.
 __device__ __forceinline__ void units_ltp(const GrowthDev& g, const NetDev<float>& n, const UnitsLoop& L, int k, int s1)
 {
-    for (int bx = k; bx * kTrialThreads < g.n; bx += L.nb_sync) g_ltp_body(g, n, s1, 2 * bx, 0);   // rows 256 bx ..
+    for (int bx = k; bx * kTrialThreads < g.n; bx += L.nb_sync) {
+        if (bx != k && threadIdx.x == 0) advance_beat(L.ctl + kCtlBeat);
+        g_ltp_body(g, n, s1, 2 * bx, 0);   // rows 256 bx ..
+    }
     __syncthreads();
     if (threadIdx.x == 0) add_release64(L.ctl + kCtlLtp, 1ull);
 }
@@ -289,7 +280,7 @@ __device__ __forceinline__ void units_newpost(const GrowthDev& g, const NetDev<f
     for (int q = 0; q < L.Q; ++q) {
         const int s0 = q == 0 ? 1 : L.sync_end[q - 1] + 1, s1 = L.sync_end[q];
         const unsigned want = (unsigned)L.ra_units;
-        if (!block_wait(g.error, [&] {
+        if (!block_wait(L, g.error, [&] {
                 const unsigned long long v = load_acquire64(L.at(kCtlRA, q));
                 s_queued = (unsigned)v;
                 return (unsigned)(v >> 32) >= want && (unsigned)load_acquire64(L.at(kCtlDone, q)) >= (unsigned)v;
@@ -320,7 +311,7 @@ __device__ __forceinline__ void units_sync(const GrowthDev& g, const NetDev<floa
     __shared__ int s_q;
     unsigned closed = 0, posts = 0;
     while (closed < (unsigned)L.Q) {
-        if (!block_wait(g.error, [&] {
+        if (!block_wait(L, g.error, [&] {
                 s_posted = load_acquire64(L.ctl + kCtlPosted);
                 s_q = (int)*(volatile unsigned long long*)(L.ctl + kCtlPosted + 1);
                 return (unsigned)(s_posted >> 32) > closed;

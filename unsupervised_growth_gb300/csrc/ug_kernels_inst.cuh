@@ -395,11 +395,13 @@ cudaError_t launch_growth_trial(const GrowthDev& g, const NetDev<R>& n, BatchDev
         L.rows = act_rows;
         L.rows_cap = 2 * n.n_ra;
         b.soma_bits = nullptr;   // the spike bits travel with the queued rows
+        GrowthDev gb = g;
+        gb.beat = ctl + kCtlBeat;
         if (b.trace_ra || b.trace_i || b.ginh_slot)
-            return L.lanes == 1 ? cudaLaunchKernelEx(&cfg, k_growth_units<float, true>, g, n, b, rc, ic, L)
-                                   : cudaLaunchKernelEx(&cfg, k_growth_units<f2, true>, g, n, b, rc, ic, L);
-        return L.lanes == 1 ? cudaLaunchKernelEx(&cfg, k_growth_units<float, false>, g, n, b, rc, ic, L)
-                               : cudaLaunchKernelEx(&cfg, k_growth_units<f2, false>, g, n, b, rc, ic, L);
+            return L.lanes == 1 ? cudaLaunchKernelEx(&cfg, k_growth_units<float, true>, gb, n, b, rc, ic, L)
+                                   : cudaLaunchKernelEx(&cfg, k_growth_units<f2, true>, gb, n, b, rc, ic, L);
+        return L.lanes == 1 ? cudaLaunchKernelEx(&cfg, k_growth_units<float, false>, gb, n, b, rc, ic, L)
+                               : cudaLaunchKernelEx(&cfg, k_growth_units<f2, false>, gb, n, b, rc, ic, L);
     } else {
         TrialLoop L = plan.trial;
         L.sync_end = sync_end;

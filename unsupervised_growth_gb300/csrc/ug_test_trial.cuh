@@ -66,22 +66,10 @@ __device__ __forceinline__ bool unit_wait(const unsigned* count, unsigned want0,
     const int lane = threadIdx.x & 31;
     const unsigned want = lane == 0 ? want0 : lane == 1 ? want1 : 0u;
     const unsigned* p = lane == 1 ? inter : count;
-    uint64_t t0 = 0;
-    for (unsigned k = 0;; ++k) {
-        const bool here = want == 0u || load_acquire(p) >= want;
-        if (__all_sync(0xffffffffu, here)) break;
-        if ((k & 255u) == 255u) {   // now and then: the time, and whether another warp gave up
-            const uint64_t t = globaltimer_ns();
-            if (t0 == 0) t0 = t;
-            const bool out = t - t0 > kWaitNs || (*(volatile int*)error & kErrTimeout);
-            if (__any_sync(0xffffffffu, out)) {
-                if (lane == 0) atomicOr(error, kErrTimeout);
-                return false;
-            }
-        }
-    }
+    const bool ok = poll_bounded(0xffffffffu, error, kErrTimeout, nullptr,
+                                 [&] { return want == 0u || load_acquire(p) >= want; });
     __syncwarp();
-    return true;
+    return ok;
 }
 
 // V: the lane type of the HVC(RA) warps (ug_ra_f32.cuh).

@@ -643,8 +643,10 @@ def calibrate_pipes(device: int = 0):
 
 
 def probe_bounded_wait(device: int = 0, which: int = 0) -> str:
-    """Runs a device wait that nothing can satisfy (0: a global flag, 1: an mbarrier) and
-    returns the status name it ends with (UG_ETIMEOUT once the bounded wait gives up)."""
+    """Runs a device wait that nothing can satisfy (0: a global flag, 1: an mbarrier, 2: a grid
+    barrier, 3: an arrival, 5: an arrival beside work that stops advancing) and returns the
+    status name it ends with (UG_ETIMEOUT once the bounded wait gives up); 4: an arrival after
+    1.6 s of advancing work, UG_OK."""
     L = load_library()
     return UG_STATUS.get(L.ug_probe_bounded_wait(device, which), "unknown")
 
