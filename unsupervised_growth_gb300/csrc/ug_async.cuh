@@ -136,31 +136,47 @@ __device__ __forceinline__ bool block_wait_geq(const unsigned* word, unsigned va
     return s_ok != 0;
 }
 
+struct PollState {
+    uint64_t t0;
+    unsigned long long seen;
+};
+// Whether a wait goes on: its time, its beat, and whether another wait gave up.
+__device__ __forceinline__ bool poll_on(unsigned mask, int* error, int timeout_bit, const unsigned long long* beat,
+                                            PollState& p)
+{
+    const uint64_t t = globaltimer_ns();
+    const unsigned long long b = beat ? *(const volatile unsigned long long*)beat : 0ull;
+    if (p.t0 == 0 || b != p.seen) {
+        p.t0 = t;
+        p.seen = b;
+    }
+    if (!__any_sync(mask, t - p.t0 > kWaitNs || (*(volatile int*)error & timeout_bit))) return true;
+    atomicOr(error, timeout_bit);
+    return false;
+}
+static __device__ __noinline__ bool poll_on_call(unsigned mask, int* error, int timeout_bit, const unsigned long long* beat,
+                                                 PollState& p)
+{
+    return poll_on(mask, error, timeout_bit, beat, p);
+}
+
 // Bounded polling by the calling thread(s) of `mask`: ready() until it holds for all of them;
 // false, with `timeout_bit` set in *error, once nothing has happened for kWaitNs or another
 // wait of the launch has given up.  beat (or null): a word that the launch's work advances
 // (advance_beat) wherever a piece of it may take long, so that a wait for much work is not
-// taken for one that nothing will satisfy.
-template <class F>
+// taken for one that nothing will satisfy.  kCall: poll_on out of line.  Inlined, it cost the
+// waits of a 300 / 100 growth trial 1 %; out of line, the registers of the test trial with two
+// neurons per thread (at most 128) 1 %.
+template <bool kCall, class F>
 __device__ __forceinline__ bool poll_bounded(unsigned mask, int* error, int timeout_bit, const unsigned long long* beat,
                                              F&& ready)
 {
-    uint64_t t0 = 0;
-    unsigned long long seen = 0;
+    PollState p = {0, 0};
     for (unsigned k = 0;; ++k) {
         if (__all_sync(mask, ready())) return true;
-        if ((k & 255u) == 255u) {   // now and then: the time, progress, and whether another warp gave up
-            const uint64_t t = globaltimer_ns();
-            const unsigned long long b = beat ? *(const volatile unsigned long long*)beat : 0ull;
-            if (t0 == 0 || b != seen) {
-                t0 = t;
-                seen = b;
-            }
-            if (__any_sync(mask, t - t0 > kWaitNs || (*(volatile int*)error & timeout_bit))) {
-                atomicOr(error, timeout_bit);
-                return false;
-            }
-        }
+        if ((k & 255u) != 255u) continue;
+        if (!(kCall ? poll_on_call(mask, error, timeout_bit, beat, p) : poll_on(mask, error, timeout_bit, beat, p)))
+            return false;
     }
 }
 __device__ __forceinline__ void advance_beat(unsigned long long* beat)

@@ -80,7 +80,7 @@ __global__ void k_wait_probe(int which, int* flag, int* error)
             }
             if (threadIdx.x == 0 && which == 4) atomicExch(flag, 1);
         } else if (threadIdx.x < 32) {
-            ok = ug::poll_bounded(0xffffffffu, error, 8, which > 3 ? beat : nullptr,
+            ok = ug::poll_bounded<true>(0xffffffffu, error, 8, which > 3 ? beat : nullptr,
                                   [&] { return *(volatile int*)flag != 0; });
         }
     } else {

@@ -98,7 +98,7 @@ __device__ __forceinline__ bool ra_wait(const UnitsLoop& L, int q, int* error)
     const int lane = threadIdx.x & 31;
     const unsigned long long* p = L.at(lane == 0 ? kCtlRA : lane == 1 ? kCtlI : kCtlDone, q);
     const unsigned want = (unsigned)(lane == 0 ? L.ra_units : L.i_units);
-    const bool ok = poll_bounded(0xffffffffu, error, kErrTimeout, L.ctl + kCtlBeat, [&] {
+    const bool ok = poll_bounded<true>(0xffffffffu, error, kErrTimeout, L.ctl + kCtlBeat, [&] {
         const unsigned long long v = lane < 3 ? load_acquire64(p) : 0ull;
         const unsigned queued = (unsigned)__shfl_sync(0xffffffffu, v, 0);
         return lane == 0 ? (unsigned)(v >> 32) >= want : lane == 1 ? (unsigned)v >= want
@@ -169,7 +169,7 @@ __device__ __forceinline__ void units_i(const NetDev<float>& n, const BatchDev<f
     for (int q = 0; q <= L.Q; ++q) {
         if (q > 0) {
             const unsigned want = (unsigned)L.ra_units;
-            const bool ok = poll_bounded(0xffffffffu, bt.error, kErrTimeout, L.ctl + kCtlBeat, [&] {
+            const bool ok = poll_bounded<true>(0xffffffffu, bt.error, kErrTimeout, L.ctl + kCtlBeat, [&] {
                 return lane != 0 || (unsigned)(load_acquire64(L.at(kCtlRA, q - 1)) >> 32) >= want;
             });
             if (!ok) return;
@@ -196,7 +196,7 @@ __device__ __forceinline__ bool block_wait(const UnitsLoop& L, int* error, F&& r
 {
     __shared__ int s_ok;
     __syncthreads();
-    if (threadIdx.x == 0) s_ok = poll_bounded(1u, error, kErrTimeout, L.ctl + kCtlBeat, ready) ? 1 : 0;
+    if (threadIdx.x == 0) s_ok = poll_bounded<true>(1u, error, kErrTimeout, L.ctl + kCtlBeat, ready) ? 1 : 0;
     __syncthreads();
     return s_ok != 0;
 }
@@ -220,7 +220,7 @@ __device__ __forceinline__ void units_rows(const GrowthDev& g, const NetDev<floa
             const unsigned want = (unsigned)L.ra_units;
             const unsigned long long* p = lane == 0 ? L.at(kCtlRA, q) : L.ctl + (lane == 1 ? kCtlPosted : kCtlLtp);
             unsigned queued = 0;
-            const bool ok = poll_bounded(0xffffffffu, g.error, kErrTimeout, L.ctl + kCtlBeat, [&] {
+            const bool ok = poll_bounded<true>(0xffffffffu, g.error, kErrTimeout, L.ctl + kCtlBeat, [&] {
                 const unsigned long long v = lane < 3 ? load_acquire64(p) : 0ull;
                 queued = (unsigned)__shfl_sync(0xffffffffu, v, 0);
                 const unsigned posts = (unsigned)__shfl_sync(0xffffffffu, v, 1);

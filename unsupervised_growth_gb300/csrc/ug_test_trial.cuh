@@ -66,7 +66,7 @@ __device__ __forceinline__ bool unit_wait(const unsigned* count, unsigned want0,
     const int lane = threadIdx.x & 31;
     const unsigned want = lane == 0 ? want0 : lane == 1 ? want1 : 0u;
     const unsigned* p = lane == 1 ? inter : count;
-    const bool ok = poll_bounded(0xffffffffu, error, kErrTimeout, nullptr,
+    const bool ok = poll_bounded<false>(0xffffffffu, error, kErrTimeout, nullptr,
                                  [&] { return want == 0u || load_acquire(p) >= want; });
     __syncwarp();
     return ok;
