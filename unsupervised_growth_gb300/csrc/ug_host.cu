@@ -298,18 +298,6 @@ private:
     ug::TestPlan test_plan_;
     static constexpr int kSegmentBatch = 15;
     bool segmented() const { return bd_.B <= kSegmentBatch && sync_steps.size() >= 64; }
-    // Where the noise pre-pass keeps its intervals: in the inhibitory channel's list memory,
-    // or, for lists drawn in segments, in an array of their own.
-    void share_gaps()
-    {
-        bd_.i_gaps = reinterpret_cast<double*>(bd_.i_events + bd_.ev_cap);
-        bd_.gap_stride = 2 * bd_.ev_cap;
-    }
-    void own_gaps()
-    {
-        bd_.i_gaps = i_gaps_.as<double>();
-        bd_.gap_stride = bd_.ev_cap;
-    }
     ug_status plan_batch(const ug::LaunchCtx& lc)
     {
         test_plan_ = ug::TestPlan();
@@ -688,7 +676,10 @@ ug_status NetImpl<R>::ensure_batch(int B)
     for (int k = 0; k < 7; ++k) b.iv[k] = iv_[k].as<R>();
     b.i_noise = i_noise_.as<double>(); b.i_noise_step = i_noise_step_.as<int>();
     b.i_events = i_events_.as<int2>(); b.i_ev_idx = i_ev_idx_.as<int>(); b.ev_cap = ev_cap;
-    share_gaps();
+    // the noise pre-pass keeps its intervals in the inhibitory channel's list memory (lists drawn
+    // in segments: issue_test_trial)
+    b.i_gaps = reinterpret_cast<double*>(b.i_events + ev_cap);
+    b.gap_stride = 2 * ev_cap;
     b.i_ev_cnt = i_ev_cnt_.as<int>();
     b.i_word = i_word_.as<uint32_t>(); b.i_flag = i_flag_.as<int>();
     b.i_nspk = i_nspk_.as<int>(); b.i_first = i_first_.as<int>();
@@ -715,18 +706,21 @@ ug_status NetImpl<R>::issue_test_trial(const ug::LaunchCtx& lc)
         UG_CUDA(ug::launch_test_trial<R>(nd_, bd_, rc_, ic_, test_plan_, ends, Q, 0, Q + 1, ctl, lc.main));
         return UG_OK;
     }
-    own_gaps();
+    // lists drawn in segments keep their intervals in an array of their own, which holds those of
+    // kSegmentBatch instances: a copy, so that no other batch's launches find it in bd_
+    ug::BatchDev<R> bs = bd_;
+    bs.i_gaps = i_gaps_.as<double>();
+    bs.gap_stride = bd_.ev_cap;
     const int qa = Q / 16;                                             // a sixteenth of the trial first,
     const int ka = std::min((bd_.ev_cap / 4 + 63) / 64 * 64, bd_.ev_cap / 2 * 2);   // a quarter of the intervals
-    UG_CUDA(ug::launch_noise_segment<R>(nd_, bd_, sync_steps[qa - 1], 0, ka, lc.main));
+    UG_CUDA(ug::launch_noise_segment<R>(nd_, bs, sync_steps[qa - 1], 0, ka, lc.main));
     UG_CUDA(cudaEventRecord(lc.fork, lc.main));
     UG_CUDA(cudaStreamWaitEvent(lc.side, lc.fork, 0));
-    UG_CUDA(ug::launch_noise_segment<R>(nd_, bd_, h.num_steps - 1, ka, bd_.ev_cap, lc.side));
+    UG_CUDA(ug::launch_noise_segment<R>(nd_, bs, h.num_steps - 1, ka, bs.ev_cap, lc.side));
     UG_CUDA(cudaEventRecord(lc.join, lc.side));
     UG_CUDA(ug::launch_test_trial<R>(nd_, bd_, rc_, ic_, test_plan_, ends, Q, 0, qa, ctl, lc.main));
     UG_CUDA(cudaStreamWaitEvent(lc.main, lc.join, 0));
     UG_CUDA(ug::launch_test_trial<R>(nd_, bd_, rc_, ic_, test_plan_, ends, Q, qa, Q + 1, ctl, lc.main));
-    share_gaps();
     return UG_OK;
 }
 
