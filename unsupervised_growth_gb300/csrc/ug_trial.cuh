@@ -19,6 +19,7 @@
 // the atomic adds: results are deterministic run to run.
 #pragma once
 #include <stdint.h>
+#include "ug_hd.h"
 #include "ug_neuron.cuh"
 #include "ug_ra_f32.cuh"
 #include "ug_i_f32.cuh"
@@ -742,8 +743,8 @@ __device__ __forceinline__ void noise_events_body(const NetDev<R>& n, const Batc
     uint32_t word = bt.i_word[x];
     double nt[2] = {bt.i_noise[2 * x], bt.i_noise[2 * x + 1]};
     int ns[2] = {bt.i_noise_step[2 * x], bt.i_noise_step[2 * x + 1]};
-    // a resumed list goes on behind the mark its last segment ended with
-    int cnt[2] = {resume ? bt.i_ev_cnt[2 * x] + 1 : 0, resume ? bt.i_ev_cnt[2 * x + 1] + 1 : 0};
+    int cnt[2] = {list_start(resume, resume ? bt.i_ev_cnt[2 * x] : 0, bt.ev_cap),
+                  list_start(resume, resume ? bt.i_ev_cnt[2 * x + 1] : 0, bt.ev_cap)};
     int2* out[2] = {bt.i_events + (x * 2) * bt.ev_cap, bt.i_events + (x * 2 + 1) * bt.ev_cap};
     const double* gaps = bt.i_gaps + x * bt.gap_stride;
     const float gscale = (float)(IConst::G_noise / 4294967295.0);
@@ -823,7 +824,7 @@ struct IEvents {
     __device__ __forceinline__ IEvents(const BatchDev<R>& bt, size_t x, int ch, bool resumed)
         : ev(bt.i_events + (x * 2 + ch) * bt.ev_cap), idx(bt.i_ev_idx[2 * x + ch])
     {
-        if (resumed) ++idx;
+        if (resumed) idx = list_start(true, idx, bt.ev_cap);
         cur = ev[idx];
         after = cur;
         if (cur.x < kEvSegmentEnd) after = ev[idx + 1];
