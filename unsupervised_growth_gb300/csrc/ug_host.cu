@@ -292,17 +292,17 @@ private:
         const int64_t per = ug::fused_interval<R>(nd_, bd_, lc) ? 1 : (h.n_i > 0 ? 2 : 1);
         return per * ((int64_t)sync_steps.size() + 1) + 1 + noise;
     }
-    // The one-launch form of the current batch.  Small batches integrate a first part of the
-    // trial while the noise of the rest is drawn beside it (they leave SMs idle); larger ones
-    // gain nothing from that.
+    // The one-launch form of the captured graph's batch, or of the one being issued.  Small
+    // batches integrate a first part of the trial while the noise of the rest is drawn beside it
+    // (they leave SMs idle); larger ones gain nothing from that.
     ug::TestPlan test_plan_;
     static constexpr int kSegmentBatch = 15;
     bool segmented() const { return bd_.B <= kSegmentBatch && sync_steps.size() >= 64; }
-    ug_status plan_batch(const ug::LaunchCtx& lc)
+    ug_status plan_batch(const ug::LaunchCtx& lc, ug::TestPlan* plan)
     {
-        test_plan_ = ug::TestPlan();
+        *plan = ug::TestPlan();
         if (sizeof(R) == 4 && lc.fuse && !lc.timer && !bd_.trace_ra && !bd_.trace_i && !sync_steps.empty())
-            UG_CUDA(ug::test_trial_plan<R>(h.n_ra, h.n_i, bd_.B, &test_plan_));
+            UG_CUDA(ug::test_trial_plan<R>(h.n_ra, h.n_i, bd_.B, plan));
         return UG_OK;
     }
     ug_status issue_test_trial(const ug::LaunchCtx& lc);
@@ -751,10 +751,12 @@ ug_status NetImpl<R>::run_test_trials(uint32_t first_trial, int n_trials, const 
 {
     cudaStream_t st = lc.main;
     UG_TRY(prepare_test(first_trial, n_trials, st));
-    if (!graph_exec_ || graph_B_ != n_trials || graph_fuse_ != lc.fuse || !graphs || lc.timer) UG_TRY(plan_batch(lc));
     if (!graphs || lc.timer) {
+        ug::TestPlan plan;   // of this call; test_plan_ stays that of the captured graph
+        UG_TRY(plan_batch(lc, &plan));
+        std::swap(plan, test_plan_);
         const ug_status s = issue_batch(lc, launches);
-        graph_B_ = -1;   // the plan in force is this call's, not a captured graph's
+        std::swap(plan, test_plan_);
         return s;
     }
     if (!graph_exec_ || graph_B_ != n_trials || graph_fuse_ != lc.fuse) {
@@ -762,6 +764,7 @@ ug_status NetImpl<R>::run_test_trials(uint32_t first_trial, int n_trials, const 
             cudaGraphExecDestroy(graph_exec_);
             graph_exec_ = nullptr;
         }
+        UG_TRY(plan_batch(lc, &test_plan_));
         cudaStream_t cap;
         UG_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
         cudaGraph_t g;
