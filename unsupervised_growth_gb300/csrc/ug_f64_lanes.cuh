@@ -8,7 +8,7 @@
 // Here lane c of a group of eight holds component c of a neuron: each component's stage sums,
 // each exponential and each rate's quotient is the same instruction on another lane, and the
 // terms of the membrane equations meet in shuffles.  Divisions by a fixed divisor take three
-// operations (div_known).  About 410 and 900 operations a step are left: 602 HVC(RA) and 150
+// operations (div_known, ug_hd.h).  About 410 and 900 operations a step are left: 602 HVC(RA) and 150
 // HVC(I) neurons, both kernels of one interval, 2.40 -> 0.41 ms.
 //
 // Every value is rounded as in the general bodies, operation by operation (this unit is
@@ -20,26 +20,6 @@ namespace ug {
 
 constexpr int kLanes = 8;           // lanes of a neuron
 constexpr int kLaneNeurons = 32 / kLanes;
-
-static __device__ __noinline__ double div_rare(double x, double d) { return x / d; }
-
-// x / d correctly rounded, z = RN(1/d), for a d > 0 whose odd part D is below 2^50 (Markstein's
-// division by a known divisor: one correction of x z by its remainder).  q is within 1.5 ulp of
-// x / d, its remainder r is exact (a multiple of D's unit below 1.5 D), and q + r z is off by at
-// most 1.5 2^-53 ulp before the last rounding, while x / d is at least 1 / (2 D) ulp away from
-// the middle of two doubles.  Quotients near the ends of the range, infinities and NaN take the
-// division; zeros keep their sign.
-__device__ __forceinline__ double div_known(double x, double d, double z)
-{
-    const double q = x * z;
-    double a = __fma_rn(__fma_rn(-d, q, x), z, q);
-    const unsigned e = ((unsigned)__double2hiint(q) >> 20) & 0x7ffu;
-    if (e - 0x80u >= 0x770u) {
-        const bool zero = (((unsigned)__double2hiint(x) << 1) | (unsigned)__double2loint(x)) == 0;
-        a = zero ? x : div_rare(x, d);
-    }
-    return a;
-}
 
 __device__ __forceinline__ double pick8(int c, double a0, double a1, double a2, double a3, double a4, double a5,
                                         double a6, double a7)
