@@ -120,10 +120,10 @@ def tune_growth_trial(engine, run_trial, sig: str | None = None, cache_path: str
     """Chooses the block shape of the one-launch growth trial for `run_trial` (a callable
     that runs the caller's next growth trial(s) through `engine` and returns when done).
 
-    A single network's trial is a chain of sync intervals separated by grid barriers, so
-    its time is the latency of the slowest block per interval: how many integrating warps
-    share an SM scheduler decides it, not occupancy.  Because an interval waits for the
-    slower of the two roles, narrowing one role alone can show no gain; so the search
+    A single network's trial is a chain of sync intervals in which each role waits for what
+    it reads (in the double build at grid barriers), so its time is the latency of the
+    slowest warps per interval: how many integrating warps share an SM scheduler decides it,
+    not occupancy.  Because an interval waits for the slower of the two roles, narrowing one role alone can show no gain; so the search
     first tries equal widths for both roles, then refines the HVC(RA) width and then the
     HVC(I) width from the best of those, keeping each faster shape.  With a cached entry
     for `sig` the shape is applied without timing.  The results are the same bits for

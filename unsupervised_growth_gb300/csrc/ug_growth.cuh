@@ -33,7 +33,6 @@ constexpr int kPreRing = 4;       // pre-synaptic events kept per pair
 constexpr int kPostRing = 8;      // post-synaptic events kept per neuron
 constexpr int kMaxStreams = 32;   // live delivery streams per row
 constexpr int kMaxNss = 16;       // largest supported Nss
-constexpr int kStreamOpen = 0;
 
 struct SynParams {
     int Nss;

@@ -2895,7 +2895,7 @@ extern "C" ug_status ug_run_test_trial_noalloc(ug_ctx* ctx, int32_t net_id, uint
     UG_TRY(noalloc_scratch(ctx->device, &base));
 
     const int nra = nd.n_ra, ni = nd.n_i;
-    const int ev_cap = (int)(nd.num_steps * 0.02 * 0.25 * 2.0) + 64;   // noise events per channel, as the batched path
+    const int ev_cap = (int)(nd.num_steps * 0.02 * 0.25 * 2.0) + 64;   // noise events per channel, as ensure_batch (no segments: no second mark)
     const int spk_cap = 16 * (2 * nra + ni);
     Carve c{base};
     ug::BatchDev<float> b{};
@@ -2921,7 +2921,7 @@ extern "C" ug_status ug_run_test_trial_noalloc(ug_ctx* ctx, int32_t net_id, uint
     b.i_events = c.take<int2>(2 * (size_t)ni * ev_cap);
     b.i_ev_idx = c.take<int>(2 * (size_t)ni);
     b.ev_cap = ev_cap;
-    b.i_gaps = reinterpret_cast<double*>(b.i_events + ev_cap);   // as the batched path
+    b.i_gaps = reinterpret_cast<double*>(b.i_events + ev_cap);   // as ensure_batch
     b.gap_stride = 2 * ev_cap;
     b.i_word = c.take<uint32_t>(ni);
     b.i_flag = c.take<int>(ni);

@@ -407,7 +407,7 @@ __device__ __forceinline__ void interval_ra_body(const NetDev<R>& n, const Batch
 }
 
 template <class R, bool kTrack = false>
-__global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 8 : 1) k_interval_ra(NetDev<R> n, BatchDev<R> bt, int q, int s0, int s1,
+__global__ void __launch_bounds__(kBlock, 1) k_interval_ra(NetDev<R> n, BatchDev<R> bt, int q, int s0, int s1,
                                                                                RAStep<R> rc)
 {
     interval_ra_body<R, kTrack>(n, bt, q, s0, s1, rc, (int)blockIdx.x, (int)blockIdx.y);
@@ -1010,7 +1010,7 @@ __device__ __forceinline__ void interval_i_body(const NetDev<R>& n, const BatchD
 }
 
 template <class R, bool kTrack = false>
-__global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 8 : 1) k_interval_i(NetDev<R> n, BatchDev<R> bt, int q, int s0, int s1,
+__global__ void __launch_bounds__(kBlock, 1) k_interval_i(NetDev<R> n, BatchDev<R> bt, int q, int s0, int s1,
                                                                               IStep<R> ic)
 {
     interval_i_body<R, kTrack>(n, bt, q, s0, s1, ic, (int)blockIdx.x, (int)blockIdx.y);
