@@ -42,11 +42,9 @@ SEED = 3
 #   I : 12 stages x 53 ops + 376 ops of the DP8 tableau sums      = 1012 FP32 ops; 12 x (4 ex2 + 1 rcp) = 60 SFU
 FP32_RA, FP32_I = 450, 1012
 MUFU_RA, MUFU_I = 40, 60
-# DRAM bytes per launch from ncu captures of the integrators at 128 trials (RA 16.4 MB and
-# interneurons 21.8 MB read, ~0 written; the fused launch 38.2 MB), scaled to a launch of
-# BATCH trials: the state read grows with the trials.
-DRAM_BYTES_RA_PER_TRIAL = 16.4e6 / 128
-DRAM_BYTES_I_PER_TRIAL = 21.8e6 / 128
+# DRAM bytes per launch from an ncu capture of the fused integrators at 128 trials (39.3 MB
+# read, ~0 written), scaled to a launch of BATCH trials: the state read grows with the trials.
+DRAM_BYTES_PER_TRIAL = 39.3e6 / 128
 CPU_WINDOWS = 8   # the headline's CPU baseline advances every core's trial in 8 equal windows
 FP64_BATCH = 64   # test trials per batch of the batched double-precision figure
 SERVE_REQUESTS, SERVE_RATE, SERVE_MAX_TRIALS = 16, 4.0, 10   # the latency leg of the headline
@@ -432,9 +430,9 @@ def run_ours(args, rank, world, local_rank):
             "gpu_launches": launches,
             "roofline": {"bound": "fp32", "achieved": achieved / 1e12, "peak": fma_peak / 1e12, "unit": "T FP32 ops/s",
                          "frac": achieved / fma_peak, "kernel": dom,
-                         "traffic": (DRAM_BYTES_RA_PER_TRIAL + DRAM_BYTES_I_PER_TRIAL) * BATCH,
-                         "traffic_source": "ncu captures of the integrators at 128 trials, scaled by the trials "
-                                           "per launch",
+                         "traffic": DRAM_BYTES_PER_TRIAL * BATCH,
+                         "traffic_source": "ncu capture of the fused integrators at 128 trials, scaled by the "
+                                           "trials per launch",
                          "split": "k_interval_ra and k_interval_i: the same batch with the integrators launched "
                                   "apart (ug_set_interval_fusion 0)",
                          "peak_source": "FP32 FMA throughput loop (ug_calibrate_pipes), measured in this run; "
@@ -566,12 +564,12 @@ def run_growth(args, local_rank):
               "gpu_launches": launches, "clocks": clk.summary(),
               "replacements": {"events": rep_events, "neurons": rep_neurons,
                                "supersynapses_at_end": sum(len(x) for x in sup32)},
-              "launch": "one cooperative kernel per trial (all sync intervals, bounded grid barriers)",
+              "launch": "one cooperative kernel per trial (all sync intervals, bounded waits of each role)",
               "trial_shape": {"ra_threads": tuned["shape"][0], "i_threads": tuned["shape"][1],
                               "cached": tuned["cached"],
                               "table": [[t["shape"][0], t["shape"][1], round(1e3 * t["seconds"], 2)]
                                         for t in tuned["table"]],
-                              "how": "autotuned [ra, i, ms per trial]; 0 = default (32 threads)"},
+                              "how": "autotuned [ra, i, ms per trial]; 0 = the default"},
               "per_interval_launches_trials_per_s": per_interval,
               "kernel_ms_per_trial": {k: round(v[0], 3) for k, v in kt.items()},
               "kernel_ms_how": "per-interval launches timed one kernel at a time"}

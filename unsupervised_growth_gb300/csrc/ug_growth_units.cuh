@@ -14,13 +14,14 @@
 //   sync blocks    close sync q: its new post-synaptic events (the first sync block, from the
 //                  queued rows that spiked), then LTP / LTD and axon remodeling of every row;
 //                  before: the deliveries of q.
-// The interneurons' interval is the longest piece; the HVC(RA) interval, the deliveries and
-// the sync run beside it.  Rows have blocks of their own, each on an SM of its own, because a
-// row is a chain of latencies: with the rows on the integrators' SMs, eight to a block, it
-// took 16 300 cycles against a third of that alone (double-precision operations of one SM
-// queue up, and the instruction caches are refilled between integration and delivery).  The
-// order of every operation on a row, a pair or a neuron is the per-interval path's, so both
-// give the same bits.
+// An interval is the HVC(RA) steps and then the slowest of the deliveries (2000 / 550: 40 900
+// cycles, of which an HVC(RA) warp steps 9700 and waits 28 300), with the interneurons' steps
+// (19 400) and the sync beside it; in small networks (300 / 100: 24 300) the interneurons' steps.
+// Rows have blocks of their own, each on an SM of its own, because a row is a chain of
+// latencies (11 200 cycles on average): on the integrators' SMs its double-precision
+// operations queue up with theirs, and the instruction caches are refilled between integration
+// and delivery.  The order of every operation on a row, a pair or a neuron is the per-interval
+// path's, so both give the same bits.
 //
 // Every wait is bounded (ug_async.cuh): one that gives up sets kErrTimeout, every block leaves
 // at its next wait, and the host reports UG_ETIMEOUT.  An interval's deliveries can take a
