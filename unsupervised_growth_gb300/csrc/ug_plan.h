@@ -39,7 +39,8 @@ constexpr int kEnoughRowBlocks = 32, kMinRowBlocks = 8;       // rather than wid
 // Measured, ms a trial, one launch / per interval, networks with 10 training neurons:
 // 2000 HVC(RA) 40.2 / 56.7, 5000 77.9 / 92.8, 7500 118 / 130, 10 000 161 / 165, 12 000
 // 204 / 200, 18 000 342 / 305; with several hundred and synapses that grow fast: 3000 131 / 148,
-// 5000 456 / 469 (1000 training neurons: 765 / 759), 7500 1668 / 1660, 10 000 16 960 / 11 530.
+// 5000 456 / 469 (1000 training neurons: 765 / 759), 7500 1668 / 1660, 8000 1473 / 1467 (1000:
+// 4334 / 4196), 10 000 16 960 / 11 530.
 constexpr int kUnitsMaxRA = 8000;
 
 // One HVC(RA) neuron per thread where the roles fit the SMs, a block each, else two.  The rows
